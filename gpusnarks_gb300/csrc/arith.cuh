@@ -11,9 +11,10 @@
 //
 // Element layout is the reference's: uint32_t limbs, little-endian
 // (cuda/device_field.h:75).  All functions keep values canonical, in [0, p).
-// Montgomery products compute a*b*R^-1 mod p with R = 2^(32*N); the NTT
-// stores twiddles as w*R so that mont_mul(x, w*R) = x*w whatever
-// representation x is held in.
+// Montgomery products compute a*b*R^-1 mod p with R = 2^(32*N); they serve
+// products of two data elements.  The transform's products are by table
+// constants: fe_mul_tw computes x*w whatever representation x is held in
+// (the one-limb field stores w*R and takes the Montgomery product).
 #pragma once
 #include <cstdint>
 
@@ -39,6 +40,12 @@ __device__ __forceinline__ void madc_hi_cc(uint32_t& d, uint32_t a, uint32_t b, 
 }
 __device__ __forceinline__ void madc_hi(uint32_t& d, uint32_t a, uint32_t b, uint32_t c) {
   asm volatile("madc.hi.u32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
+}
+__device__ __forceinline__ void mad_lo(uint32_t& d, uint32_t a, uint32_t b, uint32_t c) {
+  asm volatile("mad.lo.u32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
+}
+__device__ __forceinline__ void madc_lo(uint32_t& d, uint32_t a, uint32_t b, uint32_t c) {
+  asm volatile("madc.lo.u32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
 }
 __device__ __forceinline__ void add_cc(uint32_t& d, uint32_t a, uint32_t b) {
   asm volatile("add.cc.u32 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
@@ -292,10 +299,8 @@ __device__ __forceinline__ void pair_chain_mod(uint32_t (&acc)[P::N + 1], int of
 // 3 carry-chain adds per row instead of N+1 for a full merge, no branch.  The adds run on the ALU pipe, but a
 // full merge is a serial chain of N+1 dependent adds between one row's products and the next row's, and it
 // cost the 24-limb product a quarter of its time (6.1 against 8.3 G products/s in isolation on GB300).
-// `row(i)` returns limb i of b, the multiplier of row i; the two forms below read it from registers or from
-// memory.
-template <class P, class Row>
-__device__ __forceinline__ void fe_mul_eo_rows(Fe<P>& r, const Fe<P>& a, Row row) {
+template <class P>
+__device__ __forceinline__ void fe_mul_eo(Fe<P>& r, const Fe<P>& a, const Fe<P>& b) {
   constexpr int N = P::N;
   static_assert(N % 2 == 0 && N >= 4, "even/odd schedule needs an even limb count of at least 4");
   uint32_t E[N + 1], O[N + 1];
@@ -304,7 +309,7 @@ __device__ __forceinline__ void fe_mul_eo_rows(Fe<P>& r, const Fe<P>& a, Row row
   for (int j = 0; j <= N; ++j) E[j] = O[j] = 0u;
 #pragma unroll
   for (int i = 0; i < N; ++i) {
-    const uint32_t bi = row(i);
+    const uint32_t bi = b.l[i];
     pair_chain<N>(E, a.l, 0, bi);
     pair_chain<N>(O, a.l, 1, bi);
     const uint32_t m = E[0] * row_pinv<P>();
@@ -345,19 +350,6 @@ __device__ __forceinline__ void fe_mul_eo_rows(Fe<P>& r, const Fe<P>& a, Row row
   for (int j = 0; j < N; ++j) r.l[j] = (t[j] & mask) | (d[j] & ~mask);
 }
 
-template <class P>
-__device__ __forceinline__ void fe_mul_eo(Fe<P>& r, const Fe<P>& a, const Fe<P>& b) {
-  fe_mul_eo_rows<P>(r, a, [&](int i) { return b.l[i]; });
-}
-
-// The same product with b's limbs loaded from memory one row at a time, so b takes no registers across the
-// product: one register per row instead of N for the whole product.  The 24-limb per-pass tile uses it to fit
-// five CTAs of 128 threads per SM (96 registers, no spills) where the register operand needs 112.
-template <class P>
-__device__ __forceinline__ void fe_mul_eo_mem(Fe<P>& r, const Fe<P>& a, const uint32_t* b) {
-  fe_mul_eo_rows<P>(r, a, [=](int i) { return b[i]; });
-}
-
 // Montgomery product used by the kernels.  GSN_MONT_SCHEDULE selects the
 // multi-limb schedule: 1 = even/odd accumulators (default), 0 = row chains.
 #ifndef GSN_MONT_SCHEDULE
@@ -371,20 +363,6 @@ __device__ __forceinline__ void fe_mul(Fe<P>& r, const Fe<P>& a, const Fe<P>& b)
     fe_mul_eo<P>(r, a, b);
   } else {
     fe_mul_rows<P>(r, a, b);
-  }
-}
-
-// r = a * b R^-1 with b's limbs in memory (any address space).  The even/odd schedule reads them row by row;
-// the others load b first.
-template <class P, int S = GSN_MONT_SCHEDULE>
-__device__ __forceinline__ void fe_mul_mem(Fe<P>& r, const Fe<P>& a, const uint32_t* b) {
-  if constexpr (S == 1 && P::N % 2 == 0 && P::N >= 4) {
-    fe_mul_eo_mem<P>(r, a, b);
-  } else {
-    Fe<P> w;
-#pragma unroll
-    for (int l = 0; l < P::N; ++l) w.l[l] = b[l];
-    fe_mul<P, S>(r, a, w);
   }
 }
 
@@ -454,6 +432,237 @@ __device__ __forceinline__ void fe_store(uint32_t* p, const Fe<P>& a) {
   } else {
 #pragma unroll
     for (int k = 0; k < N; ++k) p[k] = a.l[k];
+  }
+}
+
+// ---------------------------------------------------------------------------
+// Product by a table constant w (Shoup's precomputed quotient; V. Shoup's NTL, and D. Harvey, "Faster arithmetic
+// for number-theoretic transforms", 2014).  The table holds w and w' = floor(w R / p), R = 2^(32N).  With
+// q ~ floor(x w' / R), r = x w - q p lies in [0, 2p), so only the high half of x w' and the low halves of x w and
+// q p are needed: for 24 limbs 875 wide multiply-adds and 48 single-word ones, where a Montgomery product takes
+// 1152 wide ones and 24 row factors.  The transform multiplies only by table constants.
+//
+// Bounds: floor(x w' / R) > x w / p - x / R - 1.  q leaves out the word products below word N-2, together less
+// than (N-2) 2^(32(N-1)), which can lower it by one, in (N-2) 2^-32 of all cases.  So
+// r < p (1 + x / R + (N-2) 2^-32) + (rounding) <= p (1 + (x / R) + 2^-27) for x < R.  With x < p (and p < R / 2)
+// that is below 2p and below R, so the arithmetic modulo R is exact and one conditional subtraction ends in [0, p).
+//
+// Measured on GB300 as chains of dependent products (G products/s, 128-thread blocks), Montgomery -> this form:
+// MNT4-753 7.7 -> 10.5 (16 warps per SM, 124 registers; the multiply pipe's own limit is 11.2), BLS12-381
+// 66.8 -> 90.3 (81.9 without the modulus's two low limbs taken apart below).
+//
+// The halves are summed by rows into two accumulators per half, one for products at even words and one for odd
+// ones, so that every product lands on an aligned register pair (one wide multiply-add) and no accumulator moves.
+// ---------------------------------------------------------------------------
+
+// Words per table entry: w and w', or w R alone for the one-limb field (its product is mul1).
+template <class P>
+__host__ __device__ constexpr int tw_words() {
+  return P::N == 1 ? 1 : 2 * P::N;
+}
+
+// Limb j of R - p: adding q (R - p) subtracts q p modulo R.  p is odd, so no carry leaves word 0.
+template <class P>
+__host__ __device__ constexpr uint32_t neg_mod(int j) {
+  return j == 0 ? 0u - P::mod(0) : ~P::mod(j);
+}
+
+// (lo, hi) += a * b inside a carry chain that `first` opens.
+__device__ __forceinline__ void wide_step(uint32_t& lo, uint32_t& hi, uint32_t a, uint32_t b, bool first) {
+  if (first) {
+    ptx::mad_lo_cc(lo, a, b, lo);
+  } else {
+    ptx::madc_lo_cc(lo, a, b, lo);
+  }
+  ptx::madc_hi_cc(hi, a, b, hi);
+}
+
+// E + 2^32 O += x * y * 2^(32 i) modulo 2^(32N), for limbs j >= jmin of x.  E[k] is word k, O[k] word k + 1.
+template <int N, class X>
+__device__ __forceinline__ void low_row(uint32_t (&E)[N], uint32_t (&O)[N], X x, int i, uint32_t y, int jmin = 0) {
+  const int je = jmin + ((i + jmin) & 1), jo = jmin + ((i + jmin + 1) & 1);
+#pragma unroll
+  for (int j = je; i + j <= N - 2; j += 2) wide_step(E[i + j], E[i + j + 1], x(j), y, j == je);
+#pragma unroll
+  for (int j = jo; i + j <= N - 3; j += 2) wide_step(O[i + j - 1], O[i + j], x(j), y, j == jo);
+  const int jt = N - 1 - i;  // word N-1: the low half alone
+  if (jt == jo) {
+    ptx::mad_lo(O[N - 2], x(jt), y, O[N - 2]);
+  } else if (jt > jo) {
+    ptx::madc_lo(O[N - 2], x(jt), y, O[N - 2]);
+  }
+}
+
+// The words from N-2 up of x * y * 2^(32 i): E[k] is word N-2+k, O[k] word N-1+k.  The carry out of a row's chain
+// goes into a word that only such carries (one per parity of i) have reached before.
+template <int N, class X>
+__device__ __forceinline__ void high_row(uint32_t (&E)[N + 2], uint32_t (&O)[N + 2], X x, int i, uint32_t y) {
+  const int je = i <= N - 2 ? N - 2 - i : 1, jo = N - 1 - i;
+  int k = 0;
+#pragma unroll
+  for (int j = je; j <= N - 1; j += 2) {
+    k = i + j - (N - 2);
+    wide_step(E[k], E[k + 1], x(j), y, j == je);
+  }
+  if (k + 2 <= N + 1) ptx::addc(E[k + 2], E[k + 2], 0u);
+#pragma unroll
+  for (int j = jo; j <= N - 1; j += 2) {
+    k = i + j - (N - 1);
+    wide_step(O[k], O[k + 1], x(j), y, j == jo);
+  }
+  if (k + 2 <= N) ptx::addc(O[k + 2], O[k + 2], 0u);
+}
+
+// f(i, limb i) over N limbs in memory, read as 16-byte vectors.
+template <int N, class F>
+__device__ __forceinline__ void each_limb(const uint32_t* p, F f) {
+  const uint4* q = reinterpret_cast<const uint4*>(p);
+#pragma unroll
+  for (int k = 0; k < N / 4; ++k) {
+    const uint4 v = q[k];
+    f(4 * k + 0, v.x);
+    f(4 * k + 1, v.y);
+    f(4 * k + 2, v.z);
+    f(4 * k + 3, v.w);
+  }
+}
+
+// r = t mod p for t < 2p.
+template <class P>
+__device__ __forceinline__ void fe_reduce_once(Fe<P>& r, const uint32_t (&t)[P::N]) {
+  constexpr int N = P::N;
+  uint32_t d[N], mask;
+  ptx::sub_cc(d[0], t[0], P::mod(0));
+#pragma unroll
+  for (int j = 1; j < N; ++j) ptx::subc_cc(d[j], t[j], P::mod(j));
+  ptx::subc(mask, 0u, 0u);  // 0xFFFFFFFF iff t < p
+#pragma unroll
+  for (int j = 0; j < N; ++j) r.l[j] = (t[j] & mask) | (d[j] & ~mask);
+}
+
+// r = x * w mod p, canonical, for the table entry at `e` (tw_words<P>() words).
+template <class P>
+__device__ __forceinline__ void fe_mul_tw(Fe<P>& r, const Fe<P>& x, const uint32_t* e) {
+  constexpr int N = P::N;
+  if constexpr (N == 1) {
+    r.l[0] = mul1<P>(x.l[0], e[0]);
+  } else {
+    static_assert(N % 4 == 0, "entries are read as 16-byte vectors");
+    auto xl = [&](int j) { return x.l[j]; };
+    uint32_t q[N];
+    {
+      uint32_t E[N + 2], O[N + 2], below;
+#pragma unroll
+      for (int j = 0; j < N + 2; ++j) E[j] = O[j] = 0u;
+      each_limb<N>(e + N, [&](int i, uint32_t y) { high_row<N>(E, O, xl, i, y); });
+      ptx::add_cc(below, E[1], O[0]);
+#pragma unroll
+      for (int k = 0; k < N - 1; ++k) ptx::addc_cc(q[k], E[k + 2], O[k + 1]);
+      ptx::addc(q[N - 1], E[N + 1], O[N]);
+    }
+    uint32_t E[N], O[N], t[N];
+#pragma unroll
+    for (int j = 0; j < N; ++j) E[j] = O[j] = 0u;
+    each_limb<N>(e, [&](int i, uint32_t y) { low_row<N>(E, O, xl, i, y); });
+    // BLS12-381 r has the low limbs 1 and 2^32 - 1, so R - p = (2^32 - 1) + 2^64 (...): its two low limbs'
+    // share of q (R - p) is 2^32 q - q, two carry chains on the add pipe instead of 15 word products.
+    constexpr bool low_by_adds = P::mod(0) == 1u && P::mod(1) == 0xFFFFFFFFu;
+    auto pl = [&](int j) { return neg_mod<P>(j); };
+#pragma unroll
+    for (int i = 0; i < N; ++i) low_row<N>(E, O, pl, i, q[i], low_by_adds ? 2 : 0);
+    t[0] = E[0];
+    ptx::add_cc(t[1], E[1], O[0]);
+#pragma unroll
+    for (int j = 2; j < N - 1; ++j) ptx::addc_cc(t[j], E[j], O[j - 1]);
+    ptx::addc(t[N - 1], E[N - 1], O[N - 2]);
+    if constexpr (low_by_adds) {
+      ptx::add_cc(t[1], t[1], q[0]);
+#pragma unroll
+      for (int j = 2; j < N - 1; ++j) ptx::addc_cc(t[j], t[j], q[j - 1]);
+      ptx::addc(t[N - 1], t[N - 1], q[N - 2]);
+      ptx::sub_cc(t[0], t[0], q[0]);
+#pragma unroll
+      for (int j = 1; j < N - 1; ++j) ptx::subc_cc(t[j], t[j], q[j]);
+      ptx::subc(t[N - 1], t[N - 1], q[N - 1]);
+    }
+    fe_reduce_once<P>(r, t);
+  }
+}
+
+// Table entry of w from its Montgomery form m = w R mod p.  Reducing m by R, the row factors are the limbs of
+// -m p^-1 mod R = (w R - m) / p = w', and what is left is m / R = w mod p (below p, since m < p).
+template <class P>
+__device__ __forceinline__ void fe_store_tw(uint32_t* e, const Fe<P>& m) {
+  constexpr int N = P::N;
+  if constexpr (N == 1) {
+    e[0] = m.l[0];
+  } else {
+    Fe<P> w, f;
+    uint32_t E[N + 1], O[N + 1];
+    uint32_t q = 0u;
+#pragma unroll
+    for (int j = 0; j < N; ++j) {
+      E[j] = m.l[j];
+      O[j] = 0u;
+    }
+    E[N] = O[N] = 0u;
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      f.l[i] = E[0] * row_pinv<P>();
+      pair_chain_mod<P>(E, 0, f.l[i]);
+      pair_chain_mod<P>(O, 1, f.l[i]);
+      const uint32_t e1 = E[1];  // the merge of fe_mul_eo
+      uint32_t Onew[N + 1];
+#pragma unroll
+      for (int j = 0; j <= N - 2; ++j) Onew[j] = E[j + 2];
+      Onew[N - 1] = 0u;
+      Onew[N] = 0u;
+      ptx::add_cc(E[0], O[0], e1);
+      ptx::addc_cc(E[1], O[1], q);
+      ptx::addc(q, 0u, 0u);
+#pragma unroll
+      for (int j = 2; j <= N; ++j) E[j] = O[j];
+#pragma unroll
+      for (int j = 0; j <= N; ++j) O[j] = Onew[j];
+    }
+    w.l[0] = E[0];
+    ptx::add_cc(w.l[1], E[1], O[0]);
+#pragma unroll
+    for (int j = 2; j < N - 1; ++j) ptx::addc_cc(w.l[j], E[j], O[j - 1]);
+    ptx::addc(w.l[N - 1], E[N - 1], O[N - 2]);
+    ptx::add_cc(w.l[2], w.l[2], q);
+#pragma unroll
+    for (int j = 3; j < N - 1; ++j) ptx::addc_cc(w.l[j], w.l[j], 0u);
+    ptx::addc(w.l[N - 1], w.l[N - 1], 0u);
+    fe_store<P>(e, w);
+    fe_store<P>(e + N, f);
+  }
+}
+
+// r = x / 2^k mod p, 0 < k < 32: with f = -x p^-1 mod 2^k, x + f p is a multiple of 2^k and below 2^k p.
+// N + 1 multiply-adds, where a product by the inverse of 2^k takes a whole field product.
+template <class P>
+__device__ __forceinline__ void fe_div_pow2(Fe<P>& r, const Fe<P>& x, int k) {
+  constexpr int N = P::N;
+  const uint32_t f = (x.l[0] * row_pinv<P>()) & ((1u << k) - 1u);
+  if constexpr (N == 1) {
+    r.l[0] = (uint32_t)((x.l[0] + (uint64_t)f * P::mod(0)) >> k);
+  } else {
+    uint32_t E[N + 1], O[N + 1];
+#pragma unroll
+    for (int j = 0; j < N; ++j) {
+      E[j] = x.l[j];
+      O[j] = 0u;
+    }
+    E[N] = O[N] = 0u;
+    pair_chain_mod<P>(E, 0, f);
+    pair_chain_mod<P>(O, 1, f);
+    ptx::add_cc(E[1], E[1], O[0]);
+#pragma unroll
+    for (int j = 2; j < N; ++j) ptx::addc_cc(E[j], E[j], O[j - 1]);
+    ptx::addc(E[N], E[N], O[N - 1]);
+#pragma unroll
+    for (int j = 0; j < N; ++j) r.l[j] = __funnelshift_r(E[j], E[j + 1], k);
   }
 }
 

@@ -90,8 +90,7 @@ int plan_batch(const FieldOps& F, const gsn_batch_job* jobs, size_t njobs, Batch
       J.radix_log[k] = p.radix_log[k];
       J.log_j[k] = p.log_j[k];
     }
-    J.has_pre_const = T.has_pre_const;
-    std::memcpy(J.pre_const, T.pre_const, sizeof(J.pre_const));
+    J.div_log = T.div_log;
     out->elements += (uint64_t)1 << u.log_n;
     for (int k = 0; k < p.npass; ++k) {
       out->block = std::max(out->block, p.block[k]);

@@ -42,6 +42,7 @@ template <class P>
 constexpr FieldOps make_field_ops(int max_log_n, int default_tw_log) {
   return FieldOps{P::ID,
                   P::N,
+                  tw_words<P>(),
                   P::TWO_ADICITY,
                   max_log_n,
                   default_tw_log,

@@ -12,6 +12,7 @@ namespace gsn {
 struct FieldOps {
   int id;
   int limbs;
+  int tw_words;        // 32-bit words per twiddle or coset table entry (arith.cuh tw_words)
   int two_adicity;
   int max_log_n;       // largest supported transform (2-adicity and memory)
   int default_tw_log;  // size of the shared default twiddle table

@@ -91,13 +91,7 @@ extern "C" int gsn_ntt_noalloc(int field, uint32_t* data, uint32_t log_n, int di
     return set_error(GSN_ERR_STATE, "no twiddle table for 2^%u yet: call gsn_prepare(field, log_n, NULL) first",
                      log_n);
   T.inverse = dir == GSN_INVERSE ? 1 : 0;
-  if (T.inverse) {
-    uint32_t nn[kMaxLimbs] = {0}, ninv[kMaxLimbs];
-    nn[0] = 1u << log_n;  // log_n <= 24 here
-    F->inv(nn, ninv);
-    F->to_mont(ninv, T.pre_const);
-    T.has_pre_const = 1;
-  }
+  T.div_log = T.inverse ? (int)log_n : 0;
   uint32_t* scratch = nullptr;
   int rc = noalloc_scratch(&scratch);
   if (rc) return rc;

@@ -37,9 +37,9 @@ constexpr int kMaxLimbs = 24;
 struct PassArgs {
   const uint32_t* src;
   uint32_t* dst;
-  const uint32_t* tw;         // tw[e] = (root of order 2^tw_log)^e * R, e in [0, 2^tw_log)
-  const uint32_t* pre_table;  // pass 0 only: x[i] *= pre_table[i] (Montgomery form) or null
-  const uint32_t* post_table; // last pass only: X[k] *= post_table[k] (Montgomery form) or null
+  const uint32_t* tw;         // entry e: (root of order 2^tw_log)^e, e in [0, 2^tw_log), as fe_mul_tw takes it
+  const uint32_t* pre_table;  // pass 0 only: x[i] *= pre_table[i] (such entries) or null
+  const uint32_t* post_table; // last pass only: X[k] *= post_table[k] (such entries) or null
   uint64_t tiles;             // number of tiles in this pass
   int tw_log;
   int log_n;
@@ -52,8 +52,7 @@ struct PassArgs {
   int inverse;                // 1: use w^-e
   int npass;
   int radix_log[kMaxPasses];
-  int has_pre_const;
-  uint32_t pre_const[kMaxLimbs];  // pass 0: x *= pre_const (Montgomery form), e.g. n^-1
+  int div_log;                // last pass: X[k] /= 2^div_log before the post table (n^-1 of an inverse); 0: none
 };
 
 // One job of the batched / served path: an in-place transform of one
@@ -70,8 +69,7 @@ struct BatchJob {
   int npass;
   int radix_log[kMaxPasses];
   int log_j[kMaxPasses];
-  int has_pre_const;
-  uint32_t pre_const[kMaxLimbs];
+  int div_log;
 };
 
 // Arguments of the register-blocked 32-bit pass (ntt_p32.cuh).  Tables are

@@ -44,11 +44,6 @@ __device__ __forceinline__ uint32_t tw_index32(int tw_log, int log_n, int invers
   return idx;
 }
 
-template <class P>
-__device__ __forceinline__ void tw_load(Fe<P>& w, const uint32_t* tw, uint64_t idx) {
-  fe_load<P>(w, tw + idx * P::N);
-}
-
 // Mixed-radix digit reversal of the last pass's "rest" prefix index
 // (digits k_1..k_{P-2}, row-major) into the output offset
 // k_1 + n_1 k_2 + ... (before the final multiplication by n_0).
@@ -68,15 +63,12 @@ __device__ __forceinline__ uint64_t rest_offset(uint64_t rest, int npass, const 
   return off;
 }
 
-// One tile of one pass.  `sm` holds 2^(log_r + log_j) elements.  TW_MEM: the product reads the multiplier
-// (twiddle, pre- or post-table entry) from memory row by row (fe_mul_mem) instead of loading it into registers
-// first; A must then live in addressable memory (a __grid_constant__ parameter or shared memory), since the
-// pre-scale constant is read through a pointer to A.pre_const.
+// One tile of one pass.  `sm` holds 2^(log_r + log_j) elements.
 // Element positions and twiddle exponents are 32-bit (at most 2^28 elements per transform): 64-bit index
 // arithmetic per butterfly takes multiply-pipe instructions from the products.
-template <class P, bool TW_MEM>
+template <class P>
 __device__ void ntt_tile(const PassArgs& A, uint64_t tile, uint32_t* sm) {
-  constexpr int N = P::N;
+  constexpr int N = P::N, TW = tw_words<P>();
   const int lr = A.log_r, lj = A.log_j;
   const int R = 1 << lr, J = 1 << lj;
   const int tid = threadIdx.x, nthr = blockDim.x;
@@ -111,13 +103,13 @@ __device__ void ntt_tile(const PassArgs& A, uint64_t tile, uint32_t* sm) {
   };
 
   // --- load (no arithmetic) ------------------------------------------------
-  // Multi-limb fields without a pre-scale: stage 0 reads its two rows from global memory itself, one barrier and
-  // one shared-memory store of the tile fewer (MNT4 and BLS transforms 1-2.4% faster on GB300).  Its product hides
-  // the load latency.  The 32-bit field keeps the load phase, whose many loads in flight its short butterflies
-  // need (a p32 batch ran 6.8% slower with stage-0 loads).
-  const bool pre = A.first && (A.pre_table || A.has_pre_const);
+  // Multi-limb fields: stage 0 reads its two rows from global memory itself, or the pre-scale its element, one
+  // barrier and one shared-memory store of the tile fewer (MNT4 and BLS transforms 1-2.4% faster on GB300).  The
+  // product hides the load latency.  The 32-bit field keeps the load phase, whose many loads in flight its short
+  // butterflies need (a p32 batch ran 6.8% slower with stage-0 loads).
+  const bool pre = A.first && A.pre_table;
   const bool load_in_stage0 = N >= 8 && !pre && lr >= 2;
-  if (!load_in_stage0) {
+  if (!load_in_stage0 && !(N >= 8 && pre)) {
     for (int e = tid; e < R * J; e += nthr) {
       int k, jj;
       if (!A.last) {
@@ -136,41 +128,30 @@ __device__ void ntt_tile(const PassArgs& A, uint64_t tile, uint32_t* sm) {
 
   // --- phases; every multiplication goes through the single product below, so
   // the fully unrolled product exists once in the instruction stream --------
-  //   ph = -1        pre-scale (first pass: coset powers or n^-1)
+  //   ph = -1        pre-scale (first pass of a coset transform: powers of the shift)
   //   ph = 0..lr-2   radix-2 DIF stage ph (natural in, bit-reversed out)
   //   ph = lr        the last stage (ph = lr-1, twiddle 1: each output row is the sum or the difference of two
-  //                  rows, no product) fused with the four-step twiddle (non-last) or post table (last) and the
-  //                  store.  That saves one barrier and one shared-memory store of the tile per pass.
+  //                  rows, no product) fused with the four-step twiddle (non-last) or the division by n and the
+  //                  post table (last) and the store.  That saves one barrier and one shared-memory store of the
+  //                  tile per pass.
   for (int ph = pre ? -1 : 0; ph <= lr; ++ph) {
     if (lr > 0 && ph == lr - 1) continue;  // fused into ph = lr; uniform across the block
     const bool stage = ph >= 0 && ph < lr;
     const int count = stage ? (R >> 1) * J : R * J;
     for (int b = tid; b < count; b += nthr) {
-      Fe<P> x, w;
-      const uint32_t* wsrc = nullptr;  // TW_MEM: limbs of the multiplier
-      bool mul = false;
+      Fe<P> x;
+      const uint32_t* w = nullptr;  // table entry of the multiplier
       uint32_t* out;
-      auto take = [&](const uint32_t* src) {  // the multiplier's limbs are at src
-        if constexpr (TW_MEM) {
-          wsrc = src;
-        } else {
-          fe_load<P>(w, src);
-        }
-        mul = true;
-      };
       if (ph < 0) {
         const int k = b >> lj, jj = b & (J - 1);
+        const uint32_t pos = src_pos(k, jj);
         out = sm + ((k << lj) + jj) * N;
-        fe_load<P>(x, out);
-        if (A.pre_table) {
-          take(A.pre_table + (size_t)src_pos(k, jj) * N);
-        } else if constexpr (TW_MEM) {
-          take(A.pre_const);
+        if (N >= 8) {
+          fe_load_cg<P>(x, A.src + (size_t)pos * N);
         } else {
-#pragma unroll
-          for (int l = 0; l < N; ++l) w.l[l] = A.pre_const[l];  // 4-byte aligned in PassArgs: no vector loads
-          mul = true;
+          fe_load<P>(x, out);
         }
+        w = A.pre_table + (size_t)pos * TW;
       } else if (stage) {
         // Butterfly b = (i, group, jj) with the twiddle index i slowest: the 2^(lr-1-log_half) * J
         // butterflies of twiddle 1 (i = 0) are then consecutive threads, so in the late stages whole warps
@@ -196,7 +177,7 @@ __device__ void ntt_tile(const PassArgs& A, uint64_t tile, uint32_t* sm) {
         out = sm + ((v << lj) + jj) * N;
         if (i != 0) {
           const uint32_t e = (uint32_t)i << (ph + A.log_n - lr);
-          take(A.tw + (size_t)tw_index32(A.tw_log, A.log_n, A.inverse, e) * N);
+          w = A.tw + (size_t)tw_index32(A.tw_log, A.log_n, A.inverse, e) * TW;
         }
       } else {
         const int k = b >> lj, jj = b & (J - 1);
@@ -217,53 +198,36 @@ __device__ void ntt_tile(const PassArgs& A, uint64_t tile, uint32_t* sm) {
         if (!A.last) {
           const uint32_t ex = ((jbase + (uint32_t)jj) * (uint32_t)k) << A.log_outer;  // < n
           out = A.dst + (size_t)(base + ((uint32_t)k << A.log_inner) + (uint32_t)jj) * N;
-          if (ex != 0) take(A.tw + (size_t)tw_index32(A.tw_log, A.log_n, A.inverse, ex) * N);
+          if (ex != 0) w = A.tw + (size_t)tw_index32(A.tw_log, A.log_n, A.inverse, ex) * TW;
         } else {
           const uint32_t opos = obase + (uint32_t)jj + ((uint32_t)k << A.log_outer);
           out = A.dst + (size_t)opos * N;
-          if (A.post_table) take(A.post_table + (size_t)opos * N);
+          if (A.div_log) fe_div_pow2<P>(x, x, A.div_log);
+          if (A.post_table) w = A.post_table + (size_t)opos * TW;
         }
       }
-      if (mul) {
-        if constexpr (TW_MEM) {
-          fe_mul_mem<P>(x, x, wsrc);
-        } else {
-          fe_mul<P>(x, x, w);
-        }
-      }
+      if (w) fe_mul_tw<P>(x, x, w);
       fe_store<P>(out, x);
     }
     __syncthreads();
   }
 }
 
-// The 24-limb per-pass tile reads the multiplier from memory and is capped at 96 registers (255: no cap).
-// Registers are allocated per warp in units of 256, so 96 per thread gives 5 CTAs of 128 threads per SM
-// (20 warps) and anything from 97 to 104 only 4.  With the multiplier in registers the tile needs 112, and at
-// 96 it spills.  Measured on GB300, MNT4-753 2^18 / 2^20 / 2^22 in ms (occupancy from
-// cudaOccupancyMaxActiveBlocksPerMultiprocessor):
-//   multiplier in registers, cap 102 (4 CTAs, 48 bytes of spills):  0.3783 / 1.4354 / 5.988
-//   multiplier in registers, cap 96  (5 CTAs, 112 bytes of spills): 0.3707 / 1.4383 / 6.043
-//   multiplier from memory,  cap 96  (5 CTAs, no spills):            0.3654 / 1.4172 / 6.040
-// The tile's later changes (32-bit indices, fused last stage, stage-0 loads) leave it at 94 registers, no spills.
-template <class P>
-__host__ __device__ constexpr bool pass_tw_mem() {
-  return P::N >= 16;
-}
+// Register cap of the per-pass kernel: 128 for 24 limbs, 4 CTAs of 128 threads per SM (255: no cap).
 template <class P>
 constexpr int pass_max_regs() {
-  return P::N >= 16 ? 96 : 255;
+  return P::N >= 16 ? 128 : 255;
 }
 
 template <class P>
 __global__ void __maxnreg__(pass_max_regs<P>()) ntt_pass_kernel(const __grid_constant__ PassArgs A) {
   extern __shared__ uint4 gsn_smem[];
   uint32_t* sm = reinterpret_cast<uint32_t*>(gsn_smem);
-  for (uint64_t t = blockIdx.x; t < A.tiles; t += gridDim.x) ntt_tile<P, pass_tw_mem<P>()>(A, t, sm);
+  for (uint64_t t = blockIdx.x; t < A.tiles; t += gridDim.x) ntt_tile<P>(A, t, sm);
 }
 
-// out[e] = base^e * R (Montgomery form) for e in [0, count).  `base` is
-// canonical.  Each thread produces kPowChunk consecutive powers: one
+// Entry e of `out`: base^e, for e in [0, count), in the form fe_mul_tw takes.
+// `base` is canonical.  Each thread produces kPowChunk consecutive powers: one
 // square-and-multiply for the first, then one product per entry.
 constexpr int kPowChunk = 32;
 
@@ -284,7 +248,7 @@ __global__ void gen_powers_kernel(uint32_t* out, uint64_t count, Fe<P> base) {
   }
   const uint64_t end = (e0 + kPowChunk < count) ? e0 + kPowChunk : count;
   for (uint64_t e = e0; e < end; ++e) {
-    fe_store<P>(out + e * P::N, acc);
+    fe_store_tw<P>(out + e * tw_words<P>(), acc);
     fe_mul<P>(acc, acc, bm);
   }
 }
@@ -438,9 +402,7 @@ __device__ __forceinline__ void job_pass_args(PassArgs& A, const BatchJob& J, in
   for (int i = 0; i < kMaxPasses; ++i) A.radix_log[i] = J.radix_log[i];
   A.pre_table = A.first ? J.pre_table : nullptr;
   A.post_table = A.last ? J.post_table : nullptr;
-  A.has_pre_const = A.first ? J.has_pre_const : 0;
-  if (A.has_pre_const)
-    for (int i = 0; i < kMaxLimbs; ++i) A.pre_const[i] = J.pre_const[i];
+  A.div_log = A.last ? J.div_log : 0;
   A.tiles = (uint64_t)1 << (J.log_n - A.log_r - A.log_j);
 }
 
@@ -487,7 +449,7 @@ __global__ void __maxnreg__(batch_max_regs<P>())
       }
     }
     __syncthreads();
-    ntt_tile<P, false>(s_args, tile, sm);  // ends with __syncthreads(); s_args is rewritten only after it
+    ntt_tile<P>(s_args, tile, sm);  // ends with __syncthreads(); s_args is rewritten only after it
     if (threadIdx.x == 0) {
       __threadfence();
       atomicAdd(&counters[1 + (uint64_t)job * kMaxPasses + pass], 1u);

@@ -12,7 +12,7 @@
 // conflict-free property holds for every access pattern here: row-major loads and stores of a column
 // tile, the strided register sub-steps, and the bit-reversed reads of the final phase.
 //
-// Twiddles come from the full-circle table of the transform (tw[e] = w^e R).  In sub-step stage q the
+// Twiddles come from the full-circle table of the transform.  In sub-step stage q the
 // butterfly (m, m + E/2^(q+1)) with m = g E/2^q + t has twiddle index i = low + t 2^ls within its group,
 // so every thread reads E/2^(q+1) twiddles per stage; the last stage of the tile (i = 0) has none.
 #pragma once
@@ -69,8 +69,8 @@ __device__ __forceinline__ void substep(const PassArgs& A, uint4* sm, uint32_t r
     for (int t = 0; t < (E >> (q + 1)); ++t) {
       const uint32_t i = low + ((uint32_t)t << ls);  // twiddle index within the stage's half
       const bool mul = i != 0;
-      Fe<P> w;
-      if (mul) tw_load<P>(w, A.tw, tw_index(A.tw_log, A.log_n, A.inverse, ((uint64_t)i << ph) << (A.log_n - r)));
+      const uint32_t* w =
+          A.tw + tw_index(A.tw_log, A.log_n, A.inverse, ((uint64_t)i << ph) << (A.log_n - r)) * tw_words<P>();
 #pragma unroll
       for (int g = 0; g < (1 << q); ++g) {
         const int m = g * (E >> q) + t;
@@ -80,7 +80,7 @@ __device__ __forceinline__ void substep(const PassArgs& A, uint4* sm, uint32_t r
         fe_add<P>(s, u, v);
         fe_sub<P>(d, u, v);
         u = s;
-        if (mul) fe_mul<P>(v, d, w);
+        if (mul) fe_mul_tw<P>(v, d, w);
         else v = d;
       }
     }
@@ -109,7 +109,7 @@ __global__ void __launch_bounds__(256) ntt_rb_kernel(const __grid_constant__ Pas
   using namespace rb;
   extern __shared__ uint4 gsn_smem[];
   uint4* sm = gsn_smem;
-  constexpr int N = P::N;
+  constexpr int N = P::N, TW = tw_words<P>();
   constexpr uint32_t J = 1u << LJ;
   const int r = A.log_r;
   const uint32_t R = 1u << r;
@@ -133,13 +133,8 @@ __global__ void __launch_bounds__(256) ntt_rb_kernel(const __grid_constant__ Pas
       obase = k0 + (rest_offset(rest, A.npass, A.radix_log) << lo0);
     }
 
-    // --- load (first pass: pre-scale by the coset powers or n^-1) ---
-    const bool pre = A.first && (A.pre_table || A.has_pre_const);
-    Fe<P> pc;
-    if (pre && !A.pre_table) {
-#pragma unroll
-      for (int l = 0; l < N; ++l) pc.l[l] = A.pre_const[l];
-    }
+    // --- load (first pass of a coset transform: times the powers of the shift) ---
+    const bool pre = A.first && A.pre_table;
     // column fastest in both cases: shared-memory stores in the order the swizzle keeps conflict-free; on the
     // last pass, whose input rows are contiguous, a warp then reads 2^(5-LJ) consecutive elements per row
     for (uint32_t e = tid; e < R * J; e += nthr) {
@@ -148,10 +143,7 @@ __global__ void __launch_bounds__(256) ntt_rb_kernel(const __grid_constant__ Pas
                                  : ((rowpre + ((uint64_t)jj << (A.log_outer - lo0))) << r) + k;
       Fe<P> x;
       fe_load_cg<P>(x, A.src + g * N);
-      if (pre) {
-        if (A.pre_table) fe_load<P>(pc, A.pre_table + g * N);
-        fe_mul<P>(x, x, pc);
-      }
+      if (pre) fe_mul_tw<P>(x, x, A.pre_table + g * TW);
       sm_store<P, LJ>(sm, k, jj, r, x);
     }
     __syncthreads();
@@ -175,24 +167,19 @@ __global__ void __launch_bounds__(256) ntt_rb_kernel(const __grid_constant__ Pas
       s0 += et;
     }
 
-    // --- four-step twiddle (non-last) or post table (last), store ---
+    // --- four-step twiddle (non-last), or division by n and post table (last), store ---
     for (uint32_t v = tid; v < R * J; v += nthr) {
       const uint32_t k = v >> LJ, jj = v & (J - 1);
-      Fe<P> x, w;
+      Fe<P> x;
       sm_load<P, LJ>(x, sm, bitrev_bits(k, r), jj, r);
       if (!A.last) {
         const uint64_t ex = ((jbase + jj) * (uint64_t)k) << A.log_outer;
-        if (ex != 0) {
-          tw_load<P>(w, A.tw, tw_index(A.tw_log, A.log_n, A.inverse, ex));
-          fe_mul<P>(x, x, w);
-        }
+        if (ex != 0) fe_mul_tw<P>(x, x, A.tw + tw_index(A.tw_log, A.log_n, A.inverse, ex) * TW);
         fe_store<P>(A.dst + (base + ((uint64_t)k << A.log_inner) + jj) * N, x);
       } else {
         const uint64_t opos = obase + jj + ((uint64_t)k << A.log_outer);
-        if (A.post_table) {
-          fe_load<P>(w, A.post_table + opos * N);
-          fe_mul<P>(x, x, w);
-        }
+        if (A.div_log) fe_div_pow2<P>(x, x, A.div_log);
+        if (A.post_table) fe_mul_tw<P>(x, x, A.post_table + opos * TW);
         fe_store<P>(A.dst + opos * N, x);
       }
     }

@@ -312,7 +312,7 @@ static void default_root(const FieldOps& F, int log_n, uint32_t* out) {
 }
 
 // Field inverse (canonical in and out), memoised: one costs a full host exponentiation (about a
-// millisecond for the 753-bit field), and every inverse or coset-inverse transform needs n^-1 or s^-1.
+// millisecond for the 753-bit field), and every coset-inverse transform needs s^-1.
 static void inv_memo(const FieldOps& F, const uint32_t* x, uint32_t* out) {
   static std::mutex mu;
   static std::map<std::pair<int, std::string>, std::string> memo;
@@ -327,8 +327,8 @@ static void inv_memo(const FieldOps& F, const uint32_t* x, uint32_t* out) {
   std::memcpy(out, it->second.data(), it->second.size());
 }
 
-// Returns a cached table of base^e * R for e in [0, 2^log_count); builds it
-// on first use.  Caller holds no lock.
+// Returns a cached table of base^e for e in [0, 2^log_count), entries as
+// fe_mul_tw takes them; builds it on first use.  Caller holds no lock.
 static int powers_table(const FieldOps& F, const uint32_t* base, int log_count, const uint32_t** out) {
   TableCache& C = cache();
   const int dev = current_device();
@@ -343,7 +343,7 @@ static int powers_table(const FieldOps& F, const uint32_t* base, int log_count, 
   if (!gen) GSN_CUDA(cudaStreamCreateWithFlags(&gen, cudaStreamNonBlocking));
   const uint64_t count = (uint64_t)1 << log_count;
   DevBuf b;
-  b.bytes = count * F.limbs * sizeof(uint32_t);
+  b.bytes = count * F.tw_words * sizeof(uint32_t);
   int rc = dev_alloc(&b.p, b.bytes);
   if (rc) return rc;
   cudaError_t e = F.powers(static_cast<uint32_t*>(b.p), count, base, gen);
@@ -392,20 +392,9 @@ int resolve_tables(const FieldOps& F, uint32_t log_n, const uint32_t* omega, int
   if (rc) return rc;
   std::memcpy(T->root, omega ? omega : def, sizeof(uint32_t) * N);
   T->inverse = (dir == GSN_INVERSE || dir == GSN_COSET_INVERSE) ? 1 : 0;
-  T->has_pre_const = 0;
+  T->div_log = T->inverse ? (int)log_n : 0;
   T->pre_table = nullptr;
   T->post_table = nullptr;
-  if (T->inverse) {
-    uint32_t nn[kMaxLimbs] = {0}, ninv[kMaxLimbs];
-    nn[0] = 1u << (log_n & 31);
-    if (log_n >= 32) {  // fields with more than one limb only (p32's limit is 28)
-      nn[0] = 0;
-      nn[log_n / 32] = 1u << (log_n % 32);
-    }
-    inv_memo(F, nn, ninv);
-    F.to_mont(ninv, T->pre_const);
-    T->has_pre_const = 1;
-  }
   if (dir == GSN_COSET_FORWARD || dir == GSN_COSET_INVERSE) {
     uint32_t s[kMaxLimbs] = {0};
     if (shift) {
@@ -449,8 +438,15 @@ bool find_default_twiddles(const FieldOps& F, int log_n, const uint32_t** tw, in
 int resolve_p32_tables(const FieldOps& F, const Plan& plan, Tables* T) {
   uint32_t root[kMaxLimbs];
   std::memcpy(root, T->root, sizeof(uint32_t) * F.limbs);
-  if (T->inverse) inv_memo(F, T->root, root);
   const int L = plan.log_n;
+  if (T->inverse) {
+    inv_memo(F, T->root, root);
+    uint32_t nn[kMaxLimbs] = {0}, ninv[kMaxLimbs], r[kMaxLimbs];
+    nn[0] = 1u << L;  // at most 2^28
+    inv_memo(F, nn, ninv);
+    F.to_mont(ninv, r);
+    T->p32_pre_const = r[0];
+  }
   for (int p = 0; p < plan.npass; ++p) {
     const int r = plan.radix_log[p];
     uint32_t wr[kMaxLimbs];
@@ -510,8 +506,8 @@ static int enqueue_p32(const Plan& plan, const Tables& T, uint32_t* data, uint32
     A.tiles = (uint64_t)1 << (plan.log_n - A.log_r - A.log_j);
     A.pre_table = A.first ? T.pre_table : nullptr;
     A.post_table = A.last ? T.post_table : nullptr;
-    A.has_pre_const = A.first ? T.has_pre_const : 0;
-    A.pre_const = T.pre_const[0];
+    A.has_pre_const = A.first ? T.inverse : 0;
+    A.pre_const = T.p32_pre_const;
     cudaError_t e = launch_p32_pass(A, plan.e_log, plan.block[p], sms * 16, s);
     if (e != cudaSuccess) return cuda_fail(e, "p32 NTT pass launch");
     count_launches(1);
@@ -545,8 +541,7 @@ int enqueue_ntt(const FieldOps& F, const Plan& plan, const Tables& T, uint32_t* 
     A.tiles = (uint64_t)1 << (plan.log_n - A.log_r - A.log_j);
     A.pre_table = A.first ? T.pre_table : nullptr;
     A.post_table = A.last ? T.post_table : nullptr;
-    A.has_pre_const = A.first ? T.has_pre_const : 0;
-    if (A.has_pre_const) std::memcpy(A.pre_const, T.pre_const, sizeof(A.pre_const));
+    A.div_log = A.last ? T.div_log : 0;
     cudaError_t e = rb ? F.pass_rb(A, plan.e_log, plan.block[p], s) : F.pass(A, plan.block[p], s);
     if (e != cudaSuccess) return cuda_fail(e, "NTT pass launch");
     count_launches(1);

@@ -68,12 +68,12 @@ struct Tables {
   int tw_log = 0;
   const uint32_t* pre_table = nullptr;
   const uint32_t* post_table = nullptr;
-  int has_pre_const = 0;
-  uint32_t pre_const[kMaxLimbs] = {0};
   int inverse = 0;
+  int div_log = 0;                 // inverse: the outputs are divided by 2^div_log = n
   uint32_t root[kMaxLimbs] = {0};  // canonical root actually used (omega^-1 when inverse)
   // register-blocked 32-bit pass tables, filled by resolve_p32_tables
   const uint32_t* p32_tile[kMaxPasses] = {nullptr, nullptr, nullptr, nullptr};
+  uint32_t p32_pre_const = 0;  // inverse: n^-1 R
   const uint32_t* p32_lo = nullptr;
   const uint32_t* p32_hi = nullptr;
   int p32_lo_bits = 0;
