@@ -213,10 +213,12 @@ __device__ void ntt_tile(const PassArgs& A, uint64_t tile, uint32_t* sm) {
   }
 }
 
-// Register cap of the per-pass kernel: 128 for 24 limbs, 4 CTAs of 128 threads per SM (255: no cap).
+// Register cap of the per-pass kernel (255: no cap).  24 limbs: 128, 4 CTAs of 128 threads per SM; GB300, MNT4 2^18 /
+// 2^20 inverse in us: 302 / 1167 at 128, 310 / 1216 at 112, 316 / 1224 at 96, 306 / 1264 at 168 (3 CTAs, no spills).
+// 8 limbs: 64, 8 CTAs; uncapped it takes 84 registers (BLS 2^20 197 us; 190.5 at 80, 186.4 at 72, 184.3 at 64).
 template <class P>
 constexpr int pass_max_regs() {
-  return P::N >= 16 ? 128 : 255;
+  return P::N >= 16 ? 128 : P::N == 8 ? 64 : 255;
 }
 
 template <class P>
