@@ -129,8 +129,15 @@ __device__ __forceinline__ uint32_t sub1(uint32_t a, uint32_t b) {
 // Multi-limb fields, one element per thread.
 // ---------------------------------------------------------------------------
 
-// r = a + b mod p.  Inputs canonical.
-template <class P>
+// Limb i of K p, K = 1 or 2 (2p fits the limbs: HEADROOM >= 2).
+template <class P, int K>
+__host__ __device__ constexpr uint32_t mod_times(int i) {
+  static_assert(K == 1 || (K == 2 && P::HEADROOM >= 2), "K p must fit the limbs");
+  return K == 1 ? P::mod(i) : (P::mod(i) << 1) | (i > 0 ? P::mod(i - 1) >> 31 : 0u);
+}
+
+// r = a + b mod K p.  Inputs below K p.
+template <class P, int K = 1>
 __device__ __forceinline__ void fe_add(Fe<P>& r, const Fe<P>& a, const Fe<P>& b) {
   constexpr int N = P::N;
   if constexpr (N == 1) {
@@ -141,17 +148,17 @@ __device__ __forceinline__ void fe_add(Fe<P>& r, const Fe<P>& a, const Fe<P>& b)
 #pragma unroll
     for (int j = 1; j < N; ++j) ptx::addc_cc(s[j], a.l[j], b.l[j]);
     ptx::addc(c, 0u, 0u);
-    ptx::sub_cc(d[0], s[0], P::mod(0));
+    ptx::sub_cc(d[0], s[0], mod_times<P, K>(0));
 #pragma unroll
-    for (int j = 1; j < N; ++j) ptx::subc_cc(d[j], s[j], P::mod(j));
-    ptx::subc(mask, c, 0u);  // 0xFFFFFFFF iff s < p (no carry and a borrow)
+    for (int j = 1; j < N; ++j) ptx::subc_cc(d[j], s[j], mod_times<P, K>(j));
+    ptx::subc(mask, c, 0u);  // 0xFFFFFFFF iff s < K p (no carry and a borrow)
 #pragma unroll
     for (int j = 0; j < N; ++j) r.l[j] = (s[j] & mask) | (d[j] & ~mask);
   }
 }
 
-// r = a - b mod p.  Inputs canonical.
-template <class P>
+// r = a - b mod K p.  Inputs below K p.
+template <class P, int K = 1>
 __device__ __forceinline__ void fe_sub(Fe<P>& r, const Fe<P>& a, const Fe<P>& b) {
   constexpr int N = P::N;
   if constexpr (N == 1) {
@@ -162,10 +169,10 @@ __device__ __forceinline__ void fe_sub(Fe<P>& r, const Fe<P>& a, const Fe<P>& b)
 #pragma unroll
     for (int j = 1; j < N; ++j) ptx::subc_cc(d[j], a.l[j], b.l[j]);
     ptx::subc(mask, 0u, 0u);  // 0xFFFFFFFF iff a < b
-    ptx::add_cc(r.l[0], d[0], P::mod(0) & mask);
+    ptx::add_cc(r.l[0], d[0], mod_times<P, K>(0) & mask);
 #pragma unroll
-    for (int j = 1; j < N - 1; ++j) ptx::addc_cc(r.l[j], d[j], P::mod(j) & mask);
-    ptx::addc(r.l[N - 1], d[N - 1], P::mod(N - 1) & mask);
+    for (int j = 1; j < N - 1; ++j) ptx::addc_cc(r.l[j], d[j], mod_times<P, K>(j) & mask);
+    ptx::addc(r.l[N - 1], d[N - 1], mod_times<P, K>(N - 1) & mask);
   }
 }
 
@@ -444,8 +451,9 @@ __device__ __forceinline__ void fe_store(uint32_t* p, const Fe<P>& a) {
 //
 // Bounds: floor(x w' / R) > x w / p - x / R - 1.  q leaves out the word products below word N-2, together less
 // than (N-2) 2^(32(N-1)), which can lower it by one, in (N-2) 2^-32 of all cases.  So
-// r < p (1 + x / R + (N-2) 2^-32) + (rounding) <= p (1 + (x / R) + 2^-27) for x < R.  With x < p (and p < R / 2)
-// that is below 2p and below R, so the arithmetic modulo R is exact and one conditional subtraction ends in [0, p).
+// r < p (1 + x / R + (N-2) 2^-32) + (rounding) <= p (1 + (x / R) + 2^-27) for x < R.  With x < 2p (and 2p < R by a
+// margin above 2^-27) that is below 2p and below R, so the arithmetic modulo R is exact and one conditional
+// subtraction ends in [0, p).  A caller that keeps its values in [0, 2p) leaves that subtraction out (K = 2).
 //
 // Measured on GB300 as chains of dependent products (G products/s, 128-thread blocks), Montgomery -> this form:
 // MNT4-753 7.7 -> 10.5 (16 warps per SM, 124 registers; the multiply pipe's own limit is 11.2), BLS12-381
@@ -455,11 +463,19 @@ __device__ __forceinline__ void fe_store(uint32_t* p, const Fe<P>& a) {
 // ones, so that every product lands on an aligned register pair (one wide multiply-add) and no accumulator moves.
 // ---------------------------------------------------------------------------
 
-// Words per table entry: w and w', or w R alone for the one-limb field (its product is mul1).
+// Table layout.  The one-limb field stores w R (its product is mul1), one word per entry.  The others store w and w'
+// in blocks of 8 entries, each block chunk-major: 16-byte chunk c (limbs 4c.. of w, then of w') of entry e is at word
+// (e / 8) 16N + 32 c + 4 (e mod 8).  Lanes that read neighbouring entries then share 128-byte lines, one line per
+// chunk for 8 entries, where entry-major rows take a line per lane.
 template <class P>
-__host__ __device__ constexpr int tw_words() {
-  return P::N == 1 ? 1 : 2 * P::N;
+__device__ __forceinline__ size_t tw_offset(uint32_t e) {
+  if constexpr (P::N == 1) {
+    return e;
+  } else {
+    return (size_t)(e >> 3) * (16 * P::N) + ((e & 7u) << 2);
+  }
 }
+constexpr int kTwChunk = 32;  // words from one chunk of an entry to the next
 
 // Limb j of R - p: adding q (R - p) subtracts q p modulo R.  p is odd, so no carry leaves word 0.
 template <class P>
@@ -513,13 +529,12 @@ __device__ __forceinline__ void high_row(uint32_t (&E)[N + 2], uint32_t (&O)[N +
   if (k + 2 <= N) ptx::addc(O[k + 2], O[k + 2], 0u);
 }
 
-// f(i, limb i) over N limbs in memory, read as 16-byte vectors.
+// f(i, limb i) over N limbs of a table entry, read as 16-byte chunks.
 template <int N, class F>
 __device__ __forceinline__ void each_limb(const uint32_t* p, F f) {
-  const uint4* q = reinterpret_cast<const uint4*>(p);
 #pragma unroll
   for (int k = 0; k < N / 4; ++k) {
-    const uint4 v = q[k];
+    const uint4 v = *reinterpret_cast<const uint4*>(p + k * kTwChunk);
     f(4 * k + 0, v.x);
     f(4 * k + 1, v.y);
     f(4 * k + 2, v.z);
@@ -529,7 +544,7 @@ __device__ __forceinline__ void each_limb(const uint32_t* p, F f) {
 
 // r = t mod p for t < 2p.
 template <class P>
-__device__ __forceinline__ void fe_reduce_once(Fe<P>& r, const uint32_t (&t)[P::N]) {
+__device__ __forceinline__ void fe_reduce_once(Fe<P>& r, const uint32_t (&t)[P::N]) {  // t may be r.l
   constexpr int N = P::N;
   uint32_t d[N], mask;
   ptx::sub_cc(d[0], t[0], P::mod(0));
@@ -540,8 +555,8 @@ __device__ __forceinline__ void fe_reduce_once(Fe<P>& r, const uint32_t (&t)[P::
   for (int j = 0; j < N; ++j) r.l[j] = (t[j] & mask) | (d[j] & ~mask);
 }
 
-// r = x * w mod p, canonical, for the table entry at `e` (tw_words<P>() words).
-template <class P>
+// r = x * w mod p, below K p (K = 1: canonical), for x < 2p and the table entry at `e` (table + tw_offset<P>(index)).
+template <class P, int K = 1>
 __device__ __forceinline__ void fe_mul_tw(Fe<P>& r, const Fe<P>& x, const uint32_t* e) {
   constexpr int N = P::N;
   if constexpr (N == 1) {
@@ -554,7 +569,7 @@ __device__ __forceinline__ void fe_mul_tw(Fe<P>& r, const Fe<P>& x, const uint32
       uint32_t E[N + 2], O[N + 2], below;
 #pragma unroll
       for (int j = 0; j < N + 2; ++j) E[j] = O[j] = 0u;
-      each_limb<N>(e + N, [&](int i, uint32_t y) { high_row<N>(E, O, xl, i, y); });
+      each_limb<N>(e + N / 4 * kTwChunk, [&](int i, uint32_t y) { high_row<N>(E, O, xl, i, y); });
       ptx::add_cc(below, E[1], O[0]);
 #pragma unroll
       for (int k = 0; k < N - 1; ++k) ptx::addc_cc(q[k], E[k + 2], O[k + 1]);
@@ -585,7 +600,12 @@ __device__ __forceinline__ void fe_mul_tw(Fe<P>& r, const Fe<P>& x, const uint32
       for (int j = 1; j < N - 1; ++j) ptx::subc_cc(t[j], t[j], q[j]);
       ptx::subc(t[N - 1], t[N - 1], q[N - 1]);
     }
-    fe_reduce_once<P>(r, t);
+    if constexpr (K == 1) {
+      fe_reduce_once<P>(r, t);
+    } else {
+#pragma unroll
+      for (int j = 0; j < N; ++j) r.l[j] = t[j];
+    }
   }
 }
 
@@ -634,12 +654,18 @@ __device__ __forceinline__ void fe_store_tw(uint32_t* e, const Fe<P>& m) {
 #pragma unroll
     for (int j = 3; j < N - 1; ++j) ptx::addc_cc(w.l[j], w.l[j], 0u);
     ptx::addc(w.l[N - 1], w.l[N - 1], 0u);
-    fe_store<P>(e, w);
-    fe_store<P>(e + N, f);
+#pragma unroll
+    for (int k = 0; k < N / 4; ++k) {
+      *reinterpret_cast<uint4*>(e + k * kTwChunk) =
+          make_uint4(w.l[4 * k], w.l[4 * k + 1], w.l[4 * k + 2], w.l[4 * k + 3]);
+      *reinterpret_cast<uint4*>(e + (N / 4 + k) * kTwChunk) =
+          make_uint4(f.l[4 * k], f.l[4 * k + 1], f.l[4 * k + 2], f.l[4 * k + 3]);
+    }
   }
 }
 
-// r = x / 2^k mod p, 0 < k < 32: with f = -x p^-1 mod 2^k, x + f p is a multiple of 2^k and below 2^k p.
+// r = x / 2^k mod p, 0 < k < 32: with f = -x p^-1 mod 2^k, x + f p is a multiple of 2^k and below 2^k p for x < p
+// (and below (2^k + 1) p for x < 2p, so r < 2p).
 // N + 1 multiply-adds, where a product by the inverse of 2^k takes a whole field product.
 template <class P>
 __device__ __forceinline__ void fe_div_pow2(Fe<P>& r, const Fe<P>& x, int k) {

@@ -75,6 +75,8 @@ int plan_batch(const FieldOps& F, const gsn_batch_job* jobs, size_t njobs, Batch
     if (rc) return rc;
     Plan p = force ? *force : plan_for(F, (int)u.log_n, /*batched=*/true);
     if (force && p.log_n != (int)u.log_n) return set_error(GSN_ERR_ARG, "forced plan size mismatch");
+    rc = resolve_pass_tables(F, p, &T, nullptr);
+    if (rc) return rc;
     out->plans[i] = p;
     BatchJob& J = out->jobs[i];
     std::memset(&J, 0, sizeof(J));
@@ -89,6 +91,9 @@ int plan_batch(const FieldOps& F, const gsn_batch_job* jobs, size_t njobs, Batch
     for (int k = 0; k < kMaxPasses; ++k) {
       J.radix_log[k] = p.radix_log[k];
       J.log_j[k] = p.log_j[k];
+      J.stage_tw[k] = T.stage[k];
+      J.stage_shift[k] = T.stage_shift[k];
+      J.step_tw[k] = T.step[k];
     }
     J.div_log = T.div_log;
     out->elements += (uint64_t)1 << u.log_n;

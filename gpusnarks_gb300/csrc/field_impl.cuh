@@ -7,7 +7,6 @@
 #include "host_field.h"
 #include "multiexp.cuh"
 #include "ntt_kernels.cuh"
-#include "ntt_rb.cuh"
 
 namespace gsn {
 
@@ -42,14 +41,13 @@ template <class P>
 constexpr FieldOps make_field_ops(int max_log_n, int default_tw_log) {
   return FieldOps{P::ID,
                   P::N,
-                  tw_words<P>(),
                   P::TWO_ADICITY,
                   max_log_n,
                   default_tw_log,
                   P::GENERATOR,
                   &Kernels<P>::pass,
-                  &RbKernels<P>::pass,
                   &Kernels<P>::powers,
+                  &Kernels<P>::step_table,
                   &Kernels<P>::pointwise,
                   &Kernels<P>::quotient,
                   &Kernels<P>::fill,

@@ -12,16 +12,16 @@ namespace gsn {
 struct FieldOps {
   int id;
   int limbs;
-  int tw_words;        // 32-bit words per twiddle or coset table entry (arith.cuh tw_words)
   int two_adicity;
   int max_log_n;       // largest supported transform (2-adicity and memory)
   int default_tw_log;  // size of the shared default twiddle table
   uint32_t generator;  // multiplicative generator (a quadratic non-residue)
   // device
   cudaError_t (*pass)(const PassArgs& A, int block, cudaStream_t s);
-  // register-blocked pass (ntt_rb.cuh), 2^e_log rows per thread per sub-step; BLS12-381 only
-  cudaError_t (*pass_rb)(const PassArgs& A, int e_log, int block, cudaStream_t s);
   cudaError_t (*powers)(uint32_t* out, uint64_t count, const uint32_t* base_canon, cudaStream_t s);
+  // step table of a pass of radix 2^r (ntt_common.h) from the twiddle table: out entry k 2^inner + j is
+  // tw entry (j k) << shift, k < 2^r, j < 2^inner (multi-limb fields)
+  cudaError_t (*step_table)(uint32_t* out, const uint32_t* tw, int r, int inner, int shift, cudaStream_t s);
   cudaError_t (*pointwise)(uint32_t* a, const uint32_t* b, uint64_t n, cudaStream_t s);
   // a[i] = (a[i] b[i] - c[i]) z, zr2 = z R^2 (limbs)
   cudaError_t (*quotient)(uint32_t* a, const uint32_t* b, const uint32_t* c, uint64_t n, const uint32_t* zr2,
@@ -46,6 +46,11 @@ struct FieldOps {
   void (*pow)(const uint32_t* x, uint64_t e, uint32_t* out);
   void (*modulus)(uint32_t* out);
 };
+
+// Words of a twiddle or coset table of `count` entries (arith.cuh tw_offset: blocks of 8 for the multi-limb fields).
+inline size_t table_words(const FieldOps& F, uint64_t count) {
+  return F.limbs == 1 ? (size_t)count : (size_t)((count + 7) & ~(uint64_t)7) * 2 * F.limbs;
+}
 
 extern const FieldOps kOpsP32;
 extern const FieldOps kOpsBLS12_381;

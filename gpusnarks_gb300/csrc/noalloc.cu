@@ -97,5 +97,6 @@ extern "C" int gsn_ntt_noalloc(int field, uint32_t* data, uint32_t log_n, int di
   if (rc) return rc;
   // the generic multi-pass kernels; they read only the full twiddle table
   const Plan plan = plan_for(*F, (int)log_n, /*batched=*/true);
+  full_table_passes(plan, &T);
   return enqueue_ntt(*F, plan, T, data, scratch, static_cast<cudaStream_t>(stream));
 }

@@ -38,10 +38,14 @@ struct PassArgs {
   const uint32_t* src;
   uint32_t* dst;
   const uint32_t* tw;         // entry e: (root of order 2^tw_log)^e, e in [0, 2^tw_log), as fe_mul_tw takes it
+  const uint32_t* stage_tw;   // entry e << stage_shift: w_R^e for the pass radix R, e < R/2 (`tw` or a table of its own)
+  const uint32_t* step_tw;    // entry k 2^log_inner + j': w^(outer j' k), the four-step factors in the order the tile
+                              // takes them, or null: read from `tw`
   const uint32_t* pre_table;  // pass 0 only: x[i] *= pre_table[i] (such entries) or null
   const uint32_t* post_table; // last pass only: X[k] *= post_table[k] (such entries) or null
   uint64_t tiles;             // number of tiles in this pass
   int tw_log;
+  int stage_shift;
   int log_n;
   int log_r;                  // this pass: sub-DFT size 2^log_r
   int log_inner;              // stride (log2) between consecutive sub-DFT inputs; 0 on the last pass
@@ -49,7 +53,8 @@ struct PassArgs {
   int log_j;                  // log2 columns (rows on the last pass) per tile
   int last;                   // 1 on the last pass
   int first;                  // 1 on pass 0
-  int inverse;                // 1: use w^-e
+  int inverse;                // 1: the inverse transform.  The one-limb field uses w^-e; the others use the forward
+                              // tables and write output k to position -k mod n (the inverse's definition)
   int npass;
   int radix_log[kMaxPasses];
   int div_log;                // last pass: X[k] /= 2^div_log before the post table (n^-1 of an inverse); 0: none
@@ -60,10 +65,13 @@ struct PassArgs {
 struct BatchJob {
   uint32_t* data;        // device, n elements
   uint32_t* scratch;     // device, n elements (unused when npass == 1)
-  const uint32_t* tw;    // twiddle table (see PassArgs::tw)
+  const uint32_t* tw;    // twiddle tables (see PassArgs)
+  const uint32_t* stage_tw[kMaxPasses];
+  const uint32_t* step_tw[kMaxPasses];
   const uint32_t* pre_table;
   const uint32_t* post_table;
   int tw_log;
+  int stage_shift[kMaxPasses];
   int log_n;
   int inverse;
   int npass;
@@ -90,6 +98,11 @@ struct P32Args {
   int pipe;                    // set by the launcher: non-last pass with two tile buffers (prefetch)
   int radix_log[kMaxPasses];
 };
+
+// Words of shared memory of a tile of `elems` elements: multi-limb elements lie in blocks of 8 (ntt_kernels.cuh).
+inline size_t tile_words(int limbs, uint64_t elems) {
+  return (size_t)(limbs > 1 && elems < 8 ? 8 : elems) * limbs;
+}
 
 __host__ __device__ inline uint64_t pass_tiles(int log_n, int npass, const int* radix_log, int p, int log_j) {
   (void)npass;

@@ -10,6 +10,7 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdint>
 
 #include "arith.cuh"
@@ -27,21 +28,79 @@ __device__ __forceinline__ uint32_t bitrev_bits(uint32_t x, int bits) {
   return bits == 0 ? 0u : (__brev(x) >> (32 - bits));
 }
 
-// Table index of w_n^e (e in units of the transform's own root).
-__device__ __forceinline__ uint64_t tw_index(int tw_log, int log_n, int inverse, uint64_t e) {
-  const uint64_t size = (uint64_t)1 << tw_log;
-  uint64_t idx = e << (tw_log - log_n);
-  if (inverse) idx = (size - idx) & (size - 1);
-  return idx;
+// Indices are 32-bit: every transform has at most 2^28 elements (the fields' size limits), and so does every table.
+
+// e, or -e modulo the table's 2^log entries for the one-limb field's inverse transforms.
+template <class P>
+__device__ __forceinline__ uint32_t tw_sign(uint32_t e, int log, int inverse) {
+  return P::N == 1 && inverse ? (0u - e) & ((1u << log) - 1u) : e;
 }
 
-// The same in 32 bits, for the per-element arithmetic of ntt_tile: every transform has at most 2^28 elements
-// (the fields' size limits), and so does every twiddle table.
-__device__ __forceinline__ uint32_t tw_index32(int tw_log, int log_n, int inverse, uint32_t e) {
-  const uint32_t size = 1u << tw_log;
-  uint32_t idx = e << (tw_log - log_n);
-  if (inverse) idx = (size - idx) & (size - 1u);
-  return idx;
+// Stage twiddle w_R^e of a pass, e < R/2.
+template <class P>
+__device__ __forceinline__ const uint32_t* stage_entry(const PassArgs& A, uint32_t e) {
+  return A.stage_tw + tw_offset<P>(tw_sign<P>(e << A.stage_shift, A.tw_log, A.inverse));
+}
+
+// Four-step factor w^(outer j k) of output k in column j.
+template <class P>
+__device__ __forceinline__ const uint32_t* step_entry(const PassArgs& A, uint32_t j, uint32_t k) {
+  if (P::N > 1 && A.step_tw) return A.step_tw + tw_offset<P>((k << A.log_inner) + j);
+  const uint32_t e = (j * k) << (A.log_outer + A.tw_log - A.log_n);  // < 2^tw_log
+  return A.tw + tw_offset<P>(tw_sign<P>(e, A.tw_log, A.inverse));
+}
+
+// Position of output k of the last pass: -k mod n for the multi-limb fields' inverse transforms.
+template <class P>
+__device__ __forceinline__ uint32_t out_pos(const PassArgs& A, uint32_t k) {
+  return P::N > 1 && A.inverse ? (0u - k) & ((1u << A.log_n) - 1u) : k;
+}
+
+// Multi-limb tile elements in shared memory: blocks of 8 slots, each block chunk-major (16-byte chunk c of slot s at
+// word (s / 8) 8N + 32 c + 4 (s mod 8)), so that a quarter warp's 16-byte accesses to 8 slots of different s mod 8 take
+// one pass over the banks; with element-major rows of 32 or 96 bytes every access was a two-way conflict.  Element
+// (row, jj) has slot (row 2^lj + jj) ^ tile_hash(row): with fewer than 8 columns the bits of s mod 8 above the column
+// also take in the higher row bits, because a quarter warp's rows are 2^m apart in the late stages and the bit-reversed
+// reads.  tile_hash is linear over xor, and 0 for row 1.
+template <int LJ>
+__device__ __forceinline__ uint32_t tile_hash(uint32_t row, int lj) {
+  const int l = LJ >= 0 ? LJ : lj;
+  if (l >= 3) return 0u;
+  if (l == 2) return (uint32_t)(__popc(row >> 1) & 1) << 2;
+  if (l == 1) {
+    row >>= 2;
+    row ^= row >> 4;
+    row ^= row >> 2;
+    return ((row ^ (row >> 8)) & 3u) << 1;
+  }
+  row >>= 3;
+  row ^= row >> 6;
+  return (row ^ (row >> 3)) & 7u;
+}
+template <int LJ>
+__device__ __forceinline__ uint32_t tile_slot(uint32_t row, uint32_t jj, int lj) {
+  return ((row << (LJ >= 0 ? LJ : lj)) + jj) ^ tile_hash<LJ>(row, lj);
+}
+template <class P>
+__device__ __forceinline__ uint32_t* tile_at(uint32_t* sm, uint32_t slot) {
+  return sm + (slot >> 3) * (8 * P::N) + ((slot & 7u) << 2);
+}
+template <class P>
+__device__ __forceinline__ void tile_load(Fe<P>& x, const uint32_t* p) {
+#pragma unroll
+  for (int c = 0; c < P::N / 4; ++c) {
+    const uint4 v = *reinterpret_cast<const uint4*>(p + 32 * c);
+    x.l[4 * c + 0] = v.x;
+    x.l[4 * c + 1] = v.y;
+    x.l[4 * c + 2] = v.z;
+    x.l[4 * c + 3] = v.w;
+  }
+}
+template <class P>
+__device__ __forceinline__ void tile_store(uint32_t* p, const Fe<P>& x) {
+#pragma unroll
+  for (int c = 0; c < P::N / 4; ++c)
+    *reinterpret_cast<uint4*>(p + 32 * c) = make_uint4(x.l[4 * c], x.l[4 * c + 1], x.l[4 * c + 2], x.l[4 * c + 3]);
 }
 
 // Mixed-radix digit reversal of the last pass's "rest" prefix index
@@ -63,169 +122,241 @@ __device__ __forceinline__ uint64_t rest_offset(uint64_t rest, int npass, const 
   return off;
 }
 
-// One tile of one pass.  `sm` holds 2^(log_r + log_j) elements.
-// Element positions and twiddle exponents are 32-bit (at most 2^28 elements per transform): 64-bit index
-// arithmetic per butterfly takes multiply-pipe instructions from the products.
-template <class P>
-__device__ void ntt_tile(const PassArgs& A, uint64_t tile, uint32_t* sm) {
-  constexpr int N = P::N, TW = tw_words<P>();
-  const int lr = A.log_r, lj = A.log_j;
-  const int R = 1 << lr, J = 1 << lj;
-  const int tid = threadIdx.x, nthr = blockDim.x;
+// Where a tile's elements come from and go to.
+struct TileGeom {
+  uint32_t base = 0;    // non-last: first element of the tile
+  uint32_t jbase = 0;   // non-last: first suffix index j'
+  uint32_t rowpre = 0;  // last: prefix_lin of row 0 = (k0_first << (outer_log - lo0)) + rest
+  uint32_t obase = 0;   // last: output offset of row 0 (k_0 = k0_first, k = 0)
+  int row_shift = 0;    // last: log2 of the distance between two rows' prefixes
 
-  // --- tile geometry -------------------------------------------------------
-  uint32_t base = 0;     // non-last: first element of the tile
-  uint32_t jbase = 0;    // non-last: first suffix index j'
-  uint32_t rowpre = 0;   // last: prefix_lin of row 0 = (k0_first << (outer_log - lo0)) + rest
-  uint32_t obase = 0;    // last: output offset of row 0 (k_0 = k0_first, k = 0)
-  int lo0 = 0;           // last: log2 n_0 (0 for a single pass)
-  const uint32_t t32 = (uint32_t)tile;  // tiles < 2^28
-  if (!A.last) {
-    const int per_prefix_log = A.log_inner - lj;
-    const uint32_t prefix = t32 >> per_prefix_log;
-    const uint32_t jb = t32 & ((1u << per_prefix_log) - 1u);
-    jbase = jb << lj;
-    base = (prefix << (lr + A.log_inner)) + jbase;
-  } else {
-    lo0 = (A.npass == 1) ? 0 : A.radix_log[0];
-    const int k0b_log = lo0 - lj;
-    const uint32_t k0b = t32 & ((1u << k0b_log) - 1u);
-    const uint32_t rest = t32 >> k0b_log;
-    const uint32_t k0 = k0b << lj;
-    rowpre = (k0 << (A.log_outer - lo0)) + rest;
-    obase = k0 + ((uint32_t)rest_offset(rest, A.npass, A.radix_log) << lo0);
-  }
-
-  // global position of tile element (k, jj) in the source array
-  auto src_pos = [&](int k, int jj) -> uint32_t {
-    return !A.last ? base + ((uint32_t)k << A.log_inner) + (uint32_t)jj
-                   : ((rowpre + ((uint32_t)jj << (A.log_outer - lo0))) << lr) + (uint32_t)k;
-  };
-
-  // --- load (no arithmetic) ------------------------------------------------
-  // Multi-limb fields: stage 0 reads its two rows from global memory itself, or the pre-scale its element, one
-  // barrier and one shared-memory store of the tile fewer (MNT4 and BLS transforms 1-2.4% faster on GB300).  The
-  // product hides the load latency.  The 32-bit field keeps the load phase, whose many loads in flight its short
-  // butterflies need (a p32 batch ran 6.8% slower with stage-0 loads).
-  const bool pre = A.first && A.pre_table;
-  const bool load_in_stage0 = N >= 8 && !pre && lr >= 2;
-  if (!load_in_stage0 && !(N >= 8 && pre)) {
-    for (int e = tid; e < R * J; e += nthr) {
-      int k, jj;
-      if (!A.last) {
-        k = e >> lj;
-        jj = e & (J - 1);
-      } else {
-        jj = e >> lr;  // input rows are contiguous on the last pass
-        k = e & (R - 1);
-      }
-      Fe<P> x;
-      fe_load_cg<P>(x, A.src + (size_t)src_pos(k, jj) * N);
-      fe_store<P>(sm + ((k << lj) + jj) * N, x);
+  __device__ __forceinline__ TileGeom(const PassArgs& A, uint32_t tile) {
+    if (!A.last) {
+      const int per_prefix_log = A.log_inner - A.log_j;
+      const uint32_t prefix = tile >> per_prefix_log;
+      jbase = (tile & ((1u << per_prefix_log) - 1u)) << A.log_j;
+      base = (prefix << (A.log_r + A.log_inner)) + jbase;
+    } else {
+      const int lo0 = (A.npass == 1) ? 0 : A.radix_log[0];
+      const int k0b_log = lo0 - A.log_j;
+      const uint32_t rest = tile >> k0b_log;
+      const uint32_t k0 = (tile & ((1u << k0b_log) - 1u)) << A.log_j;
+      row_shift = A.log_outer - lo0;
+      rowpre = (k0 << row_shift) + rest;
+      obase = k0 + ((uint32_t)rest_offset(rest, A.npass, A.radix_log) << lo0);
     }
-    __syncthreads();
   }
+  // position of tile element (k, jj) in the source array
+  __device__ __forceinline__ uint32_t src(const PassArgs& A, uint32_t k, uint32_t jj) const {
+    return !A.last ? base + (k << A.log_inner) + jj : ((rowpre + (jj << row_shift)) << A.log_r) + k;
+  }
+  // position of output k of column (last pass: row) jj in the destination array
+  template <class P>
+  __device__ __forceinline__ uint32_t dst(const PassArgs& A, uint32_t k, uint32_t jj) const {
+    return !A.last ? base + (k << A.log_inner) + jj : out_pos<P>(A, obase + jj + (k << A.log_outer));
+  }
+};
 
-  // --- phases; every multiplication goes through the single product below, so
-  // the fully unrolled product exists once in the instruction stream --------
-  //   ph = -1        pre-scale (first pass of a coset transform: powers of the shift)
-  //   ph = 0..lr-2   radix-2 DIF stage ph (natural in, bit-reversed out)
-  //   ph = lr        the last stage (ph = lr-1, twiddle 1: each output row is the sum or the difference of two
-  //                  rows, no product) fused with the four-step twiddle (non-last) or the division by n and the
-  //                  post table (last) and the store.  That saves one barrier and one shared-memory store of the
-  //                  tile per pass.
-  for (int ph = pre ? -1 : 0; ph <= lr; ++ph) {
+// One tile of one pass, one-limb field.  `sm` holds 2^(log_r + log_j) words.  A load phase (many loads in flight, which
+// its short butterflies need: a batch ran 6.8% slower with loads in stage 0), then phases:
+//   ph = -1        pre-scale (first pass of a coset transform: powers of the shift)
+//   ph = 0..lr-2   radix-2 DIF stage ph (natural in, bit-reversed out)
+//   ph = lr        the last stage (ph = lr-1, twiddle 1: each output row is the sum or the difference of two rows, no
+//                  product) fused with the four-step twiddle (non-last) or the division by n and the post table (last)
+//                  and the store: one barrier and one shared-memory store of the tile fewer per pass.
+template <class P>
+__device__ void word_tile(const PassArgs& A, uint32_t tile, uint32_t* sm) {
+  static_assert(P::N == 1, "one limb");
+  const int lr = A.log_r, lj = A.log_j;
+  const uint32_t R = 1u << lr, J = 1u << lj, nthr = blockDim.x;
+  const TileGeom G(A, tile);
+  for (uint32_t e = threadIdx.x; e < R * J; e += nthr) {
+    // input rows are contiguous on the last pass
+    const uint32_t k = !A.last ? e >> lj : e & (R - 1u), jj = !A.last ? e & (J - 1u) : e >> lr;
+    sm[(k << lj) + jj] = __ldcg(A.src + G.src(A, k, jj));
+  }
+  __syncthreads();
+  for (int ph = A.first && A.pre_table ? -1 : 0; ph <= lr; ++ph) {
     if (lr > 0 && ph == lr - 1) continue;  // fused into ph = lr; uniform across the block
     const bool stage = ph >= 0 && ph < lr;
-    const int count = stage ? (R >> 1) * J : R * J;
-    for (int b = tid; b < count; b += nthr) {
-      Fe<P> x;
+    const uint32_t count = stage ? (R >> 1) * J : R * J;
+    for (uint32_t b = threadIdx.x; b < count; b += nthr) {
+      const uint32_t jj = b & (J - 1u), t = b >> lj;
+      Fe<P> x, y;
       const uint32_t* w = nullptr;  // table entry of the multiplier
       uint32_t* out;
       if (ph < 0) {
-        const int k = b >> lj, jj = b & (J - 1);
-        const uint32_t pos = src_pos(k, jj);
-        out = sm + ((k << lj) + jj) * N;
-        if (N >= 8) {
-          fe_load_cg<P>(x, A.src + (size_t)pos * N);
-        } else {
-          fe_load<P>(x, out);
-        }
-        w = A.pre_table + (size_t)pos * TW;
+        out = sm + b;
+        x.l[0] = *out;
+        w = A.pre_table + G.src(A, t, jj);
       } else if (stage) {
-        // Butterfly b = (i, group, jj) with the twiddle index i slowest: the 2^(lr-1-log_half) * J
-        // butterflies of twiddle 1 (i = 0) are then consecutive threads, so in the late stages whole warps
-        // skip the product instead of idling beside lanes that compute it.
-        const int log_half = lr - 1 - ph;
-        const int groups_log = ph;  // (lr - 1) - log_half
-        const int jj = b & (J - 1);
-        const int group = (b >> lj) & ((1 << groups_log) - 1);
-        const int i = b >> (groups_log + lj);
-        const int u = (group << (log_half + 1)) + i;
-        const int v = u + (1 << log_half);
-        Fe<P> y, sum;
-        if (ph == 0 && load_in_stage0) {
-          fe_load_cg<P>(x, A.src + (size_t)src_pos(u, jj) * N);
-          fe_load_cg<P>(y, A.src + (size_t)src_pos(v, jj) * N);
-        } else {
-          fe_load<P>(x, sm + ((u << lj) + jj) * N);
-          fe_load<P>(y, sm + ((v << lj) + jj) * N);
-        }
-        fe_add<P>(sum, x, y);
-        fe_sub<P>(x, x, y);
-        fe_store<P>(sm + ((u << lj) + jj) * N, sum);
-        out = sm + ((v << lj) + jj) * N;
-        if (i != 0) {
-          const uint32_t e = (uint32_t)i << (ph + A.log_n - lr);
-          w = A.tw + (size_t)tw_index32(A.tw_log, A.log_n, A.inverse, e) * TW;
-        }
+        // butterfly b = (i, group, jj), the twiddle index i slowest: whole warps skip the products by 1
+        const uint32_t i = t >> ph, u = ((t & ((1u << ph) - 1u)) << (lr - ph)) + i;
+        uint32_t* const up = sm + (u << lj) + jj;
+        out = up + (1u << (lr - 1 - ph + lj));
+        x.l[0] = *up;
+        y.l[0] = *out;
+        *up = add1<P>(x.l[0], y.l[0]);
+        x.l[0] = sub1<P>(x.l[0], y.l[0]);
+        if (i != 0) w = stage_entry<P>(A, i << ph);
       } else {
-        const int k = b >> lj, jj = b & (J - 1);
         if (lr > 0) {
-          // row r = bitrev(k) after the last stage: the sum (r even) or difference (r odd) of rows r&~1, r|1
-          const uint32_t r = bitrev_bits((uint32_t)k, lr);
-          Fe<P> y;
-          fe_load<P>(x, sm + (((r & ~1u) << lj) + jj) * N);
-          fe_load<P>(y, sm + (((r | 1u) << lj) + jj) * N);
-          if (r & 1u) {
-            fe_sub<P>(x, x, y);
-          } else {
-            fe_add<P>(x, x, y);
-          }
+          const uint32_t r = bitrev_bits(t, lr);  // row of output t
+          x.l[0] = sm[((r & ~1u) << lj) + jj];
+          y.l[0] = sm[((r | 1u) << lj) + jj];
+          x.l[0] = (r & 1u) ? sub1<P>(x.l[0], y.l[0]) : add1<P>(x.l[0], y.l[0]);
         } else {
-          fe_load<P>(x, sm + jj * N);
+          x.l[0] = sm[jj];
         }
+        const uint32_t pos = G.dst<P>(A, t, jj);
+        out = A.dst + pos;
         if (!A.last) {
-          const uint32_t ex = ((jbase + (uint32_t)jj) * (uint32_t)k) << A.log_outer;  // < n
-          out = A.dst + (size_t)(base + ((uint32_t)k << A.log_inner) + (uint32_t)jj) * N;
-          if (ex != 0) w = A.tw + (size_t)tw_index32(A.tw_log, A.log_n, A.inverse, ex) * TW;
+          w = step_entry<P>(A, G.jbase + jj, t);
         } else {
-          const uint32_t opos = obase + (uint32_t)jj + ((uint32_t)k << A.log_outer);
-          out = A.dst + (size_t)opos * N;
           if (A.div_log) fe_div_pow2<P>(x, x, A.div_log);
-          if (A.post_table) w = A.post_table + (size_t)opos * TW;
+          if (A.post_table) w = A.post_table + pos;
         }
       }
       if (w) fe_mul_tw<P>(x, x, w);
-      fe_store<P>(out, x);
+      *out = x.l[0];
     }
     __syncthreads();
   }
 }
 
+// One tile of one pass, multi-limb fields; the phases of word_tile without its load phase (the first phase reads
+// global memory itself, and its product hides the latency).  `sm` holds 2^(log_r + log_j) elements (tile_words).  LJ:
+// the tile's log_j at compile time, or -1.
+//
+// Bound: the multiply pipe.  Each phase has its own product and straight code.  Sharing one product between the phases
+// cost register moves where their values meet, and with them went generic addresses and run-time column counts: a
+// BLS12-381 butterfly took 394 instructions, of which 218 are arithmetic, and 156 of them on the multiply pipe instead
+// of 111 (GB300, ncu); here it takes about 300, 120 on that pipe.  With the table layout and the swizzle above, BLS12-381
+// 2^20 went from 184 to 163 us and MNT4-753 2^18 / 2^20 from 302 / 1167 (inverse) to 294 / 1110.  Barriers are not what
+// is left (the stages without them: 283 / 1119 us for MNT4, 162 for BLS), nor is memory (every table and source read
+// from L1: 4% less).  At 2^18 a pass is 1024 tiles on 152 SMs; an SM's seventh tile runs alone, one warp per
+// scheduler, and one warp of carry chains reaches 66% of the pipe where two reach 96%.
+//
+// Values stay in [0, 2p) between the phases and the passes (a product's last subtraction is left out) until the last
+// pass's store.
+template <class P, int LJ>
+__device__ __forceinline__ void field_tile(const PassArgs& A, uint32_t tile, uint32_t* sm) {
+  constexpr int N = P::N;
+  const int lr = A.log_r, lj = LJ >= 0 ? LJ : A.log_j;
+  const uint32_t R = 1u << lr, J = 1u << lj, nthr = blockDim.x;
+  const TileGeom G(A, tile);
+  bool in_tile = false;  // the elements are in shared memory
+
+  auto src = [&](uint32_t row, uint32_t jj) { return A.src + (size_t)G.src(A, row, jj) * N; };
+  auto at = [&](uint32_t slot) { return tile_at<P>(sm, slot); };
+
+  if (A.first && A.pre_table) {  // coset transform: times the powers of the shift
+#pragma unroll 1
+    for (uint32_t b = threadIdx.x; b < R << lj; b += nthr) {
+      const uint32_t jj = b & (J - 1u), t = b >> lj, pos = G.src(A, t, jj);
+      Fe<P> x, r;
+      fe_load_cg<P>(x, A.src + (size_t)pos * N);
+      fe_mul_tw<P, 2>(r, x, A.pre_table + tw_offset<P>(pos));
+      tile_store<P>(at(tile_slot<LJ>(t, jj, lj)), r);
+    }
+    in_tile = true;
+    __syncthreads();
+  }
+
+  // radix-2 DIF stages 0 .. lr-2 (natural order in, bit-reversed out)
+#pragma unroll 1
+  for (int ph = 0; ph < lr - 1; ++ph) {
+    const uint32_t half = R >> (ph + 1), flip = tile_slot<LJ>(half, 0, lj);
+#pragma unroll 1
+    for (uint32_t b = threadIdx.x; b < (R >> 1) << lj; b += nthr) {
+      // butterfly b = (i, group, jj) with the twiddle index i slowest, so that in the late stages, where 2^ph of the
+      // butterflies have twiddle 1, whole warps skip the product
+      const uint32_t jj = b & (J - 1u), t = b >> lj, i = t >> ph;
+      const uint32_t u = ((t & ((1u << ph) - 1u)) << (lr - ph)) + i;
+      const uint32_t su = tile_slot<LJ>(u, jj, lj);
+      uint32_t *const pu = at(su), *const pv = at(su ^ flip);
+      Fe<P> x, y, s;
+      if (in_tile) {
+        tile_load<P>(x, pu);
+        tile_load<P>(y, pv);
+      } else {
+        fe_load_cg<P>(x, src(u, jj));
+        fe_load_cg<P>(y, src(u + half, jj));
+      }
+      fe_add<P, 2>(s, x, y);
+      tile_store<P>(pu, s);
+      fe_sub<P, 2>(s, x, y);
+      if (i != 0) {
+        Fe<P> r;
+        fe_mul_tw<P, 2>(r, s, stage_entry<P>(A, i << ph));
+        tile_store<P>(pv, r);
+      } else {
+        tile_store<P>(pv, s);
+      }
+    }
+    in_tile = true;
+    __syncthreads();
+  }
+
+  // Last stage (twiddle 1): rows r and r + 1, r = bitrev(t) even, give outputs t and t + R/2; then the four-step factor
+  // (non-last), or the division by n, the post table and the canonical form (last), and the store.
+  auto emit = [&](Fe<P>& x, uint32_t t, uint32_t jj) {
+    const uint32_t pos = G.dst<P>(A, t, jj);
+    uint32_t* const out = A.dst + (size_t)pos * N;
+    if (A.last && A.div_log) fe_div_pow2<P>(x, x, A.div_log);
+    if (!A.last || A.post_table) {
+      Fe<P> v;
+      fe_mul_tw<P, 2>(v, x, A.last ? A.post_table + tw_offset<P>(pos) : step_entry<P>(A, G.jbase + jj, t));
+      if (A.last) fe_reduce_once<P>(v, v.l);
+      fe_store<P>(out, v);
+    } else {
+      fe_reduce_once<P>(x, x.l);
+      fe_store<P>(out, x);
+    }
+  };
+#pragma unroll 1
+  for (uint32_t b = threadIdx.x; b < (lr > 0 ? (R >> 1) << lj : J); b += nthr) {
+    const uint32_t jj = b & (J - 1u), t = b >> lj, r = bitrev_bits(t, lr);
+    Fe<P> x, y, s;
+    if (in_tile) {
+      const uint32_t su = tile_slot<LJ>(r, jj, lj);
+      tile_load<P>(x, at(su));
+      if (lr > 0) tile_load<P>(y, at(su ^ (1u << lj)));
+    } else {
+      fe_load_cg<P>(x, src(r, jj));
+      if (lr > 0) fe_load_cg<P>(y, src(r + 1u, jj));
+    }
+    if (lr > 0) {
+      fe_add<P, 2>(s, x, y);
+      fe_sub<P, 2>(y, x, y);
+      emit(s, t, jj);
+      emit(y, t + (R >> 1), jj);
+    } else {
+      emit(x, t, jj);
+    }
+  }
+  __syncthreads();
+}
+
 // Register cap of the per-pass kernel (255: no cap).  24 limbs: 128, 4 CTAs of 128 threads per SM; GB300, MNT4 2^18 /
-// 2^20 inverse in us: 302 / 1167 at 128, 310 / 1216 at 112, 316 / 1224 at 96, 306 / 1264 at 168 (3 CTAs, no spills).
-// 8 limbs: 64, 8 CTAs; uncapped it takes 84 registers (BLS 2^20 197 us; 190.5 at 80, 186.4 at 72, 184.3 at 64).
+// 2^20 in us: 294 / 1104 at 128, 298 / 1141 at 144, 297 / 1137 at 168 (3 CTAs).  8 limbs: 64, 8 CTAs; without the cap
+// an earlier form of the tile took 84 registers and BLS 2^20 197 us (190.5 at 80, 186.4 at 72, 184.3 at 64).
 template <class P>
 constexpr int pass_max_regs() {
   return P::N >= 16 ? 128 : P::N == 8 ? 64 : 255;
 }
 
-template <class P>
+template <class P, int LJ>
 __global__ void __maxnreg__(pass_max_regs<P>()) ntt_pass_kernel(const __grid_constant__ PassArgs A) {
   extern __shared__ uint4 gsn_smem[];
   uint32_t* sm = reinterpret_cast<uint32_t*>(gsn_smem);
-  for (uint64_t t = blockIdx.x; t < A.tiles; t += gridDim.x) ntt_tile<P>(A, t, sm);
+  for (uint64_t t = blockIdx.x; t < A.tiles; t += gridDim.x) {  // tiles < 2^28
+    if constexpr (P::N == 1) {
+      word_tile<P>(A, (uint32_t)t, sm);
+    } else {
+      field_tile<P, LJ>(A, (uint32_t)t, sm);
+    }
+  }
 }
 
 // Entry e of `out`: base^e, for e in [0, count), in the form fe_mul_tw takes.
@@ -250,8 +381,25 @@ __global__ void gen_powers_kernel(uint32_t* out, uint64_t count, Fe<P> base) {
   }
   const uint64_t end = (e0 + kPowChunk < count) ? e0 + kPowChunk : count;
   for (uint64_t e = e0; e < end; ++e) {
-    fe_store_tw<P>(out + e * tw_words<P>(), acc);
+    fe_store_tw<P>(out + tw_offset<P>((uint32_t)e), acc);
     fe_mul<P>(acc, acc, bm);
+  }
+}
+
+// Entry k 2^inner + j of `out`: entry (j k) << shift of `tw`.  One thread per 16-byte chunk, 8 threads a line.
+template <class P>
+__global__ void step_table_kernel(uint32_t* out, const uint32_t* tw, int r, int inner, int shift) {
+  constexpr int CH = P::N / 2;  // chunks per entry
+  const uint64_t count = (uint64_t)1 << (r + inner);
+  const uint64_t total = ((count + 7) >> 3) * CH * 8;
+  for (uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; t < total;
+       t += (uint64_t)gridDim.x * blockDim.x) {
+    const uint32_t c = (uint32_t)((t >> 3) % CH);
+    const uint32_t e = (uint32_t)((t >> 3) / CH * 8 + (t & 7));
+    if (e >= count) continue;
+    const uint32_t from = ((e & ((1u << inner) - 1u)) * (e >> inner)) << shift;
+    *reinterpret_cast<uint4*>(out + tw_offset<P>(e) + c * kTwChunk) =
+        *reinterpret_cast<const uint4*>(tw + tw_offset<P>(from) + c * kTwChunk);
   }
 }
 
@@ -394,6 +542,9 @@ __device__ __forceinline__ void job_pass_args(PassArgs& A, const BatchJob& J, in
   A.dst = A.last ? J.data : J.scratch;
   A.tw = J.tw;
   A.tw_log = J.tw_log;
+  A.stage_tw = J.stage_tw[pass];
+  A.stage_shift = J.stage_shift[pass];
+  A.step_tw = J.step_tw[pass];
   A.log_n = J.log_n;
   A.log_r = J.radix_log[pass];
   A.log_outer = outer;
@@ -432,7 +583,7 @@ __global__ void __maxnreg__(batch_max_regs<P>())
     const uint64_t w = work[t];
     const uint32_t job = (uint32_t)(w >> 32);
     const int pass = (int)((w >> 28) & 0xF);
-    const uint64_t tile = w & 0x0FFFFFFFull;
+    const uint32_t tile = (uint32_t)w & 0x0FFFFFFFu;
     if (threadIdx.x == 0) {
       const BatchJob& J = jobs[job];
       job_pass_args(s_args, J, pass);
@@ -451,7 +602,12 @@ __global__ void __maxnreg__(batch_max_regs<P>())
       }
     }
     __syncthreads();
-    ntt_tile<P>(s_args, tile, sm);  // ends with __syncthreads(); s_args is rewritten only after it
+    // each ends with __syncthreads(); s_args is rewritten only after it
+    if constexpr (P::N == 1) {
+      word_tile<P>(s_args, tile, sm);
+    } else {
+      field_tile<P, -1>(s_args, tile, sm);
+    }
     if (threadIdx.x == 0) {
       __threadfence();
       atomicAdd(&counters[1 + (uint64_t)job * kMaxPasses + pass], 1u);
@@ -466,8 +622,15 @@ constexpr uint64_t kGridPerSm = 64;
 template <class P>
 struct Kernels {
   static cudaError_t pass(const PassArgs& A, int block, cudaStream_t s) {
-    const size_t smem = ((size_t)1 << (A.log_r + A.log_j)) * P::N * sizeof(uint32_t);
-    auto k = ntt_pass_kernel<P>;
+    const size_t smem = tile_words(P::N, (uint64_t)1 << (A.log_r + A.log_j)) * sizeof(uint32_t);
+    auto k = ntt_pass_kernel<P, -1>;
+    if constexpr (P::N > 1) {
+      if (A.log_j == 2) k = ntt_pass_kernel<P, 2>;
+    }
+    if constexpr (P::N == 8) {
+      if (A.log_j == 0) k = ntt_pass_kernel<P, 0>;
+      if (A.log_j == 1) k = ntt_pass_kernel<P, 1>;
+    }
     if (smem > kDefaultSmemOptIn) {
       cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
       if (e != cudaSuccess) return e;
@@ -483,6 +646,18 @@ struct Kernels {
     const int block = 128;
     gen_powers_kernel<P><<<(unsigned)((threads + block - 1) / block), block, 0, s>>>(out, count, b);
     return cudaGetLastError();
+  }
+  static cudaError_t step_table(uint32_t* out, const uint32_t* tw, int r, int inner, int shift, cudaStream_t s) {
+    if constexpr (P::N == 1) {
+      return cudaErrorInvalidValue;  // its passes read `tw` itself
+    } else {
+      const int block = 256;
+      const uint64_t threads = ((uint64_t)1 << (r + inner)) * (P::N / 2);
+      const uint64_t grid =
+          std::min<uint64_t>(threads / block + 1, kGridPerSm * (uint64_t)current_device_sms());
+      step_table_kernel<P><<<(unsigned)grid, block, 0, s>>>(out, tw, r, inner, shift);
+      return cudaGetLastError();
+    }
   }
   static cudaError_t batch(const BatchJob* jobs_dev, const uint64_t* work_dev, uint64_t nwork,
                            uint32_t* counters_dev, uint32_t* status_dev, int grid, int block, size_t smem,

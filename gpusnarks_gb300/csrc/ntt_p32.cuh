@@ -1,7 +1,7 @@
 // Register-blocked NTT pass for the 32-bit field p = 3*2^30 + 1.
 //
-// Same four-step pass decomposition and tile geometry as ntt_tile
-// (ntt_common.h), but the tile's radix-2^r DIF runs in register sub-steps:
+// Same four-step pass decomposition and tile geometry as word_tile
+// (ntt_common.h, ntt_kernels.cuh), but the tile's radix-2^r DIF runs in register sub-steps:
 // each thread holds E = 2^ET rows x 4 adjacent columns (one uint4 per row)
 // and performs ET butterfly stages on them between two shared-memory round
 // trips, so a 2^12-point tile costs three exchanges instead of twelve.
@@ -179,7 +179,7 @@ __global__ void __launch_bounds__(512) ntt_p32_kernel(const __grid_constant__ P3
   const int lj = A.log_j;  // == LCG + 2
 
   for (uint64_t tile = blockIdx.x; tile < A.tiles; tile += gridDim.x) {
-    // --- tile geometry (see ntt_tile) ---
+    // --- tile geometry (see TileGeom) ---
     uint64_t base = 0, jbase = 0, rowpre = 0, obase = 0;
     int lo0 = 0;
     if (!A.last) {

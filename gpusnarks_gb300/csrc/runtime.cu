@@ -108,13 +108,13 @@ struct FieldLimits {
 static FieldLimits limits_of(const FieldOps& F) {
   switch (F.id) {
     case GSN_P32: return {11, 3, 512};
-    case GSN_BLS12_381_FR: return {9, 2, 256};
+    case GSN_BLS12_381_FR: return {8, 2, 128};
     default: return {8, 1, 128};
   }
 }
 
 size_t plan_smem_bytes(const FieldOps& F, const Plan& p, int pass) {
-  return ((size_t)1 << (p.radix_log[pass] + p.log_j[pass])) * F.limbs * sizeof(uint32_t);
+  return tile_words(F.limbs, (uint64_t)1 << (p.radix_log[pass] + p.log_j[pass])) * sizeof(uint32_t);
 }
 
 bool plan_valid(const FieldOps& F, const Plan& p) {
@@ -125,7 +125,7 @@ bool plan_valid(const FieldOps& F, const Plan& p) {
     for (int i = 0; i < p.npass; ++i)
       if (p.log_j[i] < 2 || p.log_j[i] > 4 || p.radix_log[i] < 2 || p.block[i] > 512) return false;
   } else if (p.kernel == kKernelRB) {
-    // 16-byte limb planes, at most 4 columns per tile (the swizzle), sub-steps of 4 or 8 rows
+    // at most 4 columns per tile, sub-steps of 4 or 8 rows: what tables that name this kernel hold
     if (F.id != GSN_BLS12_381_FR || (p.e_log != 2 && p.e_log != 3)) return false;
     for (int i = 0; i < p.npass; ++i)
       if (p.log_j[i] > 2 || p.radix_log[i] < 1 || p.block[i] > 256) return false;
@@ -232,17 +232,6 @@ Plan make_p32_plan(int log_n, int max_r, int log_j, int e_log) {
   return p;
 }
 
-Plan make_rb_plan(const FieldOps& F, int log_n, const int* radix_log, int npass, int log_j, int e_log) {
-  Plan p = make_split_plan(F, log_n, radix_log, npass, log_j, 256);
-  p.kernel = kKernelRB;
-  p.e_log = e_log;
-  for (int i = 0; i < p.npass; ++i) {
-    const int elems = 1 << (p.radix_log[i] + p.log_j[i]);
-    p.block[i] = std::max(32, std::min(256, elems >> std::min(e_log, p.radix_log[i])));
-  }
-  return p;
-}
-
 Plan plan_for(const FieldOps& F, int log_n, bool batched) {
   Plan p;
   // batched plans come from their own table: a persistent launch runs every
@@ -251,14 +240,6 @@ Plan plan_for(const FieldOps& F, int log_n, bool batched) {
   const int mode = batched ? 1 : 0;
   if (get_tuned_plan(F.id, log_n, &p, mode) && plan_valid(F, p) && (!batched || p.kernel == kKernelGeneric))
     return p;
-  if (F.id == GSN_BLS12_381_FR && !batched && log_n >= 2) {
-    // register-blocked passes of radix <= 2^10 over 4-column tiles
-    const int npass = std::max(1, (log_n + 9) / 10);
-    int radix[kMaxPasses] = {0, 0, 0, 0};
-    for (int i = 0; i < npass; ++i) radix[i] = log_n / npass + (i < log_n % npass ? 1 : 0);
-    p = make_rb_plan(F, log_n, radix, npass, 2, 3);
-    if (plan_valid(F, p)) return p;
-  }
   if (F.id == GSN_P32 && !batched && log_n >= 8) {
     // tiles of at most 2^14 elements (64 KB): J = 8 columns, radix <= 2^11
     p = make_p32_plan(log_n, 11, 3, 4);
@@ -276,12 +257,21 @@ struct DevBuf {
   size_t bytes = 0;
 };
 
+struct PassTables {
+  const uint32_t* stage[kMaxPasses];
+  const uint32_t* step[kMaxPasses];
+};
+
 // Every entry belongs to the device that was current when it was built: tables and scratch are keyed by
 // device as well, so a process that drives several GPUs never hands one GPU another's memory.
 struct TableCache {
   std::mutex mu;
   // (device, field, tw_log, root limbs) -> powers of the root
   std::map<std::tuple<int, int, int, std::string>, DevBuf> powers;
+  // (device, field, log2 of the order, r, root limbs) -> four-step factors of a pass of radix 2^r
+  std::map<std::tuple<int, int, int, int, std::string>, DevBuf> steps;
+  // (device, field, log_n, split, root limbs) -> the pass tables above, one lookup per call
+  std::map<std::tuple<int, int, int, std::string>, PassTables> passes;
   std::map<std::pair<int, cudaStream_t>, DevBuf> scratch;
   std::map<int, cudaStream_t> gen_stream;  // per device
 };
@@ -343,7 +333,7 @@ static int powers_table(const FieldOps& F, const uint32_t* base, int log_count, 
   if (!gen) GSN_CUDA(cudaStreamCreateWithFlags(&gen, cudaStreamNonBlocking));
   const uint64_t count = (uint64_t)1 << log_count;
   DevBuf b;
-  b.bytes = count * F.tw_words * sizeof(uint32_t);
+  b.bytes = table_words(F, count) * sizeof(uint32_t);
   int rc = dev_alloc(&b.p, b.bytes);
   if (rc) return rc;
   cudaError_t e = F.powers(static_cast<uint32_t*>(b.p), count, base, gen);
@@ -462,6 +452,109 @@ int resolve_p32_tables(const FieldOps& F, const Plan& plan, Tables* T) {
   return powers_table(F, hb, L - T->p32_lo_bits, &T->p32_hi);
 }
 
+void full_table_passes(const Plan& plan, Tables* T) {
+  for (int p = 0; p < plan.npass; ++p) {
+    T->stage[p] = T->tw;
+    T->stage_shift[p] = T->tw_log - plan.radix_log[p];
+    T->step[p] = nullptr;
+  }
+}
+
+// Entry k 2^inner + j = w^(j k), w = (root of `tw`)^(2^shift) of order 2^(r + inner); key_root names w.
+static int step_table(const FieldOps& F, const uint32_t* tw, int shift, int r, int inner, const uint32_t* key_root,
+                      const uint32_t** out) {
+  TableCache& C = cache();
+  const int dev = current_device();
+  std::lock_guard<std::mutex> g(C.mu);
+  auto key = std::make_tuple(dev, F.id, r + inner, r, limbs_key(key_root, F.limbs));
+  auto it = C.steps.find(key);
+  if (it == C.steps.end()) {
+    cudaStream_t& gen = C.gen_stream[dev];
+    if (!gen) GSN_CUDA(cudaStreamCreateWithFlags(&gen, cudaStreamNonBlocking));
+    DevBuf b;
+    b.bytes = table_words(F, (uint64_t)1 << (r + inner)) * sizeof(uint32_t);
+    int rc = dev_alloc(&b.p, b.bytes);
+    if (rc) return rc;
+    cudaError_t e = F.step_table(static_cast<uint32_t*>(b.p), tw, r, inner, shift, gen);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(gen);
+    if (e != cudaSuccess) {
+      dev_free(b.p);
+      return cuda_fail(e, "four-step table");
+    }
+    count_launches(1);
+    it = C.steps.emplace(key, b).first;
+  }
+  *out = static_cast<const uint32_t*>(it->second.p);
+  return GSN_OK;
+}
+
+int resolve_pass_tables(const FieldOps& F, const Plan& plan, Tables* T, cudaStream_t s) {
+  full_table_passes(plan, T);
+  if (F.limbs == 1) return GSN_OK;
+  TableCache& C = cache();
+  const int dev = current_device(), L = plan.log_n;
+  std::string tail = limbs_key(T->root, F.limbs);
+  for (int p = 0; p < plan.npass; ++p) tail.push_back((char)plan.radix_log[p]);
+  const auto key = std::make_tuple(dev, F.id, L, tail);
+  PassTables t;
+  bool found = false;
+  {
+    std::lock_guard<std::mutex> g(C.mu);
+    auto it = C.passes.find(key);
+    if (it != C.passes.end()) {
+      t = it->second;
+      found = true;
+    }
+  }
+  if (!found) {
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (s && cudaStreamIsCapturing(s, &cap) != cudaSuccess) cudaGetLastError();
+    if (cap != cudaStreamCaptureStatusNone) return GSN_OK;
+    uint32_t def[kMaxLimbs];
+    default_root(F, L, def);
+    const bool is_def = std::memcmp(T->root, def, sizeof(uint32_t) * F.limbs) == 0;
+    auto power = [&](int order_log, uint32_t* out) {  // root^(2^(L - order_log))
+      if (is_def) {
+        default_root(F, order_log, out);
+      } else {
+        F.pow(T->root, (uint64_t)1 << (L - order_log), out);
+      }
+    };
+    int outer = 0;
+    for (int p = 0; p < plan.npass; ++p) {
+      const int r = plan.radix_log[p], left = L - outer;
+      uint32_t w[kMaxLimbs];
+      t.stage[p] = t.step[p] = nullptr;
+      int rc = GSN_OK;
+      if (r >= 1) {
+        power(r, w);
+        rc = powers_table(F, w, r - 1, &t.stage[p]);
+      }
+      if (!rc && p < plan.npass - 1) {
+        power(left, w);
+        rc = step_table(F, T->tw, T->tw_log - left, r, left - r, w, &t.step[p]);
+      }
+      if (rc == GSN_ERR_NOMEM) return GSN_OK;
+      if (rc) return rc;
+      outer += r;
+    }
+    std::lock_guard<std::mutex> g(C.mu);
+    C.passes[key] = t;
+  }
+  for (int p = 0; p < plan.npass; ++p) {
+    if (t.stage[p]) {
+      T->stage[p] = t.stage[p];
+      T->stage_shift[p] = 0;
+    }
+    T->step[p] = t.step[p];
+  }
+  return GSN_OK;
+}
+
+int resolve_plan_tables(const FieldOps& F, const Plan& plan, Tables* T, cudaStream_t s) {
+  return plan.kernel == kKernelP32 ? resolve_p32_tables(F, plan, T) : resolve_pass_tables(F, plan, T, s);
+}
+
 int scratch_for(cudaStream_t s, size_t bytes, uint32_t** out) {
   TableCache& C = cache();
   const int dev = current_device();
@@ -519,7 +612,6 @@ static int enqueue_p32(const Plan& plan, const Tables& T, uint32_t* data, uint32
 int enqueue_ntt(const FieldOps& F, const Plan& plan, const Tables& T, uint32_t* data, uint32_t* scratch,
                 cudaStream_t s) {
   if (plan.kernel == kKernelP32) return enqueue_p32(plan, T, data, scratch, s);
-  const bool rb = plan.kernel == kKernelRB;
   PassArgs A;
   std::memset(&A, 0, sizeof(A));
   A.tw = T.tw;
@@ -539,10 +631,13 @@ int enqueue_ntt(const FieldOps& F, const Plan& plan, const Tables& T, uint32_t* 
     A.log_inner = plan.log_n - outer - plan.radix_log[p];
     A.log_j = plan.log_j[p];
     A.tiles = (uint64_t)1 << (plan.log_n - A.log_r - A.log_j);
+    A.stage_tw = T.stage[p];
+    A.stage_shift = T.stage_shift[p];
+    A.step_tw = T.step[p];
     A.pre_table = A.first ? T.pre_table : nullptr;
     A.post_table = A.last ? T.post_table : nullptr;
     A.div_log = A.last ? T.div_log : 0;
-    cudaError_t e = rb ? F.pass_rb(A, plan.e_log, plan.block[p], s) : F.pass(A, plan.block[p], s);
+    cudaError_t e = F.pass(A, plan.block[p], s);
     if (e != cudaSuccess) return cuda_fail(e, "NTT pass launch");
     count_launches(1);
     outer += plan.radix_log[p];
@@ -578,10 +673,8 @@ static int ntt_impl(int field, uint32_t* data, uint32_t log_n, const uint32_t* o
     const FieldLimits L = limits_of(*F);
     plan = make_plan(*F, (int)log_n, L.max_r, L.target_j, L.max_block);
   }
-  if (plan.kernel == kKernelP32) {
-    rc = resolve_p32_tables(*F, plan, &T);
-    if (rc) return rc;
-  }
+  rc = resolve_plan_tables(*F, plan, &T, s);
+  if (rc) return rc;
   if (plan.npass > 1 && !scratch) {
     rc = scratch_for(s, ((size_t)1 << log_n) * F->limbs * sizeof(uint32_t), &scratch);
     if (rc) return rc;
@@ -944,7 +1037,9 @@ int gsn_prepare(int field, uint32_t log_n, const uint32_t* omega) {
   const FieldOps* F = field_ops(field);
   if (!F) return set_error(GSN_ERR_FIELD, "unknown field %d", field);
   Tables T;
-  return resolve_tables(*F, log_n, omega, GSN_FORWARD, nullptr, &T, nullptr);
+  int rc = resolve_tables(*F, log_n, omega, GSN_FORWARD, nullptr, &T, nullptr);
+  if (rc || F->limbs == 1) return rc;
+  return resolve_pass_tables(*F, plan_for(*F, (int)log_n), &T, nullptr);
 }
 
 int gsn_pointwise_mul(int field, uint32_t* a, const uint32_t* b, uint64_t n, void* stream) {
@@ -1026,6 +1121,9 @@ int gsn_release_caches(void) {
   std::lock_guard<std::mutex> g(C.mu);
   for (auto& kv : C.powers) dev_free(kv.second.p);
   C.powers.clear();
+  for (auto& kv : C.steps) dev_free(kv.second.p);
+  C.steps.clear();
+  C.passes.clear();
   for (auto& kv : C.scratch) dev_free(kv.second.p);
   C.scratch.clear();
   return GSN_OK;

@@ -37,8 +37,8 @@ struct Plan {
   int log_j[kMaxPasses] = {0, 0, 0, 0};
   int block[kMaxPasses] = {0, 0, 0, 0};
   int kernel = kKernelGeneric;  // kKernelP32: register-blocked 32-bit pass (ntt_p32.cuh);
-                                // kKernelRB: register-blocked multi-limb pass (ntt_rb.cuh)
-  int e_log = 4;                // kKernelP32 / kKernelRB: rows per thread per register sub-step (log2)
+                                // kKernelRB: named by saved tables for the 8-limb field; runs the generic pass
+  int e_log = 4;                // kKernelP32: rows per thread per register sub-step (log2)
 };
 
 // Register-blocked 32-bit pass launcher (ntt_f_p32.cu).
@@ -48,9 +48,6 @@ cudaError_t launch_p32_pass(const P32Args& A, int e_log, int block, int grid_cap
 // loaded.
 Plan plan_for(const FieldOps& F, int log_n, bool batched = false);
 Plan make_p32_plan(int log_n, int max_r, int log_j, int e_log);
-// Register-blocked multi-limb plan over an explicit radix split: 2^log_j columns per tile (<= 4), 2^e_log
-// rows per thread per sub-step.
-Plan make_rb_plan(const FieldOps& F, int log_n, const int* radix_log, int npass, int log_j, int e_log);
 // Heuristic plan with explicit limits (used by the autotuner's candidate set).
 Plan make_plan(const FieldOps& F, int log_n, int max_r, int target_j, int max_block);
 // The same tile widths and threads for an explicit split of log_n into npass radices.
@@ -70,7 +67,11 @@ struct Tables {
   const uint32_t* post_table = nullptr;
   int inverse = 0;
   int div_log = 0;                 // inverse: the outputs are divided by 2^div_log = n
-  uint32_t root[kMaxLimbs] = {0};  // canonical root actually used (omega^-1 when inverse)
+  uint32_t root[kMaxLimbs] = {0};  // canonical forward root
+  // per pass, filled by resolve_pass_tables / full_table_passes (PassArgs::stage_tw, step_tw)
+  const uint32_t* stage[kMaxPasses] = {nullptr, nullptr, nullptr, nullptr};
+  int stage_shift[kMaxPasses] = {0, 0, 0, 0};
+  const uint32_t* step[kMaxPasses] = {nullptr, nullptr, nullptr, nullptr};
   // register-blocked 32-bit pass tables, filled by resolve_p32_tables
   const uint32_t* p32_tile[kMaxPasses] = {nullptr, nullptr, nullptr, nullptr};
   uint32_t p32_pre_const = 0;  // inverse: n^-1 R
@@ -85,6 +86,17 @@ bool find_default_twiddles(const FieldOps& F, int log_n, const uint32_t** tw, in
 
 // Compact per-radix and two-level four-step tables for a kKernelP32 plan.
 int resolve_p32_tables(const FieldOps& F, const Plan& plan, Tables* T);
+
+// Pass tables read from the full twiddle table alone: no allocation, no launch.
+void full_table_passes(const Plan& plan, Tables* T);
+
+// Pass tables of a multi-limb plan: the stage twiddles of each radix and the four-step
+// factors in the order the tiles take them, built once per (root, split) and cached.  While `s` is capturing, or
+// when there is no memory for them, a plan whose tables are not there yet reads the full table instead.
+int resolve_pass_tables(const FieldOps& F, const Plan& plan, Tables* T, cudaStream_t s);
+
+// The tables a plan's kernel needs beyond resolve_tables.
+int resolve_plan_tables(const FieldOps& F, const Plan& plan, Tables* T, cudaStream_t s);
 
 // Validates arguments and resolves (and caches) all tables for a transform.
 int resolve_tables(const FieldOps& F, uint32_t log_n, const uint32_t* omega, int dir, const uint32_t* shift,

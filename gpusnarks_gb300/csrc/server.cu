@@ -245,7 +245,7 @@ void launch_single(gsn_server* S, Slot& sl, uint64_t id) {
   Tables T;
   int rc = resolve_tables(*q.F, q.r.log_n, nullptr, q.r.dir, q.has_shift ? q.shift : nullptr, &T, sl.stream);
   const Plan plan = plan_for(*q.F, (int)q.r.log_n);
-  if (!rc && plan.kernel == kKernelP32) rc = resolve_p32_tables(*q.F, plan, &T);
+  if (!rc) rc = resolve_plan_tables(*q.F, plan, &T, sl.stream);
   uint32_t* scratch = q.has_scratch ? dptr(S, q.scratch_off) : nullptr;
   if (!rc && plan.npass > 1 && !scratch) rc = set_error(GSN_ERR_STATE, "request admitted without scratch");
   if (!rc) rc = enqueue_ntt(*q.F, plan, T, dptr(S, q.data_off), scratch, sl.stream);
@@ -533,6 +533,7 @@ int gsn_server_warmup(gsn_server* S, int field, uint32_t lo, uint32_t hi) {
     for (int dir = GSN_FORWARD; dir <= GSN_COSET_INVERSE; ++dir) {
       Tables T;
       int rc = resolve_tables(*F, k, nullptr, dir, nullptr, &T, nullptr);
+      if (!rc) rc = resolve_pass_tables(*F, plan_for(*F, (int)k, /*batched=*/true), &T, nullptr);
       if (rc) return rc;
     }
   }
