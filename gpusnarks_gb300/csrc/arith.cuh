@@ -409,7 +409,8 @@ __device__ __forceinline__ void fe_load(Fe<P>& r, const uint32_t* p) {
 }
 
 // Load that bypasses L1 (ld.global.cg): used for data another CTA of the same
-// launch may have written (the batched kernel reads earlier passes' output).
+// launch may have written (the batched kernel reads earlier passes' output),
+// or a kernel that this one overlaps (chain.cuh).
 template <class P>
 __device__ __forceinline__ void fe_load_cg(Fe<P>& r, const uint32_t* p) {
   constexpr int N = P::N;

@@ -11,6 +11,7 @@
 
 #include <algorithm>
 #include <cstring>
+#include <map>
 #include <numeric>
 #include <vector>
 
@@ -66,17 +67,26 @@ int plan_batch(const FieldOps& F, const gsn_batch_job* jobs, size_t njobs, Batch
   out->block = 0;
   out->smem = 0;
   out->elements = 0;
+  std::map<std::pair<uint32_t, int32_t>, std::pair<Tables, Plan>> seen;
+  std::pair<Tables, Plan> own;
   for (size_t i = 0; i < njobs; ++i) {
     const gsn_batch_job& u = jobs[i];
     if (!u.data || reinterpret_cast<uintptr_t>(u.data) % align)
       return set_error(GSN_ERR_ARG, "job %zu: null or misaligned data pointer", i);
-    Tables T;
-    int rc = resolve_tables(F, u.log_n, u.omega, u.dir, u.shift, &T, nullptr);
-    if (rc) return rc;
-    Plan p = force ? *force : plan_for(F, (int)u.log_n, /*batched=*/true);
-    if (force && p.log_n != (int)u.log_n) return set_error(GSN_ERR_ARG, "forced plan size mismatch");
-    rc = resolve_pass_tables(F, p, &T, nullptr);
-    if (rc) return rc;
+    // jobs of one size and direction with the default root and shift share their plan and tables: one look-up each
+    const bool plain = !u.omega && !u.shift;
+    auto it = plain ? seen.find(std::make_pair(u.log_n, u.dir)) : seen.end();
+    if (it == seen.end()) {
+      int rc = resolve_tables(F, u.log_n, u.omega, u.dir, u.shift, &own.first, nullptr);
+      if (rc) return rc;
+      own.second = force ? *force : plan_for(F, (int)u.log_n, /*batched=*/true);
+      if (force && own.second.log_n != (int)u.log_n) return set_error(GSN_ERR_ARG, "forced plan size mismatch");
+      rc = resolve_pass_tables(F, own.second, &own.first, nullptr);
+      if (rc) return rc;
+      if (plain) it = seen.emplace(std::make_pair(u.log_n, u.dir), own).first;
+    }
+    const Tables& T = plain ? it->second.first : own.first;
+    const Plan& p = plain ? it->second.second : own.second;
     out->plans[i] = p;
     BatchJob& J = out->jobs[i];
     std::memset(&J, 0, sizeof(J));

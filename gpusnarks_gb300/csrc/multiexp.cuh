@@ -24,6 +24,7 @@
 #include <cstdlib>
 
 #include "arith.cuh"
+#include "chain.cuh"
 #include "ntt_common.h"
 
 namespace gsn {
@@ -154,10 +155,11 @@ __device__ __forceinline__ void block_sum(Fe<P>& x, uint32_t* sm) {
 // First launch: per-block partial sums of a[i] * b[i] (grid-stride over i), canonical, in `partial`.
 // PF: load the next element's operands before the current product (more registers, overlapped latency).
 template <class P, bool PF>
-__global__ void __launch_bounds__(256) multiexp_kernel(const uint32_t* __restrict__ a, const uint32_t* __restrict__ b,
-                                                       uint64_t n, uint32_t* __restrict__ partial, Fe<P> fix) {
+__global__ void __launch_bounds__(256) multiexp_kernel(const uint32_t* a, const uint32_t* b, uint64_t n,
+                                                       uint32_t* partial, Fe<P> fix) {
   constexpr int N = P::N;
   __shared__ uint32_t sm[8 * N];
+  chain_wait();
   uint32_t T[2 * N + 1];
 #pragma unroll
   for (int k = 0; k <= 2 * N; ++k) T[k] = 0u;
@@ -195,29 +197,30 @@ __global__ void __launch_bounds__(256) multiexp_kernel(const uint32_t* __restric
   } else if constexpr (!PF) {
     for (; i < n; i += stride) {
       Fe<P> x, y;
-      fe_load<P>(x, a + i * N);
-      fe_load<P>(y, b + i * N);
+      fe_load_cg<P>(x, a + i * N);
+      fe_load_cg<P>(y, b + i * N);
       mul_acc<N>(T, x.l, y.l);
     }
   } else {
     // the next element's operands are loaded before the current product, so their memory latency overlaps it
     Fe<P> x, y;
     if (i < n) {
-      fe_load<P>(x, a + i * N);
-      fe_load<P>(y, b + i * N);
+      fe_load_cg<P>(x, a + i * N);
+      fe_load_cg<P>(y, b + i * N);
     }
     for (; i < n; i += stride) {
       const uint64_t next = i + stride;
       Fe<P> xn, yn;
       if (next < n) {
-        fe_load<P>(xn, a + next * N);
-        fe_load<P>(yn, b + next * N);
+        fe_load_cg<P>(xn, a + next * N);
+        fe_load_cg<P>(yn, b + next * N);
       }
       mul_acc<N>(T, x.l, y.l);
       x = xn;
       y = yn;
     }
   }
+  chain_next();
   Fe<P> r;
   reduce_wide<P>(r, T);
   fe_mul<P>(r, r, fix);
@@ -227,16 +230,16 @@ __global__ void __launch_bounds__(256) multiexp_kernel(const uint32_t* __restric
 
 // Second launch (one block): out = sum of the `count` partials.
 template <class P>
-__global__ void __launch_bounds__(256) multiexp_final_kernel(const uint32_t* __restrict__ partial, int count,
-                                                             uint32_t* __restrict__ out) {
+__global__ void __launch_bounds__(256) multiexp_final_kernel(const uint32_t* partial, int count, uint32_t* out) {
   constexpr int N = P::N;
   __shared__ uint32_t sm[8 * N];
+  chain_wait();
   Fe<P> x;
 #pragma unroll
   for (int j = 0; j < N; ++j) x.l[j] = 0u;
   for (int k = threadIdx.x; k < count; k += blockDim.x) {
     Fe<P> y;
-    fe_load<P>(y, partial + (uint64_t)k * N);
+    fe_load_cg<P>(y, partial + (uint64_t)k * N);
     fe_add<P>(x, x, y);
   }
   block_sum<P>(x, sm);
@@ -282,12 +285,10 @@ struct MultiexpKernels {
                          uint32_t* out, const uint32_t* fix_limbs, cudaStream_t s) {
     Fe<P> fix;
     for (int j = 0; j < P::N; ++j) fix.l[j] = fix_limbs[j];
-    if (prefetch()) mexp::multiexp_kernel<P, true><<<grid, mexp::multiexp_block<P>(), 0, s>>>(a, b, n, partial, fix);
-    else mexp::multiexp_kernel<P, false><<<grid, mexp::multiexp_block<P>(), 0, s>>>(a, b, n, partial, fix);
-    cudaError_t e = cudaGetLastError();
+    auto k = prefetch() ? mexp::multiexp_kernel<P, true> : mexp::multiexp_kernel<P, false>;
+    cudaError_t e = launch_chained(k, (unsigned)grid, mexp::multiexp_block<P>(), 0, s, a, b, n, partial, fix);
     if (e != cudaSuccess) return e;
-    mexp::multiexp_final_kernel<P><<<1, 256, 0, s>>>(partial, grid, out);
-    return cudaGetLastError();
+    return launch_chained(mexp::multiexp_final_kernel<P>, 1, 256, 0, s, partial, grid, out);
   }
 };
 

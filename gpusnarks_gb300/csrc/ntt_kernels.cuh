@@ -14,6 +14,7 @@
 #include <cstdint>
 
 #include "arith.cuh"
+#include "chain.cuh"
 #include "ntt_common.h"
 
 namespace gsn {
@@ -179,6 +180,7 @@ __device__ void word_tile(const PassArgs& A, uint32_t tile, uint32_t* sm) {
   for (int ph = A.first && A.pre_table ? -1 : 0; ph <= lr; ++ph) {
     if (lr > 0 && ph == lr - 1) continue;  // fused into ph = lr; uniform across the block
     const bool stage = ph >= 0 && ph < lr;
+    if (ph == lr) chain_next();
     const uint32_t count = stage ? (R >> 1) * J : R * J;
     for (uint32_t b = threadIdx.x; b < count; b += nthr) {
       const uint32_t jj = b & (J - 1u), t = b >> lj;
@@ -314,6 +316,7 @@ __device__ __forceinline__ void field_tile(const PassArgs& A, uint32_t tile, uin
       fe_store<P>(out, x);
     }
   };
+  chain_next();
 #pragma unroll 1
   for (uint32_t b = threadIdx.x; b < (lr > 0 ? (R >> 1) << lj : J); b += nthr) {
     const uint32_t jj = b & (J - 1u), t = b >> lj, r = bitrev_bits(t, lr);
@@ -350,6 +353,7 @@ template <class P, int LJ>
 __global__ void __maxnreg__(pass_max_regs<P>()) ntt_pass_kernel(const __grid_constant__ PassArgs A) {
   extern __shared__ uint4 gsn_smem[];
   uint32_t* sm = reinterpret_cast<uint32_t*>(gsn_smem);
+  chain_wait();
   for (uint64_t t = blockIdx.x; t < A.tiles; t += gridDim.x) {  // tiles < 2^28
     if constexpr (P::N == 1) {
       word_tile<P>(A, (uint32_t)t, sm);
@@ -455,10 +459,11 @@ __global__ void fill_random_kernel(uint32_t* out, uint64_t n, uint64_t seed) {
 //           <-> the little-endian im_rep of cuda/device_field.h:75)
 template <class P>
 __global__ void convert_kernel(uint32_t* data, uint64_t n, int mode) {
+  chain_wait();
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
        i += (uint64_t)gridDim.x * blockDim.x) {
     Fe<P> x, r;
-    fe_load<P>(x, data + i * P::N);
+    fe_load_cg<P>(x, data + i * P::N);
     if (mode == 0) {
       fe_to_mont<P>(r, x);
     } else if (mode == 1) {
@@ -478,11 +483,12 @@ __global__ void convert_kernel(uint32_t* data, uint64_t n, int mode) {
 // products, the second by R^2.
 template <class P>
 __global__ void pointwise_mul_kernel(uint32_t* a, const uint32_t* b, uint64_t n) {
+  chain_wait();
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
        i += (uint64_t)gridDim.x * blockDim.x) {
     Fe<P> x, y, r;
-    fe_load<P>(x, a + i * P::N);
-    fe_load<P>(y, b + i * P::N);
+    fe_load_cg<P>(x, a + i * P::N);
+    fe_load_cg<P>(y, b + i * P::N);
     fe_mul<P>(r, x, y);
     fe_to_mont<P>(r, r);
     fe_store<P>(a + i * P::N, r);
@@ -495,15 +501,16 @@ __global__ void pointwise_mul_kernel(uint32_t* a, const uint32_t* b, uint64_t n)
 //   (mont(a, b) - mont(c, 1)) = (a b - c) / R  and  mont(that, z R^2) = (a b - c) z.
 template <class P>
 __global__ void coset_quotient_kernel(uint32_t* a, const uint32_t* b, const uint32_t* c, uint64_t n, Fe<P> zr2) {
+  chain_wait();
   Fe<P> one;
 #pragma unroll
   for (int j = 0; j < P::N; ++j) one.l[j] = j == 0 ? 1u : 0u;
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
        i += (uint64_t)gridDim.x * blockDim.x) {
     Fe<P> x, y, z, t, u;
-    fe_load<P>(x, a + i * P::N);
-    fe_load<P>(y, b + i * P::N);
-    fe_load<P>(z, c + i * P::N);
+    fe_load_cg<P>(x, a + i * P::N);
+    fe_load_cg<P>(y, b + i * P::N);
+    fe_load_cg<P>(z, c + i * P::N);
     fe_mul<P>(t, x, y);
     fe_mul<P>(u, z, one);
     fe_sub<P>(t, t, u);
@@ -636,8 +643,7 @@ struct Kernels {
       if (e != cudaSuccess) return e;
     }
     const uint64_t grid = A.tiles < (1u << 20) ? A.tiles : (1u << 20);
-    k<<<(unsigned)grid, block, smem, s>>>(A);
-    return cudaGetLastError();
+    return launch_chained(k, (unsigned)grid, (unsigned)block, smem, s, A);
   }
   static cudaError_t powers(uint32_t* out, uint64_t count, const uint32_t* base_canon, cudaStream_t s) {
     Fe<P> b;
@@ -683,8 +689,7 @@ struct Kernels {
     uint64_t grid = (n + block - 1) / block;
     if (grid > kGridPerSm * (uint64_t)current_device_sms()) grid = kGridPerSm * (uint64_t)current_device_sms();
     if (grid == 0) return cudaSuccess;
-    convert_kernel<P><<<(unsigned)grid, block, 0, s>>>(data, n, mode);
-    return cudaGetLastError();
+    return launch_chained(convert_kernel<P>, (unsigned)grid, block, 0, s, data, n, mode);
   }
   static cudaError_t fill(uint32_t* out, uint64_t n, uint64_t seed, cudaStream_t s) {
     const int block = 256;
@@ -698,8 +703,7 @@ struct Kernels {
     const int block = 256;
     uint64_t grid = (n + block - 1) / block;
     if (grid > kGridPerSm * (uint64_t)current_device_sms()) grid = kGridPerSm * (uint64_t)current_device_sms();
-    pointwise_mul_kernel<P><<<(unsigned)grid, block, 0, s>>>(a, b, n);
-    return cudaGetLastError();
+    return launch_chained(pointwise_mul_kernel<P>, (unsigned)grid, block, 0, s, a, b, n);
   }
   static cudaError_t quotient(uint32_t* a, const uint32_t* b, const uint32_t* c, uint64_t n, const uint32_t* zr2,
                               cudaStream_t s) {
@@ -709,8 +713,7 @@ struct Kernels {
     uint64_t grid = (n + block - 1) / block;
     if (grid > kGridPerSm * (uint64_t)current_device_sms()) grid = kGridPerSm * (uint64_t)current_device_sms();
     if (grid == 0) return cudaSuccess;
-    coset_quotient_kernel<P><<<(unsigned)grid, block, 0, s>>>(a, b, c, n, z);
-    return cudaGetLastError();
+    return launch_chained(coset_quotient_kernel<P>, (unsigned)grid, block, 0, s, a, b, c, n, z);
   }
 };
 

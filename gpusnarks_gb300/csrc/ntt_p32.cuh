@@ -177,6 +177,7 @@ __global__ void __launch_bounds__(512) ntt_p32_kernel(const __grid_constant__ P3
   const int r = A.log_r;
   const uint32_t R = 1u << r;
   const int lj = A.log_j;  // == LCG + 2
+  chain_wait();
 
   for (uint64_t tile = blockIdx.x; tile < A.tiles; tile += gridDim.x) {
     // --- tile geometry (see TileGeom) ---
@@ -242,6 +243,7 @@ __global__ void __launch_bounds__(512) ntt_p32_kernel(const __grid_constant__ P3
     }
 
     // --- four-step twiddle (or post table) and store ---
+    if (tile + gridDim.x >= A.tiles) chain_next();
     for (uint32_t v = threadIdx.x; v < R * CG; v += blockDim.x) {
       const uint32_t k = v >> LCG, cg = v & (CG - 1);
       uint4 x = sm_ld<LCG>(sm, brev(k, r), cg);
@@ -417,6 +419,7 @@ __global__ void __launch_bounds__(512) __maxnreg__(p32::max_regs<ET>()) ntt_p32_
   extern __shared__ uint4 gsn_smem[];
   constexpr uint32_t CG = 1u << LCG;
   constexpr uint32_t R = 1u << RL;
+  chain_wait();
   {
     uint4* const buf0 = gsn_smem;
     uint4* const buf1 = gsn_smem + R * CG;
@@ -447,6 +450,7 @@ __global__ void __launch_bounds__(512) __maxnreg__(p32::max_regs<ET>()) ntt_p32_
         __syncthreads();
       }
       substeps_fixed<RL, ET, LCG, 0>(cur, A.tw_tile);  // ends with __syncthreads()
+      if (next >= A.tiles) chain_next();
       store_fourstep<RL, LCG>(A, cur, base, jbase);
       __syncthreads();
       base = nbase;
@@ -465,6 +469,7 @@ __global__ void __launch_bounds__(512) __maxnreg__(p32::max_regs<ET>()) ntt_p32_
   constexpr uint32_t CG = 1u << LCG;
   constexpr uint32_t R = 1u << RL;
   constexpr int lj = LCG + 2;
+  chain_wait();
 
   for (uint64_t tile = blockIdx.x; tile < A.tiles; tile += gridDim.x) {
     uint64_t base = 0, jbase = 0, rowpre = 0, obase = 0;
@@ -513,6 +518,7 @@ __global__ void __launch_bounds__(512) __maxnreg__(p32::max_regs<ET>()) ntt_p32_
 
     substeps_fixed<RL, ET, LCG, 0>(sm, A.tw_tile);  // ends with __syncthreads()
 
+    if (tile + gridDim.x >= A.tiles) chain_next();
     if (!A.last) {
       store_fourstep<RL, LCG>(A, sm, base, jbase);
     } else {
@@ -554,8 +560,7 @@ cudaError_t launch_kernel(K k, const P32Args& A, int block, int grid_cap, cudaSt
     if (e != cudaSuccess) return e;
   }
   const uint64_t grid = A.tiles < (uint64_t)grid_cap ? A.tiles : (uint64_t)grid_cap;
-  k<<<(unsigned)grid, block, smem, s>>>(B);
-  return cudaGetLastError();
+  return launch_chained(k, (unsigned)grid, (unsigned)block, smem, s, B);
 }
 inline bool pipe_enabled() {
   static const int on = [] {
