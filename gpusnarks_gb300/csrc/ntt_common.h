@@ -34,9 +34,14 @@ int current_device_sms();
 constexpr int kMaxPasses = 4;
 constexpr int kMaxLimbs = 24;
 
+// Arrays of one size that a pass transforms alike, array blockIdx.y in each block row of the grid.
+constexpr int kMaxArrays = 3;
+struct PassArrays {
+  const uint32_t* src[kMaxArrays];
+  uint32_t* dst[kMaxArrays];
+};
+
 struct PassArgs {
-  const uint32_t* src;
-  uint32_t* dst;
   const uint32_t* tw;         // entry e: (root of order 2^tw_log)^e, e in [0, 2^tw_log), as fe_mul_tw takes it
   const uint32_t* stage_tw;   // entry e << stage_shift: w_R^e for the pass radix R, e < R/2 (`tw` or a table of its own)
   const uint32_t* step_tw;    // entry k 2^log_inner + j': w^(outer j' k), the four-step factors in the order the tile
@@ -58,6 +63,7 @@ struct PassArgs {
   int npass;
   int radix_log[kMaxPasses];
   int div_log;                // last pass: X[k] /= 2^div_log before the post table (n^-1 of an inverse); 0: none
+  PassArrays arrays;          // the batched kernel's: its job's, at 0
 };
 
 // One job of the batched / served path: an in-place transform of one
@@ -83,8 +89,7 @@ struct BatchJob {
 // Arguments of the register-blocked 32-bit pass (ntt_p32.cuh).  Tables are
 // built for the root actually used (omega^-1 for inverse transforms).
 struct P32Args {
-  const uint32_t* src;
-  uint32_t* dst;
+  PassArrays arrays;
   const uint32_t* tw_tile;     // omega_R^e * R, e < 2^(log_r - 1)
   const uint32_t* tw_lo;       // omega_n^e * R, e < 2^lo_bits
   const uint32_t* tw_hi;       // omega_n^(e << lo_bits) * R

@@ -166,7 +166,7 @@ struct TileGeom {
 //                  product) fused with the four-step twiddle (non-last) or the division by n and the post table (last)
 //                  and the store: one barrier and one shared-memory store of the tile fewer per pass.
 template <class P>
-__device__ void word_tile(const PassArgs& A, uint32_t tile, uint32_t* sm) {
+__device__ void word_tile(const PassArgs& A, unsigned array, uint32_t tile, uint32_t* sm) {
   static_assert(P::N == 1, "one limb");
   const int lr = A.log_r, lj = A.log_j;
   const uint32_t R = 1u << lr, J = 1u << lj, nthr = blockDim.x;
@@ -174,7 +174,7 @@ __device__ void word_tile(const PassArgs& A, uint32_t tile, uint32_t* sm) {
   for (uint32_t e = threadIdx.x; e < R * J; e += nthr) {
     // input rows are contiguous on the last pass
     const uint32_t k = !A.last ? e >> lj : e & (R - 1u), jj = !A.last ? e & (J - 1u) : e >> lr;
-    sm[(k << lj) + jj] = __ldcg(A.src + G.src(A, k, jj));
+    sm[(k << lj) + jj] = __ldcg(A.arrays.src[array] + G.src(A, k, jj));
   }
   __syncthreads();
   for (int ph = A.first && A.pre_table ? -1 : 0; ph <= lr; ++ph) {
@@ -211,7 +211,7 @@ __device__ void word_tile(const PassArgs& A, uint32_t tile, uint32_t* sm) {
           x.l[0] = sm[jj];
         }
         const uint32_t pos = G.dst<P>(A, t, jj);
-        out = A.dst + pos;
+        out = A.arrays.dst[array] + pos;
         if (!A.last) {
           w = step_entry<P>(A, G.jbase + jj, t);
         } else {
@@ -242,14 +242,14 @@ __device__ void word_tile(const PassArgs& A, uint32_t tile, uint32_t* sm) {
 // Values stay in [0, 2p) between the phases and the passes (a product's last subtraction is left out) until the last
 // pass's store.
 template <class P, int LJ>
-__device__ __forceinline__ void field_tile(const PassArgs& A, uint32_t tile, uint32_t* sm) {
+__device__ __forceinline__ void field_tile(const PassArgs& A, unsigned array, uint32_t tile, uint32_t* sm) {
   constexpr int N = P::N;
   const int lr = A.log_r, lj = LJ >= 0 ? LJ : A.log_j;
   const uint32_t R = 1u << lr, J = 1u << lj, nthr = blockDim.x;
   const TileGeom G(A, tile);
   bool in_tile = false;  // the elements are in shared memory
 
-  auto src = [&](uint32_t row, uint32_t jj) { return A.src + (size_t)G.src(A, row, jj) * N; };
+  auto src = [&](uint32_t row, uint32_t jj) { return A.arrays.src[array] + (size_t)G.src(A, row, jj) * N; };
   auto at = [&](uint32_t slot) { return tile_at<P>(sm, slot); };
 
   if (A.first && A.pre_table) {  // coset transform: times the powers of the shift
@@ -257,7 +257,7 @@ __device__ __forceinline__ void field_tile(const PassArgs& A, uint32_t tile, uin
     for (uint32_t b = threadIdx.x; b < R << lj; b += nthr) {
       const uint32_t jj = b & (J - 1u), t = b >> lj, pos = G.src(A, t, jj);
       Fe<P> x, r;
-      fe_load_cg<P>(x, A.src + (size_t)pos * N);
+      fe_load_cg<P>(x, A.arrays.src[array] + (size_t)pos * N);
       fe_mul_tw<P, 2>(r, x, A.pre_table + tw_offset<P>(pos));
       tile_store<P>(at(tile_slot<LJ>(t, jj, lj)), r);
     }
@@ -304,7 +304,7 @@ __device__ __forceinline__ void field_tile(const PassArgs& A, uint32_t tile, uin
   // (non-last), or the division by n, the post table and the canonical form (last), and the store.
   auto emit = [&](Fe<P>& x, uint32_t t, uint32_t jj) {
     const uint32_t pos = G.dst<P>(A, t, jj);
-    uint32_t* const out = A.dst + (size_t)pos * N;
+    uint32_t* const out = A.arrays.dst[array] + (size_t)pos * N;
     if (A.last && A.div_log) fe_div_pow2<P>(x, x, A.div_log);
     if (!A.last || A.post_table) {
       Fe<P> v;
@@ -349,16 +349,19 @@ constexpr int pass_max_regs() {
   return P::N >= 16 ? 128 : P::N == 8 ? 64 : 255;
 }
 
-template <class P, int LJ>
+// MANY: the grid has a block row per array (PassArrays).  With one array its addresses stay in the parameter bank: the
+// 8-limb passes run 1% slower with them in registers; the 24-limb ones do not notice and have the one form.
+template <class P, int LJ, bool MANY>
 __global__ void __maxnreg__(pass_max_regs<P>()) ntt_pass_kernel(const __grid_constant__ PassArgs A) {
   extern __shared__ uint4 gsn_smem[];
   uint32_t* sm = reinterpret_cast<uint32_t*>(gsn_smem);
+  const unsigned array = MANY ? blockIdx.y : 0u;
   chain_wait();
   for (uint64_t t = blockIdx.x; t < A.tiles; t += gridDim.x) {  // tiles < 2^28
     if constexpr (P::N == 1) {
-      word_tile<P>(A, (uint32_t)t, sm);
+      word_tile<P>(A, array, (uint32_t)t, sm);
     } else {
-      field_tile<P, LJ>(A, (uint32_t)t, sm);
+      field_tile<P, LJ>(A, array, (uint32_t)t, sm);
     }
   }
 }
@@ -545,8 +548,8 @@ __device__ __forceinline__ void job_pass_args(PassArgs& A, const BatchJob& J, in
   for (int i = 0; i < pass; ++i) outer += J.radix_log[i];
   A.first = pass == 0;
   A.last = pass == J.npass - 1;
-  A.src = A.first ? J.data : J.scratch;
-  A.dst = A.last ? J.data : J.scratch;
+  A.arrays.src[0] = A.first ? J.data : J.scratch;
+  A.arrays.dst[0] = A.last ? J.data : J.scratch;
   A.tw = J.tw;
   A.tw_log = J.tw_log;
   A.stage_tw = J.stage_tw[pass];
@@ -611,9 +614,9 @@ __global__ void __maxnreg__(batch_max_regs<P>())
     __syncthreads();
     // each ends with __syncthreads(); s_args is rewritten only after it
     if constexpr (P::N == 1) {
-      word_tile<P>(s_args, tile, sm);
+      word_tile<P>(s_args, 0, tile, sm);
     } else {
-      field_tile<P, -1>(s_args, tile, sm);
+      field_tile<P, -1>(s_args, 0, tile, sm);
     }
     if (threadIdx.x == 0) {
       __threadfence();
@@ -628,22 +631,27 @@ constexpr uint64_t kGridPerSm = 64;
 
 template <class P>
 struct Kernels {
-  static cudaError_t pass(const PassArgs& A, int block, cudaStream_t s) {
-    const size_t smem = tile_words(P::N, (uint64_t)1 << (A.log_r + A.log_j)) * sizeof(uint32_t);
-    auto k = ntt_pass_kernel<P, -1>;
+  using PassKernel = void (*)(PassArgs);
+  template <bool MANY>
+  static PassKernel kernel_for(int log_j) {
     if constexpr (P::N > 1) {
-      if (A.log_j == 2) k = ntt_pass_kernel<P, 2>;
+      if (log_j == 2) return ntt_pass_kernel<P, 2, MANY>;
     }
     if constexpr (P::N == 8) {
-      if (A.log_j == 0) k = ntt_pass_kernel<P, 0>;
-      if (A.log_j == 1) k = ntt_pass_kernel<P, 1>;
+      if (log_j == 0) return ntt_pass_kernel<P, 0, MANY>;
+      if (log_j == 1) return ntt_pass_kernel<P, 1, MANY>;
     }
+    return ntt_pass_kernel<P, -1, MANY>;
+  }
+  static cudaError_t pass(const PassArgs& A, int arrays, int block, cudaStream_t s) {
+    const size_t smem = tile_words(P::N, (uint64_t)1 << (A.log_r + A.log_j)) * sizeof(uint32_t);
+    auto k = arrays == 1 && P::N < 16 ? kernel_for<P::N >= 16>(A.log_j) : kernel_for<true>(A.log_j);
     if (smem > kDefaultSmemOptIn) {
       cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
       if (e != cudaSuccess) return e;
     }
     const uint64_t grid = A.tiles < (1u << 20) ? A.tiles : (1u << 20);
-    return launch_chained(k, (unsigned)grid, (unsigned)block, smem, s, A);
+    return launch_chained(k, dim3((unsigned)grid, (unsigned)arrays), (unsigned)block, smem, s, A);
   }
   static cudaError_t powers(uint32_t* out, uint64_t count, const uint32_t* base_canon, cudaStream_t s) {
     Fe<P> b;

@@ -177,6 +177,8 @@ __global__ void __launch_bounds__(512) ntt_p32_kernel(const __grid_constant__ P3
   const int r = A.log_r;
   const uint32_t R = 1u << r;
   const int lj = A.log_j;  // == LCG + 2
+  const uint32_t* const src = A.arrays.src[blockIdx.y];
+  uint32_t* const dst = A.arrays.dst[blockIdx.y];
   chain_wait();
 
   for (uint64_t tile = blockIdx.x; tile < A.tiles; tile += gridDim.x) {
@@ -202,7 +204,7 @@ __global__ void __launch_bounds__(512) ntt_p32_kernel(const __grid_constant__ P3
       for (uint32_t v = threadIdx.x; v < R * CG; v += blockDim.x) {
         const uint32_t k = v >> LCG, cg = v & (CG - 1);
         const uint64_t g = base + ((uint64_t)k << A.log_inner) + 4 * cg;
-        uint4 x = __ldcg(reinterpret_cast<const uint4*>(A.src + g));
+        uint4 x = __ldcg(reinterpret_cast<const uint4*>(src + g));
         if (A.first) x = premul(A, x, g);
         sm_st<LCG>(sm, k, cg, x);
       }
@@ -215,7 +217,7 @@ __global__ void __launch_bounds__(512) ntt_p32_kernel(const __grid_constant__ P3
         for (int i = 0; i < 4; ++i) {
           const uint64_t jj = 4 * jg + i;
           const uint64_t g = ((rowpre + (jj << row_stride_log)) << r) + 4 * k4;
-          rr[i] = __ldcg(reinterpret_cast<const uint4*>(A.src + g));
+          rr[i] = __ldcg(reinterpret_cast<const uint4*>(src + g));
           if (A.first) rr[i] = premul(A, rr[i], g);
         }
         sm_st<LCG>(sm, 4 * k4 + 0, jg, make_uint4(rr[0].x, rr[1].x, rr[2].x, rr[3].x));
@@ -256,11 +258,11 @@ __global__ void __launch_bounds__(512) ntt_p32_kernel(const __grid_constant__ P3
         w.z = tw_n(A, (jp + 2) * ek);
         w.w = tw_n(A, (jp + 3) * ek);
         x = mul4v(x, w);
-        *reinterpret_cast<uint4*>(A.dst + base + ((uint64_t)k << A.log_inner) + 4 * cg) = x;
+        *reinterpret_cast<uint4*>(dst + base + ((uint64_t)k << A.log_inner) + 4 * cg) = x;
       } else {
         const uint64_t opos = obase + 4 * cg + ((uint64_t)k << A.log_outer);
         if (A.post_table) x = mul4v(x, __ldg(reinterpret_cast<const uint4*>(A.post_table + opos)));
-        *reinterpret_cast<uint4*>(A.dst + opos) = x;
+        *reinterpret_cast<uint4*>(dst + opos) = x;
       }
     }
     __syncthreads();
@@ -360,12 +362,12 @@ __device__ __forceinline__ void column_tile(const P32Args& A, uint64_t tile, uin
 // Asynchronous global -> shared copy of a column tile into the swizzled layout (cp.async, 16 bytes per
 // chunk: base and 2^log_inner are multiples of 4 elements and the array is 16-byte aligned).
 template <int RL, int LCG>
-__device__ __forceinline__ void prefetch_columns(const P32Args& A, uint4* buf, uint64_t base) {
+__device__ __forceinline__ void prefetch_columns(const P32Args& A, const uint32_t* src, uint4* buf, uint64_t base) {
   constexpr uint32_t CG = 1u << LCG, R = 1u << RL;
   const uint32_t sb = (uint32_t)__cvta_generic_to_shared(buf);
   for (uint32_t v = threadIdx.x; v < R * CG; v += blockDim.x) {
     const uint32_t k = v >> LCG, cg = v & (CG - 1);
-    const uint32_t* g = A.src + base + ((uint64_t)k << A.log_inner) + 4 * cg;
+    const uint32_t* g = src + base + ((uint64_t)k << A.log_inner) + 4 * cg;
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(sb + 16u * chunk_of<LCG>(k, cg)), "l"(g)
                  : "memory");
   }
@@ -389,7 +391,8 @@ __device__ __forceinline__ void cp_async_wait() {
 // bit-reversed order in shared memory).  The thread visits rows k0, k0 + dk, ... (blockDim is a
 // multiple of CG, so its column group is fixed), so W advances by one product with W_c(dk) per row.
 template <int RL, int LCG>
-__device__ __forceinline__ void store_fourstep(const P32Args& A, const uint4* sm, uint64_t base, uint64_t jbase) {
+__device__ __forceinline__ void store_fourstep(const P32Args& A, uint32_t* dst, const uint4* sm, uint64_t base,
+                                               uint64_t jbase) {
   constexpr uint32_t CG = 1u << LCG, R = 1u << RL;
   const uint32_t cg = threadIdx.x & (CG - 1);
   const uint32_t k0 = threadIdx.x >> LCG, dk = blockDim.x >> LCG;
@@ -403,7 +406,7 @@ __device__ __forceinline__ void store_fourstep(const P32Args& A, const uint4* sm
   for (uint32_t k = k0; k < R; k += dk) {
     uint4 x = sm[chunk_of<LCG>(brev(k, RL), cg)];
     x = mul4v(x, w);
-    *reinterpret_cast<uint4*>(A.dst + base + ((uint64_t)k << A.log_inner) + 4 * cg) = x;
+    *reinterpret_cast<uint4*>(dst + base + ((uint64_t)k << A.log_inner) + 4 * cg) = x;
     if (k + dk < R) w = mul4v_pre(w, st, stp);
   }
 }
@@ -419,6 +422,8 @@ __global__ void __launch_bounds__(512) __maxnreg__(p32::max_regs<ET>()) ntt_p32_
   extern __shared__ uint4 gsn_smem[];
   constexpr uint32_t CG = 1u << LCG;
   constexpr uint32_t R = 1u << RL;
+  const uint32_t* const src = A.arrays.src[blockIdx.y];
+  uint32_t* const dst = A.arrays.dst[blockIdx.y];
   chain_wait();
   {
     uint4* const buf0 = gsn_smem;
@@ -426,7 +431,7 @@ __global__ void __launch_bounds__(512) __maxnreg__(p32::max_regs<ET>()) ntt_p32_
     uint64_t tile = blockIdx.x, base = 0, jbase = 0;
     if (tile < A.tiles) {
       column_tile<RL, LCG>(A, tile, base, jbase);
-      prefetch_columns<RL, LCG>(A, buf0, base);
+      prefetch_columns<RL, LCG>(A, src, buf0, base);
     }
     cp_async_commit();
     bool odd = false;
@@ -436,7 +441,7 @@ __global__ void __launch_bounds__(512) __maxnreg__(p32::max_regs<ET>()) ntt_p32_
       uint64_t nbase = 0, njbase = 0;
       if (next < A.tiles) {
         column_tile<RL, LCG>(A, next, nbase, njbase);
-        prefetch_columns<RL, LCG>(A, odd ? buf0 : buf1, nbase);
+        prefetch_columns<RL, LCG>(A, src, odd ? buf0 : buf1, nbase);
       }
       cp_async_commit();
       cp_async_wait<1>();  // this tile's copies (all but the group just committed) have landed
@@ -451,7 +456,7 @@ __global__ void __launch_bounds__(512) __maxnreg__(p32::max_regs<ET>()) ntt_p32_
       }
       substeps_fixed<RL, ET, LCG, 0>(cur, A.tw_tile);  // ends with __syncthreads()
       if (next >= A.tiles) chain_next();
-      store_fourstep<RL, LCG>(A, cur, base, jbase);
+      store_fourstep<RL, LCG>(A, dst, cur, base, jbase);
       __syncthreads();
       base = nbase;
       jbase = njbase;
@@ -469,6 +474,8 @@ __global__ void __launch_bounds__(512) __maxnreg__(p32::max_regs<ET>()) ntt_p32_
   constexpr uint32_t CG = 1u << LCG;
   constexpr uint32_t R = 1u << RL;
   constexpr int lj = LCG + 2;
+  const uint32_t* const src = A.arrays.src[blockIdx.y];
+  uint32_t* const dst = A.arrays.dst[blockIdx.y];
   chain_wait();
 
   for (uint64_t tile = blockIdx.x; tile < A.tiles; tile += gridDim.x) {
@@ -492,7 +499,7 @@ __global__ void __launch_bounds__(512) __maxnreg__(p32::max_regs<ET>()) ntt_p32_
       for (uint32_t v = threadIdx.x; v < R * CG; v += blockDim.x) {
         const uint32_t k = v >> LCG, cg = v & (CG - 1);
         const uint64_t g = base + ((uint64_t)k << A.log_inner) + 4 * cg;
-        uint4 x = __ldcg(reinterpret_cast<const uint4*>(A.src + g));
+        uint4 x = __ldcg(reinterpret_cast<const uint4*>(src + g));
         if (A.first) x = premul(A, x, g);
         sm_st<LCG>(sm, k, cg, x);
       }
@@ -505,7 +512,7 @@ __global__ void __launch_bounds__(512) __maxnreg__(p32::max_regs<ET>()) ntt_p32_
         for (int i = 0; i < 4; ++i) {
           const uint64_t jj = 4 * jg + i;
           const uint64_t g = ((rowpre + (jj << row_stride_log)) << RL) + 4 * k4;
-          rr[i] = __ldcg(reinterpret_cast<const uint4*>(A.src + g));
+          rr[i] = __ldcg(reinterpret_cast<const uint4*>(src + g));
           if (A.first) rr[i] = premul(A, rr[i], g);
         }
         sm_st<LCG>(sm, 4 * k4 + 0, jg, make_uint4(rr[0].x, rr[1].x, rr[2].x, rr[3].x));
@@ -520,14 +527,14 @@ __global__ void __launch_bounds__(512) __maxnreg__(p32::max_regs<ET>()) ntt_p32_
 
     if (tile + gridDim.x >= A.tiles) chain_next();
     if (!A.last) {
-      store_fourstep<RL, LCG>(A, sm, base, jbase);
+      store_fourstep<RL, LCG>(A, dst, sm, base, jbase);
     } else {
       for (uint32_t v = threadIdx.x; v < R * CG; v += blockDim.x) {
         const uint32_t k = v >> LCG, cg = v & (CG - 1);
         uint4 x = sm_ld<LCG>(sm, brev(k, RL), cg);
         const uint64_t opos = obase + 4 * cg + ((uint64_t)k << A.log_outer);
         if (A.post_table) x = mul4v(x, __ldg(reinterpret_cast<const uint4*>(A.post_table + opos)));
-        *reinterpret_cast<uint4*>(A.dst + opos) = x;
+        *reinterpret_cast<uint4*>(dst + opos) = x;
       }
     }
     __syncthreads();
@@ -540,7 +547,7 @@ __global__ void __launch_bounds__(512) __maxnreg__(p32::max_regs<ET>()) ntt_p32_
 // for radix 2^8..2^13, the runtime-radix kernel for everything else (and for
 // 16-column tiles, in the c1 units).
 template <int ET, int LCG>
-cudaError_t p32_launch_et_cg(const P32Args& A, int block, int grid_cap, cudaStream_t s);
+cudaError_t p32_launch_et_cg(const P32Args& A, int arrays, int block, int grid_cap, cudaStream_t s);
 
 #ifdef GSN_P32_INSTANTIATE_ET
 namespace p32 {
@@ -550,7 +557,7 @@ constexpr size_t kPipeTileMax = 48 * 1024;
 
 // buffers: tile-sized shared-memory buffers the kernel uses (1 plain, 2 with the column prefetch)
 template <class K>
-cudaError_t launch_kernel(K k, const P32Args& A, int block, int grid_cap, cudaStream_t s, int buffers = 1) {
+cudaError_t launch_kernel(K k, const P32Args& A, int arrays, int block, int grid_cap, cudaStream_t s, int buffers = 1) {
   P32Args B = A;
   B.pipe = buffers > 1 ? 1 : 0;
   const size_t tile = ((size_t)1 << (A.log_r + A.log_j)) * sizeof(uint32_t);
@@ -560,7 +567,7 @@ cudaError_t launch_kernel(K k, const P32Args& A, int block, int grid_cap, cudaSt
     if (e != cudaSuccess) return e;
   }
   const uint64_t grid = A.tiles < (uint64_t)grid_cap ? A.tiles : (uint64_t)grid_cap;
-  return launch_chained(k, (unsigned)grid, (unsigned)block, smem, s, B);
+  return launch_chained(k, dim3((unsigned)grid, (unsigned)arrays), (unsigned)block, smem, s, B);
 }
 inline bool pipe_enabled() {
   static const int on = [] {
@@ -570,29 +577,29 @@ inline bool pipe_enabled() {
   return on != 0;
 }
 template <int ET, int LCG, int RL>
-cudaError_t launch_fixed(const P32Args& A, int block, int grid_cap, cudaStream_t s) {
+cudaError_t launch_fixed(const P32Args& A, int arrays, int block, int grid_cap, cudaStream_t s) {
   if constexpr (RL <= 13) {
     if (A.log_r == RL) {
       const size_t tile = ((size_t)1 << (A.log_r + A.log_j)) * sizeof(uint32_t);
       if (!A.last && tile <= kPipeTileMax && pipe_enabled())
-        return launch_kernel(ntt_p32_pipe_kernel<RL, ET, LCG>, A, block, grid_cap, s, 2);
-      return launch_kernel(ntt_p32_fixed_kernel<RL, ET, LCG>, A, block, grid_cap, s);
+        return launch_kernel(ntt_p32_pipe_kernel<RL, ET, LCG>, A, arrays, block, grid_cap, s, 2);
+      return launch_kernel(ntt_p32_fixed_kernel<RL, ET, LCG>, A, arrays, block, grid_cap, s);
     }
-    return launch_fixed<ET, LCG, RL + 1>(A, block, grid_cap, s);
+    return launch_fixed<ET, LCG, RL + 1>(A, arrays, block, grid_cap, s);
   } else {
-    return launch_kernel(ntt_p32_kernel<ET, LCG>, A, block, grid_cap, s);
+    return launch_kernel(ntt_p32_kernel<ET, LCG>, A, arrays, block, grid_cap, s);
   }
 }
 }  // namespace p32
 
 template <>
-cudaError_t p32_launch_et_cg<GSN_P32_INSTANTIATE_ET, GSN_P32_INSTANTIATE_LCG>(const P32Args& A, int block,
+cudaError_t p32_launch_et_cg<GSN_P32_INSTANTIATE_ET, GSN_P32_INSTANTIATE_LCG>(const P32Args& A, int arrays, int block,
                                                                             int grid_cap, cudaStream_t s) {
   constexpr int ET = GSN_P32_INSTANTIATE_ET;
   constexpr int LCG = GSN_P32_INSTANTIATE_LCG;
-  if (A.log_j - 2 == LCG) return p32::launch_fixed<ET, LCG, 8>(A, block, grid_cap, s);
+  if (A.log_j - 2 == LCG) return p32::launch_fixed<ET, LCG, 8>(A, arrays, block, grid_cap, s);
   if constexpr (LCG == 1) {
-    if (A.log_j - 2 == 2) return p32::launch_kernel(ntt_p32_kernel<ET, 2>, A, block, grid_cap, s);
+    if (A.log_j - 2 == 2) return p32::launch_kernel(ntt_p32_kernel<ET, 2>, A, arrays, block, grid_cap, s);
   }
   return cudaErrorInvalidValue;
 }

@@ -575,7 +575,16 @@ int scratch_for(cudaStream_t s, size_t bytes, uint32_t** out) {
   return GSN_OK;
 }
 
-static int enqueue_p32(const Plan& plan, const Tables& T, uint32_t* data, uint32_t* scratch, cudaStream_t s) {
+static void pass_arrays(PassArrays* P, bool first, bool last, uint32_t* const* data, uint32_t* const* scratch,
+                        int arrays) {
+  for (int i = 0; i < arrays; ++i) {
+    P->src[i] = first ? data[i] : scratch[i];
+    P->dst[i] = last ? data[i] : scratch[i];
+  }
+}
+
+static int enqueue_p32(const Plan& plan, const Tables& T, uint32_t* const* data, uint32_t* const* scratch, int arrays,
+                       cudaStream_t s) {
   const int sms = current_device_sms();
   P32Args A;
   std::memset(&A, 0, sizeof(A));
@@ -589,8 +598,7 @@ static int enqueue_p32(const Plan& plan, const Tables& T, uint32_t* data, uint32
   for (int p = 0; p < plan.npass; ++p) {
     A.first = p == 0;
     A.last = p == plan.npass - 1;
-    A.src = A.first ? data : scratch;
-    A.dst = A.last ? data : scratch;
+    pass_arrays(&A.arrays, A.first, A.last, data, scratch, arrays);
     A.tw_tile = T.p32_tile[p];
     A.log_r = plan.radix_log[p];
     A.log_outer = outer;
@@ -601,7 +609,7 @@ static int enqueue_p32(const Plan& plan, const Tables& T, uint32_t* data, uint32
     A.post_table = A.last ? T.post_table : nullptr;
     A.has_pre_const = A.first ? T.inverse : 0;
     A.pre_const = T.p32_pre_const;
-    cudaError_t e = launch_p32_pass(A, plan.e_log, plan.block[p], sms * 16, s);
+    cudaError_t e = launch_p32_pass(A, arrays, plan.e_log, plan.block[p], sms * 16, s);
     if (e != cudaSuccess) return cuda_fail(e, "p32 NTT pass launch");
     count_launches(1);
     outer += plan.radix_log[p];
@@ -611,7 +619,12 @@ static int enqueue_p32(const Plan& plan, const Tables& T, uint32_t* data, uint32
 
 int enqueue_ntt(const FieldOps& F, const Plan& plan, const Tables& T, uint32_t* data, uint32_t* scratch,
                 cudaStream_t s) {
-  if (plan.kernel == kKernelP32) return enqueue_p32(plan, T, data, scratch, s);
+  return enqueue_ntts(F, plan, T, &data, &scratch, 1, s);
+}
+
+int enqueue_ntts(const FieldOps& F, const Plan& plan, const Tables& T, uint32_t* const* data, uint32_t* const* scratch,
+                 int arrays, cudaStream_t s) {
+  if (plan.kernel == kKernelP32) return enqueue_p32(plan, T, data, scratch, arrays, s);
   PassArgs A;
   std::memset(&A, 0, sizeof(A));
   A.tw = T.tw;
@@ -624,8 +637,7 @@ int enqueue_ntt(const FieldOps& F, const Plan& plan, const Tables& T, uint32_t* 
   for (int p = 0; p < plan.npass; ++p) {
     A.first = p == 0;
     A.last = p == plan.npass - 1;
-    A.src = A.first ? data : scratch;
-    A.dst = A.last ? data : scratch;
+    pass_arrays(&A.arrays, A.first, A.last, data, scratch, arrays);
     A.log_r = plan.radix_log[p];
     A.log_outer = outer;
     A.log_inner = plan.log_n - outer - plan.radix_log[p];
@@ -637,7 +649,7 @@ int enqueue_ntt(const FieldOps& F, const Plan& plan, const Tables& T, uint32_t* 
     A.pre_table = A.first ? T.pre_table : nullptr;
     A.post_table = A.last ? T.post_table : nullptr;
     A.div_log = A.last ? T.div_log : 0;
-    cudaError_t e = F.pass(A, plan.block[p], s);
+    cudaError_t e = F.pass(A, arrays, plan.block[p], s);
     if (e != cudaSuccess) return cuda_fail(e, "NTT pass launch");
     count_launches(1);
     outer += plan.radix_log[p];
@@ -653,6 +665,19 @@ static int check_data_ptr(const FieldOps& F, const void* p) {
   return GSN_OK;
 }
 
+// The plan of a single transform of arrays at `ptrs` (and of their scratch, if the caller's).
+static Plan plan_for_arrays(const FieldOps& F, int log_n, const void* const* ptrs, int count) {
+  Plan plan = plan_for(F, log_n);
+  bool aligned = true;
+  for (int i = 0; i < count; ++i) aligned = aligned && reinterpret_cast<uintptr_t>(ptrs[i]) % 16 == 0;
+  if (plan.kernel == kKernelP32 && !aligned) {
+    // the register-blocked 32-bit pass moves 16-byte vectors; 4-byte-aligned arrays take the generic pass
+    const FieldLimits L = limits_of(F);
+    plan = make_plan(F, log_n, L.max_r, L.target_j, L.max_block);
+  }
+  return plan;
+}
+
 static int ntt_impl(int field, uint32_t* data, uint32_t log_n, const uint32_t* omega, int dir,
                     const uint32_t* shift, uint32_t* scratch, cudaStream_t s) {
   const FieldOps* F = field_ops(field);
@@ -666,13 +691,8 @@ static int ntt_impl(int field, uint32_t* data, uint32_t log_n, const uint32_t* o
     rc = check_data_ptr(*F, scratch);
     if (rc) return rc;
   }
-  Plan plan = plan_for(*F, (int)log_n);
-  if (plan.kernel == kKernelP32 &&
-      (reinterpret_cast<uintptr_t>(data) % 16 || reinterpret_cast<uintptr_t>(scratch) % 16)) {
-    // the register-blocked 32-bit pass moves 16-byte vectors; 4-byte-aligned arrays take the generic pass
-    const FieldLimits L = limits_of(*F);
-    plan = make_plan(*F, (int)log_n, L.max_r, L.target_j, L.max_block);
-  }
+  const void* const ptrs[2] = {data, scratch};
+  const Plan plan = plan_for_arrays(*F, (int)log_n, ptrs, 2);
   rc = resolve_plan_tables(*F, plan, &T, s);
   if (rc) return rc;
   if (plan.npass > 1 && !scratch) {
@@ -724,6 +744,52 @@ static int quotient_impl(int field, uint32_t* a, const uint32_t* b, const uint32
   if (e != cudaSuccess) return cuda_fail(e, "coset quotient launch");
   count_launches(1);
   return GSN_OK;
+}
+
+// The three polynomials of a QAP computation go through their transforms in the same launches while they and their
+// scratch stay in half of the 129 MB L2.  A pass on one small array leaves most of the chip idle.
+static bool qap_together(const FieldOps& F, uint32_t log_n) {
+  return log_n < 32 && (((uint64_t)2 * kMaxArrays * F.limbs * sizeof(uint32_t)) << log_n) <= ((uint64_t)64 << 20);
+}
+
+// Whether scratch_for(s, bytes) would have to allocate while `s` is being captured, which ends the capture.
+static bool capture_lacks_scratch(cudaStream_t s, size_t bytes) {
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (!s || cudaStreamIsCapturing(s, &cap) != cudaSuccess) cudaGetLastError();
+  if (cap == cudaStreamCaptureStatusNone) return false;
+  TableCache& C = cache();
+  std::lock_guard<std::mutex> g(C.mu);
+  const auto it = C.scratch.find(std::make_pair(current_device(), s));
+  return it == C.scratch.end() || it->second.bytes < bytes;
+}
+
+// Inverse, then coset transform of three arrays.  GSN_ERR_NOMEM, before anything is enqueued, if there is no memory for
+// three arrays of scratch or for a table.
+static int qap_arrays(const FieldOps& F, uint32_t* const* polys, uint32_t log_n, const uint32_t* shift,
+                      cudaStream_t s) {
+  for (int i = 0; i < kMaxArrays; ++i) {
+    int rc = check_data_ptr(F, polys[i]);
+    if (rc) return rc;
+  }
+  const void* const ptrs[kMaxArrays] = {polys[0], polys[1], polys[2]};
+  const Plan plan = plan_for_arrays(F, (int)log_n, ptrs, kMaxArrays);
+  const size_t words = (((size_t)F.limbs << log_n) + 3) & ~(size_t)3;  // each array's scratch 16-byte aligned
+  const size_t need = kMaxArrays * words * sizeof(uint32_t);
+  if (plan.npass > 1 && capture_lacks_scratch(s, need)) return GSN_ERR_NOMEM;
+  Tables inv, fwd;
+  int rc = resolve_tables(F, log_n, nullptr, GSN_INVERSE, nullptr, &inv, s);
+  if (!rc) rc = resolve_tables(F, log_n, nullptr, GSN_COSET_FORWARD, shift, &fwd, s);
+  if (!rc) rc = resolve_plan_tables(F, plan, &inv, s);
+  if (!rc) rc = resolve_plan_tables(F, plan, &fwd, s);
+  if (rc) return rc;
+  uint32_t* scratch[kMaxArrays] = {nullptr, nullptr, nullptr};
+  if (plan.npass > 1) {
+    rc = scratch_for(s, need, &scratch[0]);
+    if (rc) return rc;
+    for (int i = 1; i < kMaxArrays; ++i) scratch[i] = scratch[0] + i * words;
+  }
+  rc = enqueue_ntts(F, plan, inv, polys, scratch, kMaxArrays, s);
+  return rc ? rc : enqueue_ntts(F, plan, fwd, polys, scratch, kMaxArrays, s);
 }
 
 // Device buffers, streams and events of the host-memory entry points (gsn_ntt_host, gsn_ntt_host_batch).  A
@@ -1067,12 +1133,18 @@ int gsn_qap_h(int field, uint32_t* a, uint32_t* b, uint32_t* c, uint32_t log_n, 
   if (a == b || a == c || b == c) return set_error(GSN_ERR_ARG, "a, b and c must be distinct arrays");
   const cudaStream_t s = static_cast<cudaStream_t>(stream);
   uint32_t* polys[3] = {a, b, c};
-  for (uint32_t* x : polys) {  // evaluations on the domain -> coefficients -> evaluations on the coset
-    int rc = ntt_impl(field, x, log_n, nullptr, GSN_INVERSE, nullptr, nullptr, s);
-    if (!rc) rc = ntt_impl(field, x, log_n, nullptr, GSN_COSET_FORWARD, shift, nullptr, s);
-    if (rc) return rc;
+  // evaluations on the domain -> coefficients -> evaluations on the coset
+  const FieldOps* F = field_ops(field);
+  int rc = F && qap_together(*F, log_n) ? qap_arrays(*F, polys, log_n, shift, s) : GSN_ERR_NOMEM;
+  if (rc == GSN_ERR_NOMEM) {
+    for (uint32_t* x : polys) {
+      rc = ntt_impl(field, x, log_n, nullptr, GSN_INVERSE, nullptr, nullptr, s);
+      if (!rc) rc = ntt_impl(field, x, log_n, nullptr, GSN_COSET_FORWARD, shift, nullptr, s);
+      if (rc) return rc;
+    }
   }
-  int rc = quotient_impl(field, a, b, c, log_n, shift, s);
+  if (rc) return rc;
+  rc = quotient_impl(field, a, b, c, log_n, shift, s);
   if (rc) return rc;
   return ntt_impl(field, a, log_n, nullptr, GSN_COSET_INVERSE, shift, nullptr, s);
 }

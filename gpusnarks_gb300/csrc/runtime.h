@@ -42,7 +42,7 @@ struct Plan {
 };
 
 // Register-blocked 32-bit pass launcher (ntt_f_p32.cu).
-cudaError_t launch_p32_pass(const P32Args& A, int e_log, int block, int grid_cap, cudaStream_t s);
+cudaError_t launch_p32_pass(const P32Args& A, int arrays, int e_log, int block, int grid_cap, cudaStream_t s);
 
 // Default plan for (field, log_n), or the tuned one when a tuning table is
 // loaded.
@@ -105,6 +105,9 @@ int resolve_tables(const FieldOps& F, uint32_t log_n, const uint32_t* omega, int
 // Enqueues the passes of one transform.
 int enqueue_ntt(const FieldOps& F, const Plan& plan, const Tables& T, uint32_t* data, uint32_t* scratch,
                 cudaStream_t s);
+// The same transform of `arrays` (at most kMaxArrays) arrays, each pass of all of them in one launch.
+int enqueue_ntts(const FieldOps& F, const Plan& plan, const Tables& T, uint32_t* const* data, uint32_t* const* scratch,
+                 int arrays, cudaStream_t s);
 
 // Host-side plan of one batch: per-job device descriptors (scratch left
 // null for the caller to assign), the tile work list ordered by pass level,
