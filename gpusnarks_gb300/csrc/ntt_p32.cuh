@@ -121,9 +121,12 @@ __device__ __forceinline__ uint32_t tw_n(const P32Args& A, uint64_t e) {
   return mm(lo, hi);
 }
 
+// Pre-scale of the first pass: coset powers, and n^-1 of an inverse where FOLD leaves it here.  The fixed-radix kernels
+// fold n^-1 into the seeds of their four-step factors instead, one product per thread for one per element.
+template <bool FOLD>
 __device__ __forceinline__ uint4 premul(const P32Args& A, uint4 x, uint64_t g) {
   if (A.pre_table) x = mul4v(x, __ldg(reinterpret_cast<const uint4*>(A.pre_table + g)));
-  if (A.has_pre_const) x = mul4(x, A.pre_const);
+  if (!FOLD && A.has_pre_const) x = mul4(x, A.pre_const);
   return x;
 }
 
@@ -205,7 +208,7 @@ __global__ void __launch_bounds__(512) ntt_p32_kernel(const __grid_constant__ P3
         const uint32_t k = v >> LCG, cg = v & (CG - 1);
         const uint64_t g = base + ((uint64_t)k << A.log_inner) + 4 * cg;
         uint4 x = __ldcg(reinterpret_cast<const uint4*>(src + g));
-        if (A.first) x = premul(A, x, g);
+        if (A.first) x = premul<false>(A, x, g);
         sm_st<LCG>(sm, k, cg, x);
       }
     } else {
@@ -218,7 +221,7 @@ __global__ void __launch_bounds__(512) ntt_p32_kernel(const __grid_constant__ P3
           const uint64_t jj = 4 * jg + i;
           const uint64_t g = ((rowpre + (jj << row_stride_log)) << r) + 4 * k4;
           rr[i] = __ldcg(reinterpret_cast<const uint4*>(src + g));
-          if (A.first) rr[i] = premul(A, rr[i], g);
+          if (A.first) rr[i] = premul<false>(A, rr[i], g);
         }
         sm_st<LCG>(sm, 4 * k4 + 0, jg, make_uint4(rr[0].x, rr[1].x, rr[2].x, rr[3].x));
         sm_st<LCG>(sm, 4 * k4 + 1, jg, make_uint4(rr[0].y, rr[1].y, rr[2].y, rr[3].y));
@@ -400,6 +403,7 @@ __device__ __forceinline__ void store_fourstep(const P32Args& A, uint32_t* dst, 
   const uint64_t e0 = (jbase + 4 * cg) << A.log_outer, e1 = e0 + (1ull << A.log_outer),
                  e2 = e1 + (1ull << A.log_outer), e3 = e2 + (1ull << A.log_outer);
   uint4 w = make_uint4(tw_n(A, e0 * k0), tw_n(A, e1 * k0), tw_n(A, e2 * k0), tw_n(A, e3 * k0));
+  if (A.first && A.has_pre_const) w = mul4(w, A.pre_const);
   uint4 st = make_uint4(0u, 0u, 0u, 0u);
   if (k0 + dk < R) st = make_uint4(tw_n(A, e0 * dk), tw_n(A, e1 * dk), tw_n(A, e2 * dk), tw_n(A, e3 * dk));
   const uint4 stp = make_uint4(mul1_wp<F>(st.x), mul1_wp<F>(st.y), mul1_wp<F>(st.z), mul1_wp<F>(st.w));
@@ -446,11 +450,11 @@ __global__ void __launch_bounds__(512) __maxnreg__(p32::max_regs<ET>()) ntt_p32_
       cp_async_commit();
       cp_async_wait<1>();  // this tile's copies (all but the group just committed) have landed
       __syncthreads();
-      if (A.first && (A.pre_table || A.has_pre_const)) {
+      if (A.first && A.pre_table) {
         for (uint32_t v = threadIdx.x; v < R * CG; v += blockDim.x) {
           const uint32_t k = v >> LCG, cg = v & (CG - 1);
           const uint64_t g = base + ((uint64_t)k << A.log_inner) + 4 * cg;
-          sm_st<LCG>(cur, k, cg, premul(A, sm_ld<LCG>(cur, k, cg), g));
+          sm_st<LCG>(cur, k, cg, premul<true>(A, sm_ld<LCG>(cur, k, cg), g));
         }
         __syncthreads();
       }
@@ -500,7 +504,7 @@ __global__ void __launch_bounds__(512) __maxnreg__(p32::max_regs<ET>()) ntt_p32_
         const uint32_t k = v >> LCG, cg = v & (CG - 1);
         const uint64_t g = base + ((uint64_t)k << A.log_inner) + 4 * cg;
         uint4 x = __ldcg(reinterpret_cast<const uint4*>(src + g));
-        if (A.first) x = premul(A, x, g);
+        if (A.first) x = premul<true>(A, x, g);
         sm_st<LCG>(sm, k, cg, x);
       }
     } else {
@@ -513,7 +517,7 @@ __global__ void __launch_bounds__(512) __maxnreg__(p32::max_regs<ET>()) ntt_p32_
           const uint64_t jj = 4 * jg + i;
           const uint64_t g = ((rowpre + (jj << row_stride_log)) << RL) + 4 * k4;
           rr[i] = __ldcg(reinterpret_cast<const uint4*>(src + g));
-          if (A.first) rr[i] = premul(A, rr[i], g);
+          if (A.first) rr[i] = premul<true>(A, rr[i], g);
         }
         sm_st<LCG>(sm, 4 * k4 + 0, jg, make_uint4(rr[0].x, rr[1].x, rr[2].x, rr[3].x));
         sm_st<LCG>(sm, 4 * k4 + 1, jg, make_uint4(rr[0].y, rr[1].y, rr[2].y, rr[3].y));
