@@ -188,17 +188,25 @@ Plan make_split_plan(const FieldOps& F, int log_n, const int* radix_log, int npa
   return p;
 }
 
+static void forget_calls();
+
 static std::mutex g_plan_mu;
 // (field, log_n, mode) -> plan; mode 0 = single transforms, 1 = batched kernel
 static std::map<std::tuple<int, int, int>, Plan> g_tuned;
 
 void set_tuned_plan(int field, int log_n, const Plan& p, int mode) {
-  std::lock_guard<std::mutex> g(g_plan_mu);
-  g_tuned[std::make_tuple(field, log_n, mode)] = p;
+  {
+    std::lock_guard<std::mutex> g(g_plan_mu);
+    g_tuned[std::make_tuple(field, log_n, mode)] = p;
+  }
+  forget_calls();
 }
 void clear_tuned_plans() {
-  std::lock_guard<std::mutex> g(g_plan_mu);
-  g_tuned.clear();
+  {
+    std::lock_guard<std::mutex> g(g_plan_mu);
+    g_tuned.clear();
+  }
+  forget_calls();
 }
 bool get_tuned_plan(int field, int log_n, Plan* out, int mode) {
   std::lock_guard<std::mutex> g(g_plan_mu);
@@ -490,7 +498,9 @@ static int step_table(const FieldOps& F, const uint32_t* tw, int shift, int r, i
 
 int resolve_pass_tables(const FieldOps& F, const Plan& plan, Tables* T, cudaStream_t s) {
   full_table_passes(plan, T);
+  T->own_passes = true;
   if (F.limbs == 1) return GSN_OK;
+  T->own_passes = false;
   TableCache& C = cache();
   const int dev = current_device(), L = plan.log_n;
   std::string tail = limbs_key(T->root, F.limbs);
@@ -548,6 +558,7 @@ int resolve_pass_tables(const FieldOps& F, const Plan& plan, Tables* T, cudaStre
     }
     T->step[p] = t.step[p];
   }
+  T->own_passes = true;
   return GSN_OK;
 }
 
@@ -665,17 +676,63 @@ static int check_data_ptr(const FieldOps& F, const void* p) {
   return GSN_OK;
 }
 
-// The plan of a single transform of arrays at `ptrs` (and of their scratch, if the caller's).
-static Plan plan_for_arrays(const FieldOps& F, int log_n, const void* const* ptrs, int count) {
-  Plan plan = plan_for(F, log_n);
-  bool aligned = true;
+// What a transform call resolves to, by the values of its arguments.  Resolving takes a look-up per table, and for a
+// caller's own root the test that it is primitive (2^log_n-fold squaring on the host: 72 us for 24 limbs and 2^18);
+// small transforms take 10 us on the GPU.  Dropped when a plan changes or the caches are released.
+struct Call {
+  Plan plan;
+  Tables tables;
+};
+struct Calls {
+  std::mutex mu;
+  uint64_t generation = 0;
+  // (device, field, log_n, direction, 16-byte aligned, omega limbs, shift limbs; empty strings for the defaults)
+  std::map<std::tuple<int, int, uint32_t, int, bool, std::string, std::string>, Call> known;
+};
+static Calls& calls() {
+  static Calls* c = new Calls();
+  return *c;
+}
+static void forget_calls() {
+  Calls& K = calls();
+  std::lock_guard<std::mutex> g(K.mu);
+  ++K.generation;
+  K.known.clear();
+}
+
+static int resolve_call(const FieldOps& F, uint32_t log_n, const uint32_t* omega, int dir, const uint32_t* shift,
+                        const void* const* ptrs, int count, cudaStream_t s, Call* out) {
+  bool aligned = true;  // the multi-limb fields' arrays always are
   for (int i = 0; i < count; ++i) aligned = aligned && reinterpret_cast<uintptr_t>(ptrs[i]) % 16 == 0;
-  if (plan.kernel == kKernelP32 && !aligned) {
+  const auto key = std::make_tuple(current_device(), F.id, log_n, dir, aligned,
+                                   omega ? limbs_key(omega, F.limbs) : std::string(),
+                                   shift ? limbs_key(shift, F.limbs) : std::string());
+  Calls& K = calls();
+  uint64_t generation;
+  {
+    std::lock_guard<std::mutex> g(K.mu);
+    const auto it = K.known.find(key);
+    if (it != K.known.end()) {
+      *out = it->second;
+      return GSN_OK;
+    }
+    generation = K.generation;
+  }
+  int rc = resolve_tables(F, log_n, omega, dir, shift, &out->tables, s);
+  if (rc) return rc;
+  out->plan = plan_for(F, (int)log_n);
+  if (out->plan.kernel == kKernelP32 && !aligned) {
     // the register-blocked 32-bit pass moves 16-byte vectors; 4-byte-aligned arrays take the generic pass
     const FieldLimits L = limits_of(F);
-    plan = make_plan(F, log_n, L.max_r, L.target_j, L.max_block);
+    out->plan = make_plan(F, (int)log_n, L.max_r, L.target_j, L.max_block);
   }
-  return plan;
+  rc = resolve_plan_tables(F, out->plan, &out->tables, s);
+  if (rc) return rc;
+  if (out->plan.kernel == kKernelP32 || out->tables.own_passes) {
+    std::lock_guard<std::mutex> g(K.mu);
+    if (K.generation == generation) K.known.emplace(key, *out);
+  }
+  return GSN_OK;
 }
 
 static int ntt_impl(int field, uint32_t* data, uint32_t log_n, const uint32_t* omega, int dir,
@@ -684,22 +741,20 @@ static int ntt_impl(int field, uint32_t* data, uint32_t log_n, const uint32_t* o
   if (!F) return set_error(GSN_ERR_FIELD, "unknown field %d", field);
   int rc = check_data_ptr(*F, data);
   if (rc) return rc;
-  Tables T;
-  rc = resolve_tables(*F, log_n, omega, dir, shift, &T, s);
-  if (rc) return rc;
   if (scratch) {
     rc = check_data_ptr(*F, scratch);
     if (rc) return rc;
   }
+  Call call;
   const void* const ptrs[2] = {data, scratch};
-  const Plan plan = plan_for_arrays(*F, (int)log_n, ptrs, 2);
-  rc = resolve_plan_tables(*F, plan, &T, s);
+  rc = resolve_call(*F, log_n, omega, dir, shift, ptrs, 2, s, &call);
   if (rc) return rc;
+  const Plan& plan = call.plan;
   if (plan.npass > 1 && !scratch) {
     rc = scratch_for(s, ((size_t)1 << log_n) * F->limbs * sizeof(uint32_t), &scratch);
     if (rc) return rc;
   }
-  return enqueue_ntt(*F, plan, T, data, scratch, s);
+  return enqueue_ntt(*F, plan, call.tables, data, scratch, s);
 }
 
 // zr2 = z * R^2 with z = 1 / Z(shift * w^i) = 1 / (shift^n - 1), the inverse vanishing polynomial of the
@@ -772,24 +827,21 @@ static int qap_arrays(const FieldOps& F, uint32_t* const* polys, uint32_t log_n,
     if (rc) return rc;
   }
   const void* const ptrs[kMaxArrays] = {polys[0], polys[1], polys[2]};
-  const Plan plan = plan_for_arrays(F, (int)log_n, ptrs, kMaxArrays);
+  Call inv, fwd;
+  int rc = resolve_call(F, log_n, nullptr, GSN_INVERSE, nullptr, ptrs, kMaxArrays, s, &inv);
+  if (!rc) rc = resolve_call(F, log_n, nullptr, GSN_COSET_FORWARD, shift, ptrs, kMaxArrays, s, &fwd);
+  if (rc) return rc;
   const size_t words = (((size_t)F.limbs << log_n) + 3) & ~(size_t)3;  // each array's scratch 16-byte aligned
   const size_t need = kMaxArrays * words * sizeof(uint32_t);
-  if (plan.npass > 1 && capture_lacks_scratch(s, need)) return GSN_ERR_NOMEM;
-  Tables inv, fwd;
-  int rc = resolve_tables(F, log_n, nullptr, GSN_INVERSE, nullptr, &inv, s);
-  if (!rc) rc = resolve_tables(F, log_n, nullptr, GSN_COSET_FORWARD, shift, &fwd, s);
-  if (!rc) rc = resolve_plan_tables(F, plan, &inv, s);
-  if (!rc) rc = resolve_plan_tables(F, plan, &fwd, s);
-  if (rc) return rc;
   uint32_t* scratch[kMaxArrays] = {nullptr, nullptr, nullptr};
-  if (plan.npass > 1) {
+  if (std::max(inv.plan.npass, fwd.plan.npass) > 1) {
+    if (capture_lacks_scratch(s, need)) return GSN_ERR_NOMEM;
     rc = scratch_for(s, need, &scratch[0]);
     if (rc) return rc;
     for (int i = 1; i < kMaxArrays; ++i) scratch[i] = scratch[0] + i * words;
   }
-  rc = enqueue_ntts(F, plan, inv, polys, scratch, kMaxArrays, s);
-  return rc ? rc : enqueue_ntts(F, plan, fwd, polys, scratch, kMaxArrays, s);
+  rc = enqueue_ntts(F, inv.plan, inv.tables, polys, scratch, kMaxArrays, s);
+  return rc ? rc : enqueue_ntts(F, fwd.plan, fwd.tables, polys, scratch, kMaxArrays, s);
 }
 
 // Device buffers, streams and events of the host-memory entry points (gsn_ntt_host, gsn_ntt_host_batch).  A
@@ -1184,6 +1236,7 @@ int gsn_host_free(void* ptr) {
 
 int gsn_release_caches(void) {
   GSN_CUDA(cudaDeviceSynchronize());
+  forget_calls();
   {
     std::lock_guard<std::mutex> gh(g_host_pool_mu);
     for (HostState* h : g_host_idle) host_state_destroy(h);

@@ -71,6 +71,7 @@ struct Tables {
   // per pass, filled by resolve_pass_tables / full_table_passes (PassArgs::stage_tw, step_tw)
   const uint32_t* stage[kMaxPasses] = {nullptr, nullptr, nullptr, nullptr};
   int stage_shift[kMaxPasses] = {0, 0, 0, 0};
+  bool own_passes = false;  // the pass tables are the plan's own where the field has them
   const uint32_t* step[kMaxPasses] = {nullptr, nullptr, nullptr, nullptr};
   // register-blocked 32-bit pass tables, filled by resolve_p32_tables
   const uint32_t* p32_tile[kMaxPasses] = {nullptr, nullptr, nullptr, nullptr};
