@@ -158,77 +158,100 @@ struct TileGeom {
   }
 };
 
-// One tile of one pass, one-limb field.  `sm` holds 2^(log_r + log_j) words.  A load phase (many loads in flight, which
-// its short butterflies need: a batch ran 6.8% slower with loads in stage 0), then phases:
-//   ph = -1        pre-scale (first pass of a coset transform: powers of the shift)
-//   ph = 0..lr-2   radix-2 DIF stage ph (natural in, bit-reversed out)
-//   ph = lr        the last stage (ph = lr-1, twiddle 1: each output row is the sum or the difference of two rows, no
-//                  product) fused with the four-step twiddle (non-last) or the division by n and the post table (last)
-//                  and the store: one barrier and one shared-memory store of the tile fewer per pass.
+// One tile of one pass, one-limb field.  `sm` holds 2^(log_r + log_j) words.  Small transforms and batches of them come
+// here (ntt_p32.cuh has the large ones), so latency and instructions count: a load phase (times the powers of the shift on
+// the first pass of a coset transform), radix-4 sub-steps of 4 rows a thread (one radix-2 stage first for odd log_r), and
+// a last phase with the four-step factor (non-last) or the division by n and the post table (last) and the store.  With a
+// butterfly per thread and stage a warp took 977 instructions for a radix-2^8 tile and twice the barriers and exchanges.
+// Products by 1 are computed (the table's entry 0) rather than branched around.
+//
+// Element (row, jj) is word word_slot((row << lj) + jj): the low 5 bits take in the higher ones so that a sub-step's rows
+// at any distance and (mostly) the bit-reversed reads fall on 32 banks.  The map is linear over xor, so the rows of a
+// sub-step differ by constants.
+__device__ __forceinline__ uint32_t word_slot(uint32_t i) {
+  const uint32_t u = i >> 5;
+  return i ^ ((u ^ (u << 2) ^ (u << 3) ^ (u >> 5)) & 31u);
+}
+
 template <class P>
 __device__ void word_tile(const PassArgs& A, unsigned array, uint32_t tile, uint32_t* sm) {
   static_assert(P::N == 1, "one limb");
   const int lr = A.log_r, lj = A.log_j;
   const uint32_t R = 1u << lr, J = 1u << lj, nthr = blockDim.x;
   const TileGeom G(A, tile);
+  const bool pre = A.first && A.pre_table;
+#pragma unroll 4
   for (uint32_t e = threadIdx.x; e < R * J; e += nthr) {
     // input rows are contiguous on the last pass
     const uint32_t k = !A.last ? e >> lj : e & (R - 1u), jj = !A.last ? e & (J - 1u) : e >> lr;
-    sm[(k << lj) + jj] = __ldcg(A.arrays.src[array] + G.src(A, k, jj));
+    const uint32_t pos = G.src(A, k, jj);
+    uint32_t x = __ldcg(A.arrays.src[array] + pos);
+    if (pre) x = mul1<P>(x, A.pre_table[pos]);
+    sm[word_slot((k << lj) + jj)] = x;
   }
   __syncthreads();
-  for (int ph = A.first && A.pre_table ? -1 : 0; ph <= lr; ++ph) {
-    if (lr > 0 && ph == lr - 1) continue;  // fused into ph = lr; uniform across the block
-    const bool stage = ph >= 0 && ph < lr;
-    if (ph == lr) chain_next();
-    const uint32_t count = stage ? (R >> 1) * J : R * J;
-    for (uint32_t b = threadIdx.x; b < count; b += nthr) {
-      const uint32_t jj = b & (J - 1u), t = b >> lj;
-      Fe<P> x, y;
-      const uint32_t* w = nullptr;  // table entry of the multiplier
-      uint32_t* out;
-      if (ph < 0) {
-        out = sm + b;
-        x.l[0] = *out;
-        w = A.pre_table + G.src(A, t, jj);
-      } else if (stage) {
-        // butterfly b = (i, group, jj), the twiddle index i slowest: whole warps skip the products by 1
-        const uint32_t i = t >> ph, u = ((t & ((1u << ph) - 1u)) << (lr - ph)) + i;
-        uint32_t* const up = sm + (u << lj) + jj;
-        out = up + (1u << (lr - 1 - ph + lj));
-        x.l[0] = *up;
-        y.l[0] = *out;
-        *up = add1<P>(x.l[0], y.l[0]);
-        x.l[0] = sub1<P>(x.l[0], y.l[0]);
-        if (i != 0) w = stage_entry<P>(A, i << ph);
-      } else {
-        if (lr > 0) {
-          const uint32_t r = bitrev_bits(t, lr);  // row of output t
-          x.l[0] = sm[((r & ~1u) << lj) + jj];
-          y.l[0] = sm[((r | 1u) << lj) + jj];
-          x.l[0] = (r & 1u) ? sub1<P>(x.l[0], y.l[0]) : add1<P>(x.l[0], y.l[0]);
-        } else {
-          x.l[0] = sm[jj];
-        }
-        const uint32_t pos = G.dst<P>(A, t, jj);
-        out = A.arrays.dst[array] + pos;
-        if (!A.last) {
-          w = step_entry<P>(A, G.jbase + jj, t);
-        } else {
-          if (A.div_log) fe_div_pow2<P>(x, x, A.div_log);
-          if (A.post_table) w = A.post_table + pos;
-        }
-      }
-      if (w) fe_mul_tw<P>(x, x, w);
-      *out = x.l[0];
+  if (lr & 1) {
+    const uint32_t half = word_slot(R * J >> 1);
+    for (uint32_t u = threadIdx.x; u < R * J >> 1; u += nthr) {
+      const uint32_t w = *stage_entry<P>(A, lr > 1 ? u >> lj : 0u);
+      const uint32_t s = word_slot(u), x = sm[s], y = sm[s ^ half];
+      sm[s] = add1<P>(x, y);
+      sm[s ^ half] = mul1<P>(sub1<P>(x, y), w);
     }
     __syncthreads();
   }
+  for (int s0 = lr & 1; s0 < lr; s0 += 2) {  // stages s0 and s0 + 1 on rows row + m 2^ls
+    const int ls = lr - s0 - 2;
+    const uint32_t d1 = word_slot(1u << (ls + lj)), d2 = word_slot(2u << (ls + lj));
+    for (uint32_t u = threadIdx.x; u < R * J >> 2; u += nthr) {
+      const uint32_t low = (u >> lj) & ((1u << ls) - 1u);
+      const uint32_t w1 = *stage_entry<P>(A, (low + (1u << ls)) << s0);
+      const uint32_t s = word_slot(((u >> (ls + lj)) << (ls + lj + 2)) + (u & ((1u << (ls + lj)) - 1u)));
+      uint32_t x0 = sm[s], x1 = sm[s ^ d1], x2 = sm[s ^ d2], x3 = sm[s ^ d1 ^ d2];
+      const uint32_t t0 = add1<P>(x0, x2), t1 = add1<P>(x1, x3);
+      x2 = sub1<P>(x0, x2);
+      x3 = mul1<P>(sub1<P>(x1, x3), w1);
+      x0 = add1<P>(t0, t1);
+      x1 = sub1<P>(t0, t1);
+      if (ls != 0) {
+        x2 = mul1<P>(x2, *stage_entry<P>(A, low << s0));
+        const uint32_t w = *stage_entry<P>(A, low << (s0 + 1));
+        x1 = mul1<P>(x1, w);
+        const uint32_t t2 = sub1<P>(x2, x3);
+        x2 = add1<P>(x2, x3);
+        x3 = mul1<P>(t2, w);
+      } else {
+        const uint32_t t2 = sub1<P>(x2, x3);
+        x2 = add1<P>(x2, x3);
+        x3 = t2;
+      }
+      sm[s] = x0;
+      sm[s ^ d1] = x1;
+      sm[s ^ d2] = x2;
+      sm[s ^ d1 ^ d2] = x3;
+    }
+    __syncthreads();
+  }
+  chain_next();
+#pragma unroll 4
+  for (uint32_t e = threadIdx.x; e < R * J; e += nthr) {
+    const uint32_t k = e >> lj, jj = e & (J - 1u), pos = G.dst<P>(A, k, jj);
+    Fe<P> x;
+    x.l[0] = sm[word_slot((bitrev_bits(k, lr) << lj) + jj)];
+    if (!A.last) {
+      fe_mul_tw<P>(x, x, step_entry<P>(A, G.jbase + jj, k));
+    } else {
+      if (A.div_log) fe_div_pow2<P>(x, x, A.div_log);
+      if (A.post_table) fe_mul_tw<P>(x, x, A.post_table + pos);
+    }
+    A.arrays.dst[array][pos] = x.l[0];
+  }
+  __syncthreads();
 }
 
-// One tile of one pass, multi-limb fields; the phases of word_tile without its load phase (the first phase reads
-// global memory itself, and its product hides the latency).  `sm` holds 2^(log_r + log_j) elements (tile_words).  LJ:
-// the tile's log_j at compile time, or -1.
+// One tile of one pass, multi-limb fields: a radix-2 DIF stage per phase, the first reading global memory itself (its
+// product hides the latency), the last fused with the four-step factors and the store.  `sm` holds 2^(log_r + log_j)
+// elements (tile_words).  LJ: the tile's log_j at compile time, or -1.
 //
 // Bound: the multiply pipe.  Each phase has its own product and straight code.  Sharing one product between the phases
 // cost register moves where their values meet, and with them went generic addresses and run-time column counts: a
@@ -343,10 +366,11 @@ __device__ __forceinline__ void field_tile(const PassArgs& A, unsigned array, ui
 
 // Register cap of the per-pass kernel (255: no cap).  24 limbs: 128, 4 CTAs of 128 threads per SM; GB300, MNT4 2^18 /
 // 2^20 in us: 294 / 1104 at 128, 298 / 1141 at 144, 297 / 1137 at 168 (3 CTAs).  8 limbs: 64, 8 CTAs; without the cap
-// an earlier form of the tile took 84 registers and BLS 2^20 197 us (190.5 at 80, 186.4 at 72, 184.3 at 64).
+// an earlier form of the tile took 84 registers and BLS 2^20 197 us (190.5 at 80, 186.4 at 72, 184.3 at 64).  One limb:
+// 64, so that blocks of 1024 threads launch.
 template <class P>
 constexpr int pass_max_regs() {
-  return P::N >= 16 ? 128 : P::N == 8 ? 64 : 255;
+  return P::N >= 16 ? 128 : 64;
 }
 
 // MANY: the grid has a block row per array (PassArrays).  With one array its addresses stay in the parameter bank: the
@@ -651,7 +675,9 @@ struct Kernels {
       if (e != cudaSuccess) return e;
     }
     const uint64_t grid = A.tiles < (1u << 20) ? A.tiles : (1u << 20);
-    return launch_chained(k, dim3((unsigned)grid, (unsigned)arrays), (unsigned)block, smem, s, A);
+    // a plan's block may be larger than the register cap lets a block be; the tile loops over any block
+    const int most = 65536 / pass_max_regs<P>() / 32 * 32;
+    return launch_chained(k, dim3((unsigned)grid, (unsigned)arrays), (unsigned)std::min(block, most), smem, s, A);
   }
   static cudaError_t powers(uint32_t* out, uint64_t count, const uint32_t* base_canon, cudaStream_t s) {
     Fe<P> b;
