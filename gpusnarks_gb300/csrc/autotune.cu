@@ -58,6 +58,28 @@ std::vector<Plan> candidates(const FieldOps& F, int log_n) {
           }
       }
   }
+  if (F.id == GSN_MNT4753_FR && log_n >= 1 && log_n <= 16) {
+    // four lanes per product: one to three passes of radix <= 2^8, narrow tiles
+    auto lanes = [&](const int* radix, int np) {
+      for (int tj = 0; tj <= 2; ++tj)
+        for (int block : {64, 128, 256}) {
+          Plan p = make_split_plan(F, log_n, radix, np, tj, block);
+          p.kernel = kKernelLanes;
+          for (int i = 0; i < np; ++i)  // up to four threads per output
+            p.block[i] = std::max(32, std::min(block, 4 << (p.radix_log[i] + p.log_j[i])));
+          add(p);
+        }
+    };
+    if (log_n <= 8) lanes(&log_n, 1);
+    for (int a = 2; a <= 8; ++a) {
+      const int two[2] = {a, log_n - a};
+      if (two[1] >= 2 && two[1] <= 8) lanes(two, 2);
+      for (int b = 3; b <= 6 && log_n >= 12; ++b) {
+        const int three[3] = {a, b, log_n - a - b};
+        if (three[2] >= 3 && three[2] <= 6) lanes(three, 3);
+      }
+    }
+  }
   if (F.id == GSN_P32 && log_n >= 8) {
     for (int max_r = 7; max_r <= 14; ++max_r)
       for (int lj = 2; lj <= 3; ++lj)

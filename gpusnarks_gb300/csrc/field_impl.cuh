@@ -7,6 +7,7 @@
 #include "host_field.h"
 #include "multiexp.cuh"
 #include "ntt_kernels.cuh"
+#include "ntt_lanes.cuh"
 
 namespace gsn {
 
@@ -46,6 +47,7 @@ constexpr FieldOps make_field_ops(int max_log_n, int default_tw_log) {
                   default_tw_log,
                   P::GENERATOR,
                   &Kernels<P>::pass,
+                  &LanesKernels<P>::pass,
                   &Kernels<P>::powers,
                   &Kernels<P>::step_table,
                   &Kernels<P>::pointwise,

@@ -18,6 +18,8 @@ struct FieldOps {
   uint32_t generator;  // multiplicative generator (a quadratic non-residue)
   // device
   cudaError_t (*pass)(const PassArgs& A, int arrays, int block, cudaStream_t s);
+  // the same with four lanes per product (ntt_lanes.cuh); MNT4-753 only
+  cudaError_t (*pass_lanes)(const PassArgs& A, int arrays, int block, cudaStream_t s);
   cudaError_t (*powers)(uint32_t* out, uint64_t count, const uint32_t* base_canon, cudaStream_t s);
   // step table of a pass of radix 2^r (ntt_common.h) from the twiddle table: out entry k 2^inner + j is
   // tw entry (j k) << shift, k < 2^r, j < 2^inner (multi-limb fields)

@@ -129,6 +129,8 @@ bool plan_valid(const FieldOps& F, const Plan& p) {
     if (F.id != GSN_BLS12_381_FR || (p.e_log != 2 && p.e_log != 3)) return false;
     for (int i = 0; i < p.npass; ++i)
       if (p.log_j[i] > 2 || p.radix_log[i] < 1 || p.block[i] > 256) return false;
+  } else if (p.kernel == kKernelLanes) {
+    if (F.id != GSN_MNT4753_FR) return false;
   } else if (p.kernel != kKernelGeneric) {
     return false;
   }
@@ -636,6 +638,7 @@ int enqueue_ntt(const FieldOps& F, const Plan& plan, const Tables& T, uint32_t* 
 int enqueue_ntts(const FieldOps& F, const Plan& plan, const Tables& T, uint32_t* const* data, uint32_t* const* scratch,
                  int arrays, cudaStream_t s) {
   if (plan.kernel == kKernelP32) return enqueue_p32(plan, T, data, scratch, arrays, s);
+  const bool lanes = plan.kernel == kKernelLanes;
   PassArgs A;
   std::memset(&A, 0, sizeof(A));
   A.tw = T.tw;
@@ -660,7 +663,7 @@ int enqueue_ntts(const FieldOps& F, const Plan& plan, const Tables& T, uint32_t*
     A.pre_table = A.first ? T.pre_table : nullptr;
     A.post_table = A.last ? T.post_table : nullptr;
     A.div_log = A.last ? T.div_log : 0;
-    cudaError_t e = F.pass(A, arrays, plan.block[p], s);
+    cudaError_t e = lanes ? F.pass_lanes(A, arrays, plan.block[p], s) : F.pass(A, arrays, plan.block[p], s);
     if (e != cudaSuccess) return cuda_fail(e, "NTT pass launch");
     count_launches(1);
     outer += plan.radix_log[p];
@@ -686,8 +689,9 @@ struct Call {
 struct Calls {
   std::mutex mu;
   uint64_t generation = 0;
-  // (device, field, log_n, direction, 16-byte aligned, omega limbs, shift limbs; empty strings for the defaults)
-  std::map<std::tuple<int, int, uint32_t, int, bool, std::string, std::string>, Call> known;
+  // (device, field, log_n, direction, 16-byte aligned, within a QAP computation, omega limbs, shift limbs; empty
+  // strings for the defaults)
+  std::map<std::tuple<int, int, uint32_t, int, bool, bool, std::string, std::string>, Call> known;
 };
 static Calls& calls() {
   static Calls* c = new Calls();
@@ -700,11 +704,17 @@ static void forget_calls() {
   K.known.clear();
 }
 
+// Four lanes per product pay while the chip is not full, and a kernel's code has to be fetched anew when others run
+// between its launches. QAP computations on GB300, lanes against a thread per product: 2^12 144 and 163 us, 2^13 217 and
+// 179 (206 with lanes in the last, single transform alone).
+constexpr uint32_t kLanesMaxLogQap = 12;
+
+// ptrs: the arrays, and the caller's scratch, whose alignment counts; qap: a step of a QAP computation.
 static int resolve_call(const FieldOps& F, uint32_t log_n, const uint32_t* omega, int dir, const uint32_t* shift,
-                        const void* const* ptrs, int count, cudaStream_t s, Call* out) {
+                        const void* const* ptrs, int count, bool qap, cudaStream_t s, Call* out) {
   bool aligned = true;  // the multi-limb fields' arrays always are
   for (int i = 0; i < count; ++i) aligned = aligned && reinterpret_cast<uintptr_t>(ptrs[i]) % 16 == 0;
-  const auto key = std::make_tuple(current_device(), F.id, log_n, dir, aligned,
+  const auto key = std::make_tuple(current_device(), F.id, log_n, dir, aligned, qap,
                                    omega ? limbs_key(omega, F.limbs) : std::string(),
                                    shift ? limbs_key(shift, F.limbs) : std::string());
   Calls& K = calls();
@@ -726,6 +736,10 @@ static int resolve_call(const FieldOps& F, uint32_t log_n, const uint32_t* omega
     const FieldLimits L = limits_of(F);
     out->plan = make_plan(F, (int)log_n, L.max_r, L.target_j, L.max_block);
   }
+  if (out->plan.kernel == kKernelLanes && qap && log_n > kLanesMaxLogQap) {
+    const int radix[2] = {(int)log_n / 2, (int)log_n - (int)log_n / 2};
+    out->plan = make_split_plan(F, (int)log_n, radix, 2, /*target_j=*/0, 128);
+  }
   rc = resolve_plan_tables(F, out->plan, &out->tables, s);
   if (rc) return rc;
   if (out->plan.kernel == kKernelP32 || out->tables.own_passes) {
@@ -736,7 +750,7 @@ static int resolve_call(const FieldOps& F, uint32_t log_n, const uint32_t* omega
 }
 
 static int ntt_impl(int field, uint32_t* data, uint32_t log_n, const uint32_t* omega, int dir,
-                    const uint32_t* shift, uint32_t* scratch, cudaStream_t s) {
+                    const uint32_t* shift, uint32_t* scratch, cudaStream_t s, bool qap = false) {
   const FieldOps* F = field_ops(field);
   if (!F) return set_error(GSN_ERR_FIELD, "unknown field %d", field);
   int rc = check_data_ptr(*F, data);
@@ -747,7 +761,7 @@ static int ntt_impl(int field, uint32_t* data, uint32_t log_n, const uint32_t* o
   }
   Call call;
   const void* const ptrs[2] = {data, scratch};
-  rc = resolve_call(*F, log_n, omega, dir, shift, ptrs, 2, s, &call);
+  rc = resolve_call(*F, log_n, omega, dir, shift, ptrs, 2, qap, s, &call);
   if (rc) return rc;
   const Plan& plan = call.plan;
   if (plan.npass > 1 && !scratch) {
@@ -828,8 +842,8 @@ static int qap_arrays(const FieldOps& F, uint32_t* const* polys, uint32_t log_n,
   }
   const void* const ptrs[kMaxArrays] = {polys[0], polys[1], polys[2]};
   Call inv, fwd;
-  int rc = resolve_call(F, log_n, nullptr, GSN_INVERSE, nullptr, ptrs, kMaxArrays, s, &inv);
-  if (!rc) rc = resolve_call(F, log_n, nullptr, GSN_COSET_FORWARD, shift, ptrs, kMaxArrays, s, &fwd);
+  int rc = resolve_call(F, log_n, nullptr, GSN_INVERSE, nullptr, ptrs, kMaxArrays, true, s, &inv);
+  if (!rc) rc = resolve_call(F, log_n, nullptr, GSN_COSET_FORWARD, shift, ptrs, kMaxArrays, true, s, &fwd);
   if (rc) return rc;
   const size_t words = (((size_t)F.limbs << log_n) + 3) & ~(size_t)3;  // each array's scratch 16-byte aligned
   const size_t need = kMaxArrays * words * sizeof(uint32_t);
@@ -1198,7 +1212,7 @@ int gsn_qap_h(int field, uint32_t* a, uint32_t* b, uint32_t* c, uint32_t log_n, 
   if (rc) return rc;
   rc = quotient_impl(field, a, b, c, log_n, shift, s);
   if (rc) return rc;
-  return ntt_impl(field, a, log_n, nullptr, GSN_COSET_INVERSE, shift, nullptr, s);
+  return ntt_impl(field, a, log_n, nullptr, GSN_COSET_INVERSE, shift, nullptr, s, /*qap=*/true);
 }
 
 int gsn_convert(int field, uint32_t* data, uint64_t n, int mode, void* stream) {

@@ -28,7 +28,7 @@ void count_launches(uint64_t n);
 
 // A transform plan: pass split, tile shape and threads per pass, and which
 // kernel runs the passes.
-enum PlanKernel { kKernelGeneric = 0, kKernelP32 = 1, kKernelRB = 2 };
+enum PlanKernel { kKernelGeneric = 0, kKernelP32 = 1, kKernelRB = 2, kKernelLanes = 3 };
 
 struct Plan {
   int log_n = 0;
@@ -37,7 +37,8 @@ struct Plan {
   int log_j[kMaxPasses] = {0, 0, 0, 0};
   int block[kMaxPasses] = {0, 0, 0, 0};
   int kernel = kKernelGeneric;  // kKernelP32: register-blocked 32-bit pass (ntt_p32.cuh);
-                                // kKernelRB: named by saved tables for the 8-limb field; runs the generic pass
+                                // kKernelRB: named by saved tables for the 8-limb field; runs the generic pass;
+                                // kKernelLanes: four lanes per product, 24 limbs (ntt_lanes.cuh)
   int e_log = 4;                // kKernelP32: rows per thread per register sub-step (log2)
 };
 

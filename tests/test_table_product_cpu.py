@@ -89,6 +89,53 @@ def test_product_by_a_table_constant(fid):
             assert mul_tw(x, w, wp, p, n) == x * w % p
 
 
+def mul_lanes(x, w, wp, p, n):
+    """Four lanes per product (ntt_lanes.cuh): lane g takes limbs 4c + g of the constants, its operand shifted up g words."""
+    R = 1 << (32 * n)
+    wl, ql, neg = _limbs(w, n), _limbs(wp, n), _limbs(R - p, n)
+    h = 0
+    for g in range(4):
+        xs = _limbs(x << (32 * g), n + 3)
+        E, Od = [0] * (n + 2), [0] * (n + 2)
+        for c in range(n // 4):
+            i, y = 4 * c, ql[4 * c + g]
+            for acc, j0, base, last, top in ((E, max(0, n - 2 - i), n - 2, n + 2, n + 1),
+                                             (Od, n - 1 - i if i < n - 1 else 1, n - 1, n + 1, n)):
+                js = list(range(j0, last + 1, 2))
+                cy = _chain(acc, i + j0 - base, [xs[j] * y for j in js])
+                k = i + js[-1] - base + 2
+                if k <= top:
+                    acc[k] += cy
+                    assert acc[k] <= M, "a carry was lost"
+                else:
+                    assert cy == 0, "the product overflowed its words"
+        h += _value(E) + (_value(Od[:n + 1]) << 32)
+        assert Od[n + 1] == 0
+    assert h < 1 << (32 * (n + 2))
+    q = h >> 64
+    assert x * wp // R - 1 <= q <= x * wp // R
+    t = 0
+    for g in range(4):
+        xs, qs = _limbs(x << (32 * g), n), _limbs(q << (32 * g), n)
+        E, Od = [0] * n, [0] * n
+        for c in range(n // 4):
+            _low_row(E, Od, xs, 4 * c, wl[4 * c + g], n)
+        for c in range(n // 4):
+            _low_row(E, Od, qs, 4 * c, neg[4 * c + g], n)
+        t += _value(E) + (_value(Od[:n - 1]) << 32)
+    t %= R
+    assert t < 2 * p
+    return t % p
+
+
+def test_product_shared_by_four_lanes():
+    p, n = O.MODULI[2], O.LIMBS[2]
+    for w in _operands(2, 8, 71):
+        wp = (w << (32 * n)) // p
+        for x in _operands(2, 12, 81) + [2 * p - 1, p, p + 1]:  # values below 2p enter
+            assert mul_lanes(x, w, wp, p, n) == x * w % p
+
+
 @pytest.mark.parametrize("fid", [1, 2])
 def test_table_entry_from_the_montgomery_form(fid):
     p, n = O.MODULI[fid], O.LIMBS[fid]
