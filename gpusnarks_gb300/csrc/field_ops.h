@@ -34,11 +34,12 @@ struct FieldOps {
                        uint32_t* counters_dev, uint32_t* status_dev, int grid, int block, size_t smem,
                        cudaStream_t s, long long wait_cycles /* <= 0: default (~1 s) */);
   int (*batch_occupancy)(int block, size_t smem);
-  // sum_i a[i] b[i]: per-block partials of the first launch (multiexp_grid(n) of them, in `partial`), then
-  // one block sums them into `out`; fix = the representation constant (multiexp.cuh)
+  // sum_i a[i] b[i]: per-block partials of the first launch (multiexp_grid(n) of them, multiexp_bytes
+  // in `partial`), then one block sums them into `out`; fix = the representation constant (multiexp.cuh)
   int (*multiexp_grid)(uint64_t n);
-  cudaError_t (*multiexp)(const uint32_t* a, const uint32_t* b, uint64_t n, uint32_t* partial, int grid,
-                          uint32_t* out, const uint32_t* fix, cudaStream_t s);
+  size_t (*multiexp_bytes)(int grid);
+  cudaError_t (*multiexp)(const uint32_t* a, const uint32_t* b, uint64_t n, void* partial, int grid, uint32_t* out,
+                          const uint32_t* fix, cudaStream_t s);
   // host (canonical limbs in/out)
   void (*root)(int log_n, uint32_t* out);
   bool (*is_primitive)(const uint32_t* w, int log_n);

@@ -9,13 +9,15 @@
 //     the per-element cost is the N^2 word products of a*b (PTX mad.lo.cc/madc.hi.cc pair chains, the
 //     even/odd split of arith.cuh, so each pair can issue as one wide multiply-add) and one add chain;
 //     there is no reduction and no modular add in the loop;
-//   * once per thread the accumulator T (< count * p^2 < p * 2^(32(N+1))) is Montgomery-reduced with
-//     N+1 word steps, giving T * 2^(-32(N+1)) in [0, 2p), and one Montgomery product by a host constant
-//     turns that into the requested representation:
-//       canonical   (inputs x, y as integers):           T mod p,        fix = 2^(32(2N+1)) mod p
-//       Montgomery  (inputs xR, yR, output (sum x y) R):  T R^-1 mod p,   fix = 2^(32(N+1)) mod p;
-//   * per-thread results are canonical and combined with modular adds: warp shuffles, then shared memory,
-//     then the second launch over the per-block partials.
+//   * the threads' accumulators are added as integers, word column by word column in 64 bits: through shared memory in a
+//     block, then by the second launch over the blocks. No thread reduces or normalises anything;
+//   * one warp of the second launch reduces the total T < 2^40 p^2 by N+2 Montgomery word steps, a lane per column, to
+//     T * 2^(-32(N+2)) in [0, 2p), and one Montgomery product by a host constant, again a lane per column, turns that into
+//     the requested representation:
+//       canonical   (inputs x, y as integers):           T mod p,        fix = 2^(32(2N+2)) mod p
+//       Montgomery  (inputs xR, yR, output (sum x y) R):  T R^-1 mod p,   fix = 2^(32(N+2)) mod p.
+// Before, every thread reduced its own accumulator and multiplied it by the constant, and the canonical results went
+// through modular shuffle trees: about 10 us of a 24-limb call whatever its length.
 // The 32-bit field accumulates 64-bit products (mul.wide) into a 96-bit sum with 16-byte loads.
 #pragma once
 #include <cuda_runtime.h>
@@ -83,82 +85,102 @@ __device__ __forceinline__ void mul_acc(uint32_t (&T)[2 * N + 1], const uint32_t
   ptx::addc(T[2 * N], T[2 * N], 0u);
 }
 
-// x = T * 2^(-32(N+1)) mod p, canonical, for T < p * 2^(32(N+1)) held in 2N+1 words.  Once per thread.
+// Threads per block: 256 up to 8 limbs, 128 for 24 (register-bound).
 template <class P>
-__device__ __forceinline__ void reduce_wide(Fe<P>& x, const uint32_t (&T)[2 * P::N + 1]) {
-  constexpr int N = P::N;
-  uint32_t t[2 * N + 2];
-#pragma unroll
-  for (int k = 0; k <= 2 * N; ++k) t[k] = T[k];
-  t[2 * N + 1] = 0u;
-#pragma unroll
-  for (int k = 0; k <= N; ++k) {
-    const uint32_t m = t[k] * row_pinv<P>();
-    uint64_t c = 0;
-#pragma unroll
-    for (int j = 0; j < N; ++j) {
-      const uint64_t s = (uint64_t)m * P::mod(j) + t[k + j] + c;
-      t[k + j] = (uint32_t)s;
-      c = s >> 32;
-    }
-#pragma unroll
-    for (int j = k + N; j <= 2 * N + 1; ++j) {
-      const uint64_t s = (uint64_t)t[j] + c;
-      t[j] = (uint32_t)s;
-      c = s >> 32;
-    }
+__host__ __device__ constexpr int multiexp_block() {
+  return P::N > 8 ? 128 : 256;
+}
+
+// Word columns of an accumulator.
+template <class P>
+__host__ __device__ constexpr int columns() {
+  return 2 * P::N + 1;
+}
+
+// Sums over `count` rows of W columns, load(r * W + k) the word of row r and column k: thread k < W of the block gets column
+// k's.  `part` holds blockDim.x values.  W is odd, so rows in shared memory conflict neither in their stores nor here.
+template <int W, class Load>
+__device__ __forceinline__ uint64_t column_sum(Load load, int count, uint64_t* part) {
+  const int segs = blockDim.x / W, k = threadIdx.x % W, seg = threadIdx.x / W;
+  uint64_t sum = 0;
+  if (seg < segs) {
+#pragma unroll 8
+    for (int r = seg; r < count; r += segs) sum += load((size_t)r * W + k);
+    part[threadIdx.x] = sum;
   }
-  // value t[N+1 .. 2N+1] < 2p: one conditional subtraction
-  uint32_t d[N], mask;
-  ptx::sub_cc(d[0], t[N + 1], P::mod(0));
-#pragma unroll
-  for (int j = 1; j < N; ++j) ptx::subc_cc(d[j], t[N + 1 + j], P::mod(j));
-  ptx::subc(mask, t[2 * N + 1], 0u);  // 0xFFFFFFFF iff the value is below p
-#pragma unroll
-  for (int j = 0; j < N; ++j) x.l[j] = (t[N + 1 + j] & mask) | (d[j] & ~mask);
+  __syncthreads();
+  sum = 0;
+  if (threadIdx.x < W) {
+#pragma unroll 4
+    for (int g = 0; g < segs; ++g) sum += part[g * W + threadIdx.x];
+  }
+  return sum;
 }
 
-template <class P>
-__device__ __forceinline__ void shfl_down_fe(Fe<P>& y, const Fe<P>& x, int off) {
-#pragma unroll
-  for (int j = 0; j < P::N; ++j) y.l[j] = __shfl_down_sync(0xFFFFFFFFu, x.l[j], off);
-}
-
-// Sum of x over the block (modular); thread 0 gets it.  `sm` holds blockDim/32 elements.
-template <class P>
-__device__ __forceinline__ void block_sum(Fe<P>& x, uint32_t* sm) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+// The same for the few columns of the one-limb field, each thread's in registers: shuffles, then over the warps.
+template <int W>
+__device__ __forceinline__ uint64_t thread_columns_sum(uint64_t (&v)[W], uint64_t* part) {
 #pragma unroll
   for (int off = 16; off > 0; off >>= 1) {
-    Fe<P> y;
-    shfl_down_fe<P>(y, x, off);
-    fe_add<P>(x, x, y);
+#pragma unroll
+    for (int k = 0; k < W; ++k) v[k] += __shfl_down_sync(0xFFFFFFFFu, v[k], off);
   }
-  if (lane == 0) fe_store<P>(sm + warp * P::N, x);
+  if ((threadIdx.x & 31u) == 0) {
+#pragma unroll
+    for (int k = 0; k < W; ++k) part[(threadIdx.x >> 5) * W + k] = v[k];
+  }
   __syncthreads();
-  if (warp == 0) {
-    if (lane < warps) {
-      fe_load<P>(x, sm + lane * P::N);
-    } else {
-#pragma unroll
-      for (int j = 0; j < P::N; ++j) x.l[j] = 0u;
-    }
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
-      Fe<P> y;
-      shfl_down_fe<P>(y, x, off);
-      fe_add<P>(x, x, y);
-    }
+  uint64_t sum = 0;
+  if (threadIdx.x < W) {
+#pragma unroll 8
+    for (unsigned g = 0; g < blockDim.x / 32; ++g) sum += part[g * W + threadIdx.x];
   }
+  return sum;
 }
 
-// First launch: per-block partial sums of a[i] * b[i] (grid-stride over i), canonical, in `partial`.
+// One warp, a lane per 32-bit column (columns may hold more than 32 bits): acc = (acc + m p) / 2^32 with the m that makes
+// it whole, plus `lo` in each column and `hi` one column up.  `in` enters at lane 31.
+__device__ __forceinline__ uint64_t lane_step(uint64_t acc, uint32_t p_lane, uint32_t pinv, uint64_t hi, uint64_t in) {
+  const int lane = threadIdx.x & 31;
+  const uint32_t m = __shfl_sync(0xFFFFFFFFu, (uint32_t)acc * pinv, 0);
+  const uint64_t prod = (uint64_t)m * p_lane;
+  acc += (uint32_t)prod;
+  const uint64_t up = __shfl_down_sync(0xFFFFFFFFu, acc, 1);
+  return (lane == 31 ? in : up) + (prod >> 32) + hi + (lane == 0 ? acc >> 32 : 0u);
+}
+
+// The lanes' columns, a value below 2p, as a canonical element in every lane.  `cols` holds 32 values.
+template <class P>
+__device__ __forceinline__ void lane_gather(Fe<P>& x, uint64_t acc, uint64_t* cols) {
+  constexpr int N = P::N;
+  __syncwarp();
+  cols[threadIdx.x & 31] = acc;
+  __syncwarp();
+  uint32_t t[N], d[N], mask;
+  uint64_t c = 0;
+#pragma unroll
+  for (int j = 0; j < N; ++j) {
+    c += cols[j];
+    t[j] = (uint32_t)c;
+    c >>= 32;
+  }
+  const uint32_t top = (uint32_t)(c + cols[N]);
+  ptx::sub_cc(d[0], t[0], P::mod(0));
+#pragma unroll
+  for (int j = 1; j < N; ++j) ptx::subc_cc(d[j], t[j], P::mod(j));
+  ptx::subc(mask, top, 0u);  // 0xFFFFFFFF iff the value is below p
+#pragma unroll
+  for (int j = 0; j < N; ++j) x.l[j] = (t[j] & mask) | (d[j] & ~mask);
+}
+
+// First launch: per-block sums of a[i] * b[i] (grid-stride over i) as columns()<P> columns each, in `partial`.
 // PF: load the next element's operands before the current product (more registers, overlapped latency).
 template <class P, bool PF>
 __global__ void __launch_bounds__(256) multiexp_kernel(const uint32_t* a, const uint32_t* b, uint64_t n,
-                                                       uint32_t* partial, Fe<P> fix) {
-  constexpr int N = P::N;
-  __shared__ uint32_t sm[8 * N];
+                                                       uint64_t* partial) {
+  constexpr int N = P::N, W = columns<P>();
+  __shared__ uint32_t sums[N > 1 ? multiexp_block<P>() * W : 1];
+  __shared__ uint64_t part[multiexp_block<P>()];
   chain_wait();
   uint32_t T[2 * N + 1];
 #pragma unroll
@@ -221,35 +243,66 @@ __global__ void __launch_bounds__(256) multiexp_kernel(const uint32_t* a, const 
     }
   }
   chain_next();
-  Fe<P> r;
-  reduce_wide<P>(r, T);
-  fe_mul<P>(r, r, fix);
-  block_sum<P>(r, sm);
-  if (threadIdx.x == 0) fe_store<P>(partial + (uint64_t)blockIdx.x * N, r);
-}
-
-// Second launch (one block): out = sum of the `count` partials.
-template <class P>
-__global__ void __launch_bounds__(256) multiexp_final_kernel(const uint32_t* partial, int count, uint32_t* out) {
-  constexpr int N = P::N;
-  __shared__ uint32_t sm[8 * N];
-  chain_wait();
-  Fe<P> x;
+  uint64_t sum;
+  if constexpr (N == 1) {
+    uint64_t v[W];
 #pragma unroll
-  for (int j = 0; j < N; ++j) x.l[j] = 0u;
-  for (int k = threadIdx.x; k < count; k += blockDim.x) {
-    Fe<P> y;
-    fe_load_cg<P>(y, partial + (uint64_t)k * N);
-    fe_add<P>(x, x, y);
+    for (int k = 0; k < W; ++k) v[k] = T[k];
+    sum = thread_columns_sum<W>(v, part);
+  } else {
+#pragma unroll
+    for (int k = 0; k < W; ++k) sums[threadIdx.x * W + k] = T[k];
+    __syncthreads();
+    sum = column_sum<W>([&](size_t at) { return sums[at]; }, (int)blockDim.x, part);
   }
-  block_sum<P>(x, sm);
-  if (threadIdx.x == 0) fe_store<P>(out, x);
+  if (threadIdx.x < W) partial[(uint64_t)blockIdx.x * W + threadIdx.x] = sum;
 }
 
-// Threads per block: 256 up to 8 limbs, 128 for 24 (register-bound).
+// Second launch (one block): the columns of all blocks, then the reduction of their sum in one warp.
+constexpr int kFinalBlock = 1024;
 template <class P>
-constexpr int multiexp_block() {
-  return P::N > 8 ? 128 : 256;
+__global__ void __launch_bounds__(kFinalBlock) multiexp_final_kernel(const uint64_t* partial, int count, uint32_t* out,
+                                                                     Fe<P> fix) {
+  constexpr int N = P::N, W = columns<P>(), ROWS = N + 2;
+  __shared__ uint64_t part[kFinalBlock], cols[ROWS + 32 > W ? ROWS + 32 : W], gather[32];
+  if (threadIdx.x >= W && threadIdx.x < ROWS + 32) cols[threadIdx.x] = 0u;
+  chain_wait();
+  uint64_t sum;
+  if constexpr (N == 1) {
+    uint64_t v[W] = {0u, 0u, 0u};
+    for (int r = threadIdx.x; r < count; r += kFinalBlock) {
+#pragma unroll
+      for (int k = 0; k < W; ++k) v[k] += __ldcg(partial + (size_t)r * W + k);
+    }
+    sum = thread_columns_sum<W>(v, part);
+  } else {
+    sum = column_sum<W>([&](size_t at) { return __ldcg(partial + at); }, count, part);
+  }
+  if (threadIdx.x < W) cols[threadIdx.x] = sum;
+  __syncthreads();
+  if (threadIdx.x >= 32) return;
+  const int lane = threadIdx.x;
+  uint32_t p_lane = 0u, fix_lane = 0u;
+#pragma unroll
+  for (int j = 0; j < N; ++j) {
+    if (lane == j) {
+      p_lane = P::mod(j);
+      fix_lane = fix.l[j];
+    }
+  }
+  uint64_t acc = cols[lane];
+#pragma unroll 1
+  for (int r = 0; r < ROWS; ++r) acc = lane_step(acc, p_lane, P::PINV, 0u, cols[r + 32]);
+  Fe<P> x;
+  lane_gather<P>(x, acc, gather);
+  acc = 0u;
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    const uint64_t prod = (uint64_t)x.l[i] * fix_lane;
+    acc = lane_step(acc + (uint32_t)prod, p_lane, P::PINV, prod >> 32, 0u);
+  }
+  lane_gather<P>(x, acc, gather);
+  if (lane == 0) fe_store<P>(out, x);
 }
 
 }  // namespace mexp
@@ -281,14 +334,16 @@ struct MultiexpKernels {
     const uint64_t need = (n + 255) / 256;
     return (int)(need < 1 ? 1 : (need < full ? need : full));
   }
-  static cudaError_t run(const uint32_t* a, const uint32_t* b, uint64_t n, uint32_t* partial, int grid,
-                         uint32_t* out, const uint32_t* fix_limbs, cudaStream_t s) {
+  static size_t partial_bytes(int grid) { return (size_t)grid * mexp::columns<P>() * sizeof(uint64_t); }
+  static cudaError_t run(const uint32_t* a, const uint32_t* b, uint64_t n, void* partial, int grid, uint32_t* out,
+                         const uint32_t* fix_limbs, cudaStream_t s) {
     Fe<P> fix;
     for (int j = 0; j < P::N; ++j) fix.l[j] = fix_limbs[j];
+    uint64_t* const sums = static_cast<uint64_t*>(partial);
     auto k = prefetch() ? mexp::multiexp_kernel<P, true> : mexp::multiexp_kernel<P, false>;
-    cudaError_t e = launch_chained(k, (unsigned)grid, mexp::multiexp_block<P>(), 0, s, a, b, n, partial, fix);
+    cudaError_t e = launch_chained(k, (unsigned)grid, mexp::multiexp_block<P>(), 0, s, a, b, n, sums);
     if (e != cudaSuccess) return e;
-    return launch_chained(mexp::multiexp_final_kernel<P>, 1, 256, 0, s, partial, grid, out);
+    return launch_chained(mexp::multiexp_final_kernel<P>, 1, mexp::kFinalBlock, 0, s, sums, grid, out, fix);
   }
 };
 

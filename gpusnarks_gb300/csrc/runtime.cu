@@ -1068,7 +1068,7 @@ int gsn_ntt_host_batch(int field, uint32_t* const* data, size_t count, uint32_t 
 // multi-exponentiation over field elements (cuda/multi_exp.cu:104-137, test/multiexp.h:3-13)
 // ---------------------------------------------------------------------------
 namespace gsn {
-// The representation constant of multiexp.cuh: 2^(32(2N+1)) mod p (canonical) or 2^(32(N+1)) mod p
+// The representation constant of multiexp.cuh: 2^(32(2N+2)) mod p (canonical) or 2^(32(N+2)) mod p
 // (Montgomery), canonical limbs.  Computed once per (field, mode): the host exponentiation takes longer
 // than a whole small multi-exponentiation on the GPU.
 static void multiexp_fix(const FieldOps& F, int mode, uint32_t* fix) {
@@ -1081,7 +1081,7 @@ static void multiexp_fix(const FieldOps& F, int mode, uint32_t* fix) {
     uint32_t two[kMaxLimbs] = {0}, r[kMaxLimbs] = {0};
     two[0] = 2;
     const int N = F.limbs;
-    F.pow(two, (uint64_t)32 * (mode == GSN_MULTIEXP_CANONICAL ? 2 * N + 1 : N + 1), r);
+    F.pow(two, (uint64_t)32 * (mode == GSN_MULTIEXP_CANONICAL ? 2 * N + 2 : N + 2), r);
     it = memo.emplace(key, limbs_key(r, N)).first;
   }
   std::memcpy(fix, it->second.data(), it->second.size());
@@ -1091,7 +1091,7 @@ static int multiexp_impl(const FieldOps& F, const uint32_t* a, const uint32_t* b
                          int mode, cudaStream_t s) {
   const int grid = F.multiexp_grid(n);
   uint32_t* partial = nullptr;
-  int rc = scratch_for(s, (size_t)grid * F.limbs * sizeof(uint32_t), &partial);
+  int rc = scratch_for(s, F.multiexp_bytes(grid), &partial);
   if (rc) return rc;
   uint32_t fix[kMaxLimbs];
   multiexp_fix(F, mode, fix);
@@ -1109,7 +1109,7 @@ static int multiexp_check(const FieldOps* F, int field, const void* a, const voi
     return set_error(GSN_ERR_ARG, "bad multiexp mode %d", mode);
   if (!out) return set_error(GSN_ERR_ARG, "null output");
   if (n && (!a || !b)) return set_error(GSN_ERR_ARG, "null input array");
-  // every thread's integer accumulator stays below p * 2^(32(N+1)) while it adds fewer than 2^32 products
+  // each thread adds fewer than 2^32 products to its 2N+1 words, and the total stays below p * 2^(32(N+2))
   if (n > ((uint64_t)1 << 40)) return set_error(GSN_ERR_SIZE, "n = %llu exceeds 2^40", (unsigned long long)n);
   return GSN_OK;
 }
