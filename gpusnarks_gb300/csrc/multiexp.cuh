@@ -8,7 +8,8 @@
 //   * each thread adds the plain 2N-word products a[i]*b[i] into a (2N+1)-word integer accumulator, so
 //     the per-element cost is the N^2 word products of a*b (PTX mad.lo.cc/madc.hi.cc pair chains, the
 //     even/odd split of arith.cuh, so each pair can issue as one wide multiply-add) and one add chain;
-//     there is no reduction and no modular add in the loop;
+//     there is no reduction and no modular add in the loop. With 24 limbs the multiply pipe bounds it, and
+//     one Karatsuba step takes 432 of the 576 (1,000,003 elements on GB300: 78.7 -> 67.0 us);
 //   * the threads' accumulators are added as integers, word column by word column in 64 bits: through shared memory in a
 //     block, then by the second launch over the blocks. No thread reduces or normalises anything;
 //   * one warp of the second launch reduces the total T < 2^40 p^2 by N+2 Montgomery word steps, a lane per column, to
@@ -84,6 +85,92 @@ __device__ __forceinline__ void mul_acc(uint32_t (&T)[2 * N + 1], const uint32_t
   for (int k = 2; k < 2 * N; ++k) ptx::addc_cc(T[k], T[k], B[k - 1]);
   ptx::addc(T[2 * N], T[2 * N], 0u);
 }
+
+// The accumulator of one thread: T += a * b, and T's words at the end.
+template <int N>
+struct Accumulator {
+  uint32_t T[2 * N + 1];
+  __device__ __forceinline__ void clear() {
+#pragma unroll
+    for (int k = 0; k <= 2 * N; ++k) T[k] = 0u;
+  }
+  __device__ __forceinline__ void add(const uint32_t* a, const uint32_t* b) { mul_acc<N>(T, a, b); }
+  __device__ __forceinline__ void words(uint32_t (&out)[2 * N + 1]) const {
+#pragma unroll
+    for (int k = 0; k <= 2 * N; ++k) out[k] = T[k];
+  }
+};
+
+// 24 limbs: one Karatsuba step, kept apart over the whole sum. With halves a = a0 + a1 B, B = 2^384, the thread adds up
+// a0 b0, a1 b1 and (a0 + a1)(b0 + b1), 432 word products an element for 576, and takes the middle part out once at the end.
+// The sums of halves have a carry bit each, whose products are masked additions on the add pipe.
+template <>
+struct Accumulator<24> {
+  static constexpr int H = 12;
+  uint32_t L[2 * H + 1], U[2 * H + 1], M[2 * H + 2];
+  __device__ __forceinline__ void clear() {
+#pragma unroll
+    for (int k = 0; k <= 2 * H; ++k) L[k] = U[k] = M[k] = 0u;
+    M[2 * H + 1] = 0u;
+  }
+  __device__ __forceinline__ void add(const uint32_t* a, const uint32_t* b) {
+    uint32_t s[H], t[H], cs, ct;
+    ptx::add_cc(s[0], a[0], a[H]);
+#pragma unroll
+    for (int k = 1; k < H; ++k) ptx::addc_cc(s[k], a[k], a[H + k]);
+    ptx::addc(cs, 0u, 0u);
+    ptx::add_cc(t[0], b[0], b[H]);
+#pragma unroll
+    for (int k = 1; k < H; ++k) ptx::addc_cc(t[k], b[k], b[H + k]);
+    ptx::addc(ct, 0u, 0u);
+    uint32_t low[2 * H + 1];
+#pragma unroll
+    for (int k = 0; k <= 2 * H; ++k) low[k] = M[k];
+    mul_acc<H>(low, s, t);  // the sum of fewer than 2^32 such products fits with M's last word
+    const bool wrapped = low[2 * H] < M[2 * H];
+#pragma unroll
+    for (int k = 0; k <= 2 * H; ++k) M[k] = low[k];
+    M[2 * H + 1] += wrapped ? 1u : 0u;
+    // + 2^384 (cs t + ct s) + 2^768 cs ct
+    const uint32_t ms = 0u - cs, mt = 0u - ct;
+    ptx::add_cc(M[H], M[H], t[0] & ms);
+#pragma unroll
+    for (int k = 1; k < H; ++k) ptx::addc_cc(M[H + k], M[H + k], t[k] & ms);
+    ptx::addc_cc(M[2 * H], M[2 * H], cs & ct);
+    ptx::addc(M[2 * H + 1], M[2 * H + 1], 0u);
+    ptx::add_cc(M[H], M[H], s[0] & mt);
+#pragma unroll
+    for (int k = 1; k < H; ++k) ptx::addc_cc(M[H + k], M[H + k], s[k] & mt);
+    ptx::addc_cc(M[2 * H], M[2 * H], 0u);
+    ptx::addc(M[2 * H + 1], M[2 * H + 1], 0u);
+    mul_acc<H>(L, a, b);
+    mul_acc<H>(U, a + H, b + H);
+  }
+  __device__ __forceinline__ void words(uint32_t (&out)[4 * H + 1]) const {
+    uint32_t m[2 * H + 2];  // the middle part, M - L - U >= 0
+    ptx::sub_cc(m[0], M[0], L[0]);
+#pragma unroll
+    for (int k = 1; k <= 2 * H; ++k) ptx::subc_cc(m[k], M[k], L[k]);
+    ptx::subc(m[2 * H + 1], M[2 * H + 1], 0u);
+    ptx::sub_cc(m[0], m[0], U[0]);
+#pragma unroll
+    for (int k = 1; k <= 2 * H; ++k) ptx::subc_cc(m[k], m[k], U[k]);
+    ptx::subc(m[2 * H + 1], m[2 * H + 1], 0u);
+    // L + 2^768 U overlap in word 2H
+#pragma unroll
+    for (int k = 0; k < 2 * H; ++k) out[k] = L[k];
+    ptx::add_cc(out[2 * H], L[2 * H], U[0]);
+#pragma unroll
+    for (int k = 1; k < 2 * H; ++k) ptx::addc_cc(out[2 * H + k], U[k], 0u);
+    ptx::addc(out[4 * H], U[2 * H], 0u);
+    ptx::add_cc(out[H], out[H], m[0]);
+#pragma unroll
+    for (int k = 1; k < 2 * H + 2; ++k) ptx::addc_cc(out[H + k], out[H + k], m[k]);
+#pragma unroll
+    for (int k = 3 * H + 2; k < 4 * H; ++k) ptx::addc_cc(out[k], out[k], 0u);
+    ptx::addc(out[4 * H], out[4 * H], 0u);
+  }
+};
 
 // Threads per block: 256 up to 8 limbs, 128 for 24 (register-bound).
 template <class P>
@@ -185,6 +272,8 @@ __global__ void __launch_bounds__(256) multiexp_kernel(const uint32_t* a, const 
   uint32_t T[2 * N + 1];
 #pragma unroll
   for (int k = 0; k <= 2 * N; ++k) T[k] = 0u;
+  Accumulator<N> sum_ab;
+  sum_ab.clear();
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
   uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if constexpr (N == 1) {
@@ -221,7 +310,7 @@ __global__ void __launch_bounds__(256) multiexp_kernel(const uint32_t* a, const 
       Fe<P> x, y;
       fe_load_cg<P>(x, a + i * N);
       fe_load_cg<P>(y, b + i * N);
-      mul_acc<N>(T, x.l, y.l);
+      sum_ab.add(x.l, y.l);
     }
   } else {
     // the next element's operands are loaded before the current product, so their memory latency overlaps it
@@ -237,12 +326,13 @@ __global__ void __launch_bounds__(256) multiexp_kernel(const uint32_t* a, const 
         fe_load_cg<P>(xn, a + next * N);
         fe_load_cg<P>(yn, b + next * N);
       }
-      mul_acc<N>(T, x.l, y.l);
+      sum_ab.add(x.l, y.l);
       x = xn;
       y = yn;
     }
   }
   chain_next();
+  if constexpr (N > 1) sum_ab.words(T);
   uint64_t sum;
   if constexpr (N == 1) {
     uint64_t v[W];
@@ -313,7 +403,7 @@ namespace gsn {
 // Host launchers, instantiated per field.
 template <class P>
 struct MultiexpKernels {
-  // CTAs of the first launch for n elements: enough to fill every SM, at most one per 256 elements.
+  // CTAs of the first launch for n elements: enough to fill every SM, at most one thread per element.
   // Prefetching variant: on for the multi-limb fields (the 24-limb loop gained 23% from it on GB300);
   // GSN_MEXP_PREFETCH=0/1 overrides.
   static bool prefetch() {
@@ -331,7 +421,7 @@ struct MultiexpKernels {
       per_sm = 1;
     }
     const uint64_t full = (uint64_t)current_device_sms() * (uint64_t)(per_sm > 0 ? per_sm : 1);
-    const uint64_t need = (n + 255) / 256;
+    const uint64_t need = (n + mexp::multiexp_block<P>() - 1) / mexp::multiexp_block<P>();
     return (int)(need < 1 ? 1 : (need < full ? need : full));
   }
   static size_t partial_bytes(int grid) { return (size_t)grid * mexp::columns<P>() * sizeof(uint64_t); }
