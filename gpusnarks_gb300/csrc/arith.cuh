@@ -583,14 +583,27 @@ __device__ __forceinline__ void fe_mul_tw(Fe<P>& r, const Fe<P>& x, const uint32
     // BLS12-381 r has the low limbs 1 and 2^32 - 1, so R - p = (2^32 - 1) + 2^64 (...): its two low limbs'
     // share of q (R - p) is 2^32 q - q, two carry chains on the add pipe instead of 15 word products.
     constexpr bool low_by_adds = P::mod(0) == 1u && P::mod(1) == 0xFFFFFFFFu;
-    auto pl = [&](int j) { return neg_mod<P>(j); };
+    // MNT4-753 r has the low limb 2^30 + 1: q p = q + 2^30 q + 2^32 q p', p' the limbs above, whose negative modulo R / 2^32
+    // multiplies q from word 1 up.
+    constexpr bool low_by_shift = P::mod(0) == 0x40000001u && P::mod(1) != 0u;
+    auto pl = [&](int j) { return low_by_shift && j == 1 ? 0u - P::mod(1) : neg_mod<P>(j); };
 #pragma unroll
-    for (int i = 0; i < N; ++i) low_row<N>(E, O, pl, i, q[i], low_by_adds ? 2 : 0);
+    for (int i = 0; i < N; ++i) low_row<N>(E, O, pl, i, q[i], low_by_adds ? 2 : low_by_shift ? 1 : 0);
     t[0] = E[0];
     ptx::add_cc(t[1], E[1], O[0]);
 #pragma unroll
     for (int j = 2; j < N - 1; ++j) ptx::addc_cc(t[j], E[j], O[j - 1]);
     ptx::addc(t[N - 1], E[N - 1], O[N - 2]);
+    if constexpr (low_by_shift) {
+      ptx::sub_cc(t[0], t[0], q[0]);
+#pragma unroll
+      for (int j = 1; j < N - 1; ++j) ptx::subc_cc(t[j], t[j], q[j]);
+      ptx::subc(t[N - 1], t[N - 1], q[N - 1]);
+      ptx::sub_cc(t[0], t[0], q[0] << 30);
+#pragma unroll
+      for (int j = 1; j < N - 1; ++j) ptx::subc_cc(t[j], t[j], __funnelshift_l(q[j - 1], q[j], 30));
+      ptx::subc(t[N - 1], t[N - 1], __funnelshift_l(q[N - 2], q[N - 1], 30));
+    }
     if constexpr (low_by_adds) {
       ptx::add_cc(t[1], t[1], q[0]);
 #pragma unroll

@@ -63,12 +63,18 @@ def mul_tw(x, w, wp, p, n):
     for i, y in enumerate(_limbs(w, n)):
         _low_row(E, Od, xl, i, y, n)
     by_adds = p & ((1 << 64) - 1) == 1 + (M << 32)
+    by_shift = p & M == (1 << 30) + 1
     neg = _limbs(R - p, n)
+    if by_shift:
+        neg[1] = -(p >> 32) & M
+        assert _value(neg[1:]) == R // (1 << 32) - (p >> 32)
     for i, y in enumerate(_limbs(q, n)):
-        _low_row(E, Od, neg, i, y, n, 2 if by_adds else 0)
+        _low_row(E, Od, neg, i, y, n, 2 if by_adds else 1 if by_shift else 0)
     t = _value(E) + (_value(Od[:n - 1]) << 32)
     if by_adds:
         t += (q << 32) - q
+    if by_shift:
+        t -= q + (q << 30)
     t %= R
     assert t < 2 * p
     return t - p if t >= p else t
