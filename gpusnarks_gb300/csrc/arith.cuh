@@ -176,6 +176,44 @@ __device__ __forceinline__ void fe_sub(Fe<P>& r, const Fe<P>& a, const Fe<P>& b)
   }
 }
 
+// Sums and differences without a reduction, for a field whose limbs have room for many multiples of p (MNT4-753 r: 2^15).
+// Values below 2^k p in, below 2^(k+1) p out; a difference adds 2^k p to stay positive.
+constexpr int kMaxLazyLog = 12;
+template <class P>
+struct ShiftedMod {
+  uint32_t limb[kMaxLazyLog + 1][P::N];
+  constexpr ShiftedMod() : limb{} {
+    for (int k = 0; k <= kMaxLazyLog; ++k)
+      for (int j = 0; j < P::N; ++j)
+        limb[k][j] = (P::mod(j) << k) | (k > 0 && j > 0 ? P::mod(j - 1) >> (32 - k) : 0u);
+  }
+};
+template <class P>
+static __constant__ ShiftedMod<P> c_shifted_mod{};
+
+template <class P>
+__device__ __forceinline__ void fe_add_lazy(Fe<P>& r, const Fe<P>& a, const Fe<P>& b) {
+  constexpr int N = P::N;
+  ptx::add_cc(r.l[0], a.l[0], b.l[0]);
+#pragma unroll
+  for (int j = 1; j < N - 1; ++j) ptx::addc_cc(r.l[j], a.l[j], b.l[j]);
+  ptx::addc(r.l[N - 1], a.l[N - 1], b.l[N - 1]);
+}
+template <class P>
+__device__ __forceinline__ void fe_sub_lazy(Fe<P>& r, const Fe<P>& a, const Fe<P>& b, int k) {
+  constexpr int N = P::N;
+  uint32_t d[N];
+  ptx::sub_cc(d[0], a.l[0], b.l[0]);
+#pragma unroll
+  for (int j = 1; j < N - 1; ++j) ptx::subc_cc(d[j], a.l[j], b.l[j]);
+  ptx::subc(d[N - 1], a.l[N - 1], b.l[N - 1]);
+  const uint32_t* const m = c_shifted_mod<P>.limb[k];
+  ptx::add_cc(r.l[0], d[0], m[0]);
+#pragma unroll
+  for (int j = 1; j < N - 1; ++j) ptx::addc_cc(r.l[j], d[j], m[j]);
+  ptx::addc(r.l[N - 1], d[N - 1], m[N - 1]);
+}
+
 // -p^-1 mod 2^32, the factor of each reduction row's m = t_0 * (-p^-1).  For a modulus with p_0 = 1
 // (BLS12-381 r) it is 0xFFFFFFFF.  When the compiler can see that value it rewrites m = -t_0 and the
 // reduction row that uses m, at a cost of about 44 more multiply-pipe instructions per 8-limb product
@@ -454,7 +492,8 @@ __device__ __forceinline__ void fe_store(uint32_t* p, const Fe<P>& a) {
 // than (N-2) 2^(32(N-1)), which can lower it by one, in (N-2) 2^-32 of all cases.  So
 // r < p (1 + x / R + (N-2) 2^-32) + (rounding) <= p (1 + (x / R) + 2^-27) for x < R.  With x < 2p (and 2p < R by a
 // margin above 2^-27) that is below 2p and below R, so the arithmetic modulo R is exact and one conditional
-// subtraction ends in [0, p).  A caller that keeps its values in [0, 2p) leaves that subtraction out (K = 2).
+// subtraction ends in [0, p).  A caller that keeps its values in [0, 2p) leaves that subtraction out (K = 2).  MNT4-753
+// r is below 2^-15 R, so there x may be any value below 2^13 p.
 //
 // Measured on GB300 as chains of dependent products (G products/s, 128-thread blocks), Montgomery -> this form:
 // MNT4-753 7.7 -> 10.5 (16 warps per SM, 124 registers; the multiply pipe's own limit is 11.2), BLS12-381
@@ -554,6 +593,30 @@ __device__ __forceinline__ void fe_reduce_once(Fe<P>& r, const uint32_t (&t)[P::
   ptx::subc(mask, 0u, 0u);  // 0xFFFFFFFF iff t < p
 #pragma unroll
   for (int j = 0; j < N; ++j) r.l[j] = (t[j] & mask) | (d[j] & ~mask);
+}
+
+// r = x mod p for x < 2^(kMaxLazyLog + 1) p of a field with that room. The quotient from the top words alone,
+// q = floor(x_top / (p_top + 1)) up to 2^-16, is the true one or one less: the two differ by less than
+// 2^13 / p_top + 1 / p_top + 2^-16 < 0.08 before they are rounded down (p_top = 0x1c4c6).
+template <class P>
+__device__ __forceinline__ void fe_reduce_lazy(Fe<P>& r, const Fe<P>& x) {
+  constexpr int N = P::N;
+  static_assert(P::mod(N - 1) > (1u << 16) && P::mod(N - 1) < (1u << 18), "the quotient's error bound");
+  constexpr uint64_t inv = (1ull << 48) / (P::mod(N - 1) + 1u);
+  const uint32_t q = (uint32_t)((x.l[N - 1] * inv) >> 48);
+  uint32_t E[N], O[N], t[N];
+#pragma unroll
+  for (int j = 0; j < N; ++j) {
+    E[j] = x.l[j];
+    O[j] = 0u;
+  }
+  low_row<N>(E, O, [](int j) { return neg_mod<P>(j); }, 0, q);
+  t[0] = E[0];
+  ptx::add_cc(t[1], E[1], O[0]);
+#pragma unroll
+  for (int j = 2; j < N - 1; ++j) ptx::addc_cc(t[j], E[j], O[j - 1]);
+  ptx::addc(t[N - 1], E[N - 1], O[N - 2]);
+  fe_reduce_once<P>(r, t);
 }
 
 // r = x * w mod p, below K p (K = 1: canonical), for x < 2p and the table entry at `e` (table + tw_offset<P>(index)).

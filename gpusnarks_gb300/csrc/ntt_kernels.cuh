@@ -264,6 +264,32 @@ __device__ void word_tile(const PassArgs& A, unsigned array, uint32_t tile, uint
 //
 // Values stay in [0, 2p) between the phases and the passes (a product's last subtraction is left out) until the last
 // pass's store.
+//
+// The 24-limb field has room for 2^15 p: its sums and differences are not reduced at all. Stage ph takes values below
+// 2^(ph+1) p (2p from the pass before), the last one gives values below 2^(log_r+1) p, and a four-step product brings them
+// below 2p again; the last pass reduces by a quotient from the top word. log_r is at most 11 (shared memory), and 2^12 p
+// bounds what kMaxLazyLog names.
+template <class P>
+__host__ __device__ constexpr bool tile_lazy() {
+  return P::N >= 16;
+}
+template <class P>
+__device__ __forceinline__ void tile_add(Fe<P>& r, const Fe<P>& x, const Fe<P>& y) {
+  if constexpr (tile_lazy<P>()) {
+    fe_add_lazy<P>(r, x, y);
+  } else {
+    fe_add<P, 2>(r, x, y);
+  }
+}
+template <class P>
+__device__ __forceinline__ void tile_sub(Fe<P>& r, const Fe<P>& x, const Fe<P>& y, int k) {  // x, y < 2^k p if lazy
+  if constexpr (tile_lazy<P>()) {
+    fe_sub_lazy<P>(r, x, y, k);
+  } else {
+    fe_sub<P, 2>(r, x, y);
+  }
+}
+
 template <class P, int LJ>
 __device__ __forceinline__ void field_tile(const PassArgs& A, unsigned array, uint32_t tile, uint32_t* sm) {
   constexpr int N = P::N;
@@ -308,9 +334,9 @@ __device__ __forceinline__ void field_tile(const PassArgs& A, unsigned array, ui
         fe_load_cg<P>(x, src(u, jj));
         fe_load_cg<P>(y, src(u + half, jj));
       }
-      fe_add<P, 2>(s, x, y);
+      tile_add<P>(s, x, y);
       tile_store<P>(pu, s);
-      fe_sub<P, 2>(s, x, y);
+      tile_sub<P>(s, x, y, ph + 1);
       if (i != 0) {
         Fe<P> r;
         fe_mul_tw<P, 2>(r, s, stage_entry<P>(A, i << ph));
@@ -328,6 +354,9 @@ __device__ __forceinline__ void field_tile(const PassArgs& A, unsigned array, ui
   auto emit = [&](Fe<P>& x, uint32_t t, uint32_t jj) {
     const uint32_t pos = G.dst<P>(A, t, jj);
     uint32_t* const out = A.arrays.dst[array] + (size_t)pos * N;
+    if constexpr (tile_lazy<P>()) {
+      if (A.last) fe_reduce_lazy<P>(x, x);
+    }
     if (A.last && A.div_log) fe_div_pow2<P>(x, x, A.div_log);
     if (!A.last || A.post_table) {
       Fe<P> v;
@@ -335,7 +364,7 @@ __device__ __forceinline__ void field_tile(const PassArgs& A, unsigned array, ui
       if (A.last) fe_reduce_once<P>(v, v.l);
       fe_store<P>(out, v);
     } else {
-      fe_reduce_once<P>(x, x.l);
+      if (!tile_lazy<P>()) fe_reduce_once<P>(x, x.l);
       fe_store<P>(out, x);
     }
   };
@@ -353,8 +382,8 @@ __device__ __forceinline__ void field_tile(const PassArgs& A, unsigned array, ui
       if (lr > 0) fe_load_cg<P>(y, src(r + 1u, jj));
     }
     if (lr > 0) {
-      fe_add<P, 2>(s, x, y);
-      fe_sub<P, 2>(y, x, y);
+      tile_add<P>(s, x, y);
+      tile_sub<P>(y, x, y, lr);
       emit(s, t, jj);
       emit(y, t + (R >> 1), jj);
     } else {

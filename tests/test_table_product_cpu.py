@@ -142,6 +142,21 @@ def test_product_shared_by_four_lanes():
             assert mul_lanes(x, w, wp, p, n) == x * w % p
 
 
+def test_products_and_reduction_of_unreduced_values():
+    """MNT4-753: values up to 2^13 p enter products and the last pass's reduction by the top word."""
+    p, n = O.MODULI[2], O.LIMBS[2]
+    rnd = random.Random(101)
+    top = (1 << 13) * p
+    xs = [0, p, top - 1, top - p, (1 << 12) * p] + [rnd.randrange(top) for _ in range(40)]
+    xs += [m * p + d for m in (1, 2, 3, 4095, 8191) for d in (-1, 0, 1)]
+    inv = (1 << 48) // ((p >> 736) + 1)
+    for x in xs:
+        q = (x >> 736) * inv >> 48
+        assert 0 <= x - q * p < 2 * p
+        for w in (1, p - 1, rnd.randrange(p)):
+            assert mul_tw(x, w, (w << (32 * n)) // p, p, n) == x * w % p
+
+
 @pytest.mark.parametrize("fid", [1, 2])
 def test_table_entry_from_the_montgomery_form(fid):
     p, n = O.MODULI[fid], O.LIMBS[fid]
