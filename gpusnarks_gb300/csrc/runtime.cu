@@ -282,7 +282,7 @@ struct TableCache {
   std::map<std::tuple<int, int, int, int, std::string>, DevBuf> steps;
   // (device, field, log_n, split, root limbs) -> the pass tables above, one lookup per call
   std::map<std::tuple<int, int, int, std::string>, PassTables> passes;
-  std::map<std::pair<int, cudaStream_t>, DevBuf> scratch;
+  std::map<std::tuple<int, cudaStream_t, int>, DevBuf> scratch;
   std::map<int, cudaStream_t> gen_stream;  // per device
 };
 
@@ -498,6 +498,12 @@ static int step_table(const FieldOps& F, const uint32_t* tw, int shift, int r, i
   return GSN_OK;
 }
 
+static bool capturing(cudaStream_t s) {
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (s && cudaStreamIsCapturing(s, &cap) != cudaSuccess) cudaGetLastError();
+  return cap != cudaStreamCaptureStatusNone;
+}
+
 int resolve_pass_tables(const FieldOps& F, const Plan& plan, Tables* T, cudaStream_t s) {
   full_table_passes(plan, T);
   T->own_passes = true;
@@ -519,9 +525,7 @@ int resolve_pass_tables(const FieldOps& F, const Plan& plan, Tables* T, cudaStre
     }
   }
   if (!found) {
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    if (s && cudaStreamIsCapturing(s, &cap) != cudaSuccess) cudaGetLastError();
-    if (cap != cudaStreamCaptureStatusNone) return GSN_OK;
+    if (capturing(s)) return GSN_OK;
     uint32_t def[kMaxLimbs];
     default_root(F, L, def);
     const bool is_def = std::memcmp(T->root, def, sizeof(uint32_t) * F.limbs) == 0;
@@ -568,11 +572,11 @@ int resolve_plan_tables(const FieldOps& F, const Plan& plan, Tables* T, cudaStre
   return plan.kernel == kKernelP32 ? resolve_p32_tables(F, plan, T) : resolve_pass_tables(F, plan, T, s);
 }
 
-int scratch_for(cudaStream_t s, size_t bytes, uint32_t** out) {
+int scratch_for(cudaStream_t s, size_t bytes, uint32_t** out, int slot) {
   TableCache& C = cache();
   const int dev = current_device();
   std::lock_guard<std::mutex> g(C.mu);
-  DevBuf& b = C.scratch[std::make_pair(dev, s)];
+  DevBuf& b = C.scratch[std::make_tuple(dev, s, slot)];
   if (b.bytes < bytes) {
     if (b.p) {
       GSN_CUDA(cudaStreamSynchronize(s));
@@ -586,6 +590,13 @@ int scratch_for(cudaStream_t s, size_t bytes, uint32_t** out) {
   }
   *out = static_cast<uint32_t*>(b.p);
   return GSN_OK;
+}
+
+static size_t scratch_held(cudaStream_t s, int slot) {
+  TableCache& C = cache();
+  std::lock_guard<std::mutex> g(C.mu);
+  const auto it = C.scratch.find(std::make_tuple(current_device(), s, slot));
+  return it == C.scratch.end() ? 0 : it->second.bytes;
 }
 
 static void pass_arrays(PassArrays* P, bool first, bool last, uint32_t* const* data, uint32_t* const* scratch,
@@ -821,17 +832,6 @@ static bool qap_together(const FieldOps& F, uint32_t log_n) {
   return log_n < 32 && (((uint64_t)2 * kMaxArrays * F.limbs * sizeof(uint32_t)) << log_n) <= ((uint64_t)64 << 20);
 }
 
-// Whether scratch_for(s, bytes) would have to allocate while `s` is being captured, which ends the capture.
-static bool capture_lacks_scratch(cudaStream_t s, size_t bytes) {
-  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-  if (!s || cudaStreamIsCapturing(s, &cap) != cudaSuccess) cudaGetLastError();
-  if (cap == cudaStreamCaptureStatusNone) return false;
-  TableCache& C = cache();
-  std::lock_guard<std::mutex> g(C.mu);
-  const auto it = C.scratch.find(std::make_pair(current_device(), s));
-  return it == C.scratch.end() || it->second.bytes < bytes;
-}
-
 // Inverse, then coset transform of three arrays.  GSN_ERR_NOMEM, before anything is enqueued, if there is no memory for
 // three arrays of scratch or for a table.
 static int qap_arrays(const FieldOps& F, uint32_t* const* polys, uint32_t log_n, const uint32_t* shift,
@@ -845,14 +845,18 @@ static int qap_arrays(const FieldOps& F, uint32_t* const* polys, uint32_t log_n,
   int rc = resolve_call(F, log_n, nullptr, GSN_INVERSE, nullptr, ptrs, kMaxArrays, true, s, &inv);
   if (!rc) rc = resolve_call(F, log_n, nullptr, GSN_COSET_FORWARD, shift, ptrs, kMaxArrays, true, s, &fwd);
   if (rc) return rc;
-  const size_t words = (((size_t)F.limbs << log_n) + 3) & ~(size_t)3;  // each array's scratch 16-byte aligned
-  const size_t need = kMaxArrays * words * sizeof(uint32_t);
+  // One array's scratch is a transform's own, so that no buffer a captured transform holds grows here; the others' lie
+  // in a buffer beside it.
+  const size_t one = ((size_t)F.limbs << log_n) * sizeof(uint32_t);
+  const size_t step = (one + 15) & ~(size_t)15, others = (kMaxArrays - 1) * step;  // 16-byte aligned
   uint32_t* scratch[kMaxArrays] = {nullptr, nullptr, nullptr};
   if (std::max(inv.plan.npass, fwd.plan.npass) > 1) {
-    if (capture_lacks_scratch(s, need)) return GSN_ERR_NOMEM;
-    rc = scratch_for(s, need, &scratch[0]);
+    // growing a buffer would end a capture
+    if (capturing(s) && (scratch_held(s, 0) < one || scratch_held(s, kScratchArrays) < others)) return GSN_ERR_NOMEM;
+    rc = scratch_for(s, one, &scratch[0]);
+    if (!rc) rc = scratch_for(s, others, &scratch[1], kScratchArrays);
     if (rc) return rc;
-    for (int i = 1; i < kMaxArrays; ++i) scratch[i] = scratch[0] + i * words;
+    for (int i = 2; i < kMaxArrays; ++i) scratch[i] = scratch[1] + (i - 1) * (step / sizeof(uint32_t));
   }
   rc = enqueue_ntts(F, inv.plan, inv.tables, polys, scratch, kMaxArrays, s);
   return rc ? rc : enqueue_ntts(F, fwd.plan, fwd.tables, polys, scratch, kMaxArrays, s);
@@ -1087,11 +1091,22 @@ static void multiexp_fix(const FieldOps& F, int mode, uint32_t* fix) {
   std::memcpy(fix, it->second.data(), it->second.size());
 }
 
+// Scratch for the blocks' column sums.  A transform's buffer is not grown for them, since a captured transform may hold
+// it: they take a buffer of their own, or, while `s` is captured, as few blocks as fit.
+static int multiexp_scratch(const FieldOps& F, cudaStream_t s, int* grid, uint32_t** out) {
+  const size_t need = F.multiexp_bytes(*grid), block = F.multiexp_bytes(1), held = scratch_held(s, 0);
+  if (scratch_held(s, kScratchSums) >= need) return scratch_for(s, need, out, kScratchSums);
+  if (held >= need || held < block) return scratch_for(s, need, out);
+  if (!capturing(s)) return scratch_for(s, need, out, kScratchSums);
+  *grid = (int)(held / block);
+  return scratch_for(s, held, out);
+}
+
 static int multiexp_impl(const FieldOps& F, const uint32_t* a, const uint32_t* b, uint64_t n, uint32_t* out,
                          int mode, cudaStream_t s) {
-  const int grid = F.multiexp_grid(n);
+  int grid = F.multiexp_grid(n);
   uint32_t* partial = nullptr;
-  int rc = scratch_for(s, F.multiexp_bytes(grid), &partial);
+  int rc = multiexp_scratch(F, s, &grid, &partial);
   if (rc) return rc;
   uint32_t fix[kMaxLimbs];
   multiexp_fix(F, mode, fix);

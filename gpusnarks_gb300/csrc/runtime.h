@@ -128,8 +128,9 @@ int plan_batch(const FieldOps& F, const struct gsn_batch_job* jobs, size_t njobs
                const Plan* force = nullptr);
 uint64_t job_scratch_bytes(const FieldOps& F, const Plan& p);
 
-// Library-owned per-stream scratch (grow-only).
-int scratch_for(cudaStream_t s, size_t bytes, uint32_t** out);
+// Library-owned per-stream scratch (grow-only); slot 0: transforms.
+constexpr int kScratchArrays = 1, kScratchSums = 2;
+int scratch_for(cudaStream_t s, size_t bytes, uint32_t** out, int slot = 0);
 
 // Device allocation bookkeeping (for tests / stats).
 int dev_alloc(void** p, size_t bytes);
