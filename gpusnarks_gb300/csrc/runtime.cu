@@ -704,6 +704,7 @@ struct Calls {
   // strings for the defaults)
   std::map<std::tuple<int, int, uint32_t, int, bool, bool, std::string, std::string>, Call> known;
 };
+constexpr size_t kMaxCalls = 4096;  // about 1 KB each
 static Calls& calls() {
   static Calls* c = new Calls();
   return *c;
@@ -755,6 +756,7 @@ static int resolve_call(const FieldOps& F, uint32_t log_n, const uint32_t* omega
   if (rc) return rc;
   if (out->plan.kernel == kKernelP32 || out->tables.own_passes) {
     std::lock_guard<std::mutex> g(K.mu);
+    if (K.known.size() >= kMaxCalls) K.known.clear();  // a shift drawn anew for every call
     if (K.generation == generation) K.known.emplace(key, *out);
   }
   return GSN_OK;

@@ -58,3 +58,16 @@ def test_calls_in_turn(gsn, cuda_device, tmp_path, fname, log_n):
         gsn.clear_tuning()
         if TUNING_FILE.exists():
             gsn.load_tuning(TUNING_FILE)
+
+
+def test_more_shifts_than_are_kept(gsn, cuda_device):
+    import torch
+    f = gsn.P32
+    try:
+        for shift in [*range(2, 4202), 2, 3]:
+            d = torch.tensor([5, 7], dtype=torch.int32, device="cuda")
+            gsn.ntt(f, d, direction=gsn.COSET_FORWARD, shift=shift)
+            if shift < 4 or shift > 4090:  # x0 + x1 s, x0 - x1 s
+                assert d.tolist() == [5 + 7 * shift, (5 - 7 * shift) % f.p - (1 << 32)], shift
+    finally:
+        assert gsn.load().gsn_release_caches() == 0
