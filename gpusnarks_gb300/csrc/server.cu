@@ -235,6 +235,11 @@ int occupancy(gsn_server* S, const FieldOps* F, int block, size_t smem) {
   return v;
 }
 
+// A request above this much work goes by per-pass launches, alone.
+double launch_work_cap(const gsn_server* S) {
+  return S->cfg.max_launch_work ? (double)S->cfg.max_launch_work : 4e10;
+}
+
 // A lone request whose work exceeds the launch cap: its passes run as ordinary per-pass launches on the
 // slot's stream.  Their CTAs each take one tile and exit, so packed launches of later, smaller requests on
 // the other slots get SMs as tiles finish, instead of waiting for a persistent launch that holds every SM
@@ -271,7 +276,7 @@ void launch_single(gsn_server* S, Slot& sl, uint64_t id) {
 void launch(gsn_server* S, int si) {
   Slot& sl = S->slots[si];
   const size_t cap = S->cfg.max_batch_jobs > 0 ? (size_t)S->cfg.max_batch_jobs : 4096;
-  const double work_cap = S->cfg.max_launch_work ? (double)S->cfg.max_launch_work : 4e10;
+  const double work_cap = launch_work_cap(S);
   auto work_of = [&](uint64_t id) {
     const Req& q = S->reqs[id];
     return request_work(q.F, q.r.log_n);
@@ -533,7 +538,10 @@ int gsn_server_warmup(gsn_server* S, int field, uint32_t lo, uint32_t hi) {
     for (int dir = GSN_FORWARD; dir <= GSN_COSET_INVERSE; ++dir) {
       Tables T;
       int rc = resolve_tables(*F, k, nullptr, dir, nullptr, &T, nullptr);
-      if (!rc) rc = resolve_pass_tables(*F, plan_for(*F, (int)k, /*batched=*/true), &T, nullptr);
+      // the pass tables of the plan that such a request will run (0.8 GB for MNT4-753 at 2^22: 150 ms if left to the
+      // scheduler's first one)
+      const bool single = request_work(F, k) > launch_work_cap(S);
+      if (!rc) rc = resolve_plan_tables(*F, plan_for(*F, (int)k, /*batched=*/!single), &T, nullptr);
       if (rc) return rc;
     }
   }
