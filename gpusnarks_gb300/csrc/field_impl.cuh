@@ -56,6 +56,7 @@ constexpr FieldOps make_field_ops(int max_log_n, int default_tw_log) {
                   &Kernels<P>::convert,
                   &Kernels<P>::batch,
                   &Kernels<P>::batch_occupancy,
+                  &Kernels<P>::load,
                   &MultiexpKernels<P>::grid,
                   &MultiexpKernels<P>::partial_bytes,
                   &MultiexpKernels<P>::run,

@@ -740,6 +740,14 @@ struct Kernels {
                                 wait_cycles > 0 ? wait_cycles : kWaitBudgetCycles);
     return cudaGetLastError();
   }
+  // Loads the transform kernels' code, which CUDA otherwise does at each one's first launch.
+  static cudaError_t load() {
+    cudaFuncAttributes attr;
+    cudaError_t e = cudaFuncGetAttributes(&attr, batch_kernel<P>);
+    for (int lj = 0; lj <= 3 && e == cudaSuccess; ++lj)
+      e = cudaFuncGetAttributes(&attr, kernel_for<P::N >= 16>(lj));
+    return e;
+  }
   static int batch_occupancy(int block, size_t smem) {
     auto k = batch_kernel<P>;
     if (smem > kDefaultSmemOptIn) cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
