@@ -8,7 +8,7 @@ launching stream.  ``e2e`` is the same transform through the C-ABI host entry
 point gsn_ntt_host (the best_fft drop-in) on a pinned host buffer: the input
 is copied in from and the result copied back to host memory inside the timed
 region.  ``roofline`` compares the transform's algorithmic integer
-multiply-adds (2352 per 24-limb Montgomery product, (n/2) log2 n products)
+multiply-adds (1751 per 24-limb product by a table constant, (n/2) log2 n products)
 with the measured throughput of the same PTX carry-chain instructions
 (gsn_microbench_imad) in the same process.
 
@@ -238,7 +238,7 @@ def imad_peak(g) -> dict:
 
 def montgomery_schedules(g, iters: int = 2000) -> dict:
     """Montgomery products per second on the whole GPU for the one-thread schedules (0 row chains,
-    1 even/odd accumulators merged every row, the kernels' default) and the 24-limb product split over
+    1 even/odd accumulators merged every row, the default of the pointwise kernels) and the 24-limb product split over
     2 or 4 cooperating lanes."""
     lib = g.load()
     out = {}
@@ -377,10 +377,14 @@ def profiled_pipe(key: str):
     return None
 
 
+# Multiply-adds of one product by a table constant, by limbs: (wide word products, single-word ones).  A wide one
+# counts as two of the denominator's multiply-adds, a low and a high one.
+TABLE_PRODUCT = {8: (86, 14), 24: (852, 47)}
+
+
 def imad_work(f, log_n: int) -> float:
-    s = f.limbs
-    per_mul = 2 * (2 * s * s + s)
-    return per_mul * (2 ** (log_n - 1)) * log_n
+    wide, single = TABLE_PRODUCT[f.limbs]
+    return (2 * wide + single) * (2 ** (log_n - 1)) * log_n
 
 
 def p32_sweep(g, torch, flush, hbm_gbs, steps=5):
@@ -511,7 +515,7 @@ def multiexp_bench(g, torch, hbm_gbs, imad_per_s, reps=10):
     """sum_i a[i] b[i] (the reference's multiexp for field elements) per field at a size well above L2:
     device-resident inputs, CUDA-event time of the two launches, elements/s against the HBM roofline (both
     arrays read once: 2 x 4N bytes per element) and against the multiply-add roofline (N^2 word products
-    per element, 2 IMAD each); a 4097-element case checked against the oracle; the oracle's serial
+    per element, 3/4 of that for 24 limbs, 2 IMAD each); a 4097-element case checked against the oracle; the oracle's serial
     restatement of test/multiexp.h (as the reference runs it) timed on a subset beside it."""
     import oracle
     from gpusnarks_gb300.batch import fill_random
@@ -547,7 +551,7 @@ def multiexp_bench(g, torch, hbm_gbs, imad_per_s, reps=10):
         oracle.multiexp(f.fid, xc, yc)
         t_cpu = time.perf_counter() - t0
         nbytes = 2 * 4 * f.limbs * n
-        imad = 2 * f.limbs * f.limbs * n
+        imad = 2 * f.limbs * f.limbs * n * (0.75 if f.limbs == 24 else 1)
         out[f.name] = {"log_n": log_n, "ms": round(t * 1e3, 4), "Gelem_s": round(n / t / 1e9, 3),
                        "hbm_frac": round(nbytes / t / 1e9 / hbm_gbs, 4),
                        "imad_frac": round(imad / t / imad_per_s, 4), "launches": 2,
@@ -684,7 +688,7 @@ def run_gpu(args, rank, local, ws):
                      "frac": round(achieved / ip["mads_per_s"], 4), "traffic": None,
                      "peak_source": "gsn_microbench_imad in this process (PTX mad.lo.cc/madc.hi.cc chains, "
                                     "all SMs, full occupancy)",
-                     "algorithmic_work": "2352 IMAD per 24-limb Montgomery product x (n/2) log2 n",
+                     "algorithmic_work": "1751 IMAD per 24-limb product by a table constant x (n/2) log2 n",
                      "launches_per_step": per_step},
         "gpu_launches": int(launches),
         "clocks": clk.summary(),

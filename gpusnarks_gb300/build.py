@@ -7,7 +7,8 @@ are rebuilt when their source or any header in csrc/ or include/ is newer,
 or when the build-time options below change.
 
 Build-time options (environment variables, passed to nvcc as -D defines):
-  GSN_MONT_SCHEDULE  Montgomery product schedule of the multi-limb fields:
+  GSN_MONT_SCHEDULE  Montgomery product schedule of the multi-limb fields
+                     (pointwise and quotient products, table building):
                      1 even/odd accumulators (default), 0 row chains.
 """
 from __future__ import annotations

@@ -485,8 +485,9 @@ __device__ __forceinline__ void fe_store(uint32_t* p, const Fe<P>& a) {
 // Product by a table constant w (Shoup's precomputed quotient; V. Shoup's NTL, and D. Harvey, "Faster arithmetic
 // for number-theoretic transforms", 2014).  The table holds w and w' = floor(w R / p), R = 2^(32N).  With
 // q ~ floor(x w' / R), r = x w - q p lies in [0, 2p), so only the high half of x w' and the low halves of x w and
-// q p are needed: for 24 limbs 875 wide multiply-adds and 48 single-word ones, where a Montgomery product takes
-// 1152 wide ones and 24 row factors.  The transform multiplies only by table constants.
+// q p are needed: for MNT4-753 852 wide multiply-adds and 47 single-word ones, where a Montgomery product takes
+// 1152 wide ones and 24 row factors (BLS12-381: 86 and 14, against 128 and 8).  The transform multiplies only by table
+// constants.
 //
 // Bounds: floor(x w' / R) > x w / p - x / R - 1.  q leaves out the word products below word N-2, together less
 // than (N-2) 2^(32(N-1)), which can lower it by one, in (N-2) 2^-32 of all cases.  So
@@ -496,8 +497,9 @@ __device__ __forceinline__ void fe_store(uint32_t* p, const Fe<P>& a) {
 // r is below 2^-15 R, so there x may be any value below 2^13 p.
 //
 // Measured on GB300 as chains of dependent products (G products/s, 128-thread blocks), Montgomery -> this form:
-// MNT4-753 7.7 -> 10.5 (16 warps per SM, 124 registers; the multiply pipe's own limit is 11.2), BLS12-381
-// 66.8 -> 90.3 (81.9 without the modulus's two low limbs taken apart below).
+// MNT4-753 7.7 -> 10.5 (16 warps per SM, 124 registers; before its modulus's low limb went to shifts, which took 875
+// wide multiply-adds to 852 and the multiply pipe's own limit from 11.2 to 11.5), BLS12-381 66.8 -> 90.3 (81.9 without
+// the modulus's two low limbs taken apart below).
 //
 // The halves are summed by rows into two accumulators per half, one for products at even words and one for odd
 // ones, so that every product lands on an aligned register pair (one wide multiply-add) and no accumulator moves.

@@ -4,7 +4,7 @@
 // stream drains, and waits at chain_wait() until that one has ended and its writes are visible.  Every thread of a
 // kernel launched this way calls chain_wait() before it touches global memory that any kernel writes, also a thread
 // without work: a kernel's end then implies the end of all before it.  What an earlier kernel wrote is read with
-// ld.global.cg, and no pointer to it is const __restrict__: such loads might be moved ahead of the wait.  
+// ld.global.cg, and no pointer to it is const __restrict__: such loads might be moved ahead of the wait.
 // chain_next() lets the following kernel be set up once every block of this one has called it or ended (a kernel without
 // it, a caller's own, is followed only at its end).  It stands before a block's last stores, not at its start: blocks
 // set up early wait on whatever SMs have room, and a small pass then left its successor unevenly placed (BLS12-381 QAP

@@ -257,9 +257,10 @@ __device__ void word_tile(const PassArgs& A, unsigned array, uint32_t tile, uint
 // cost register moves where their values meet, and with them went generic addresses and run-time column counts: a
 // BLS12-381 butterfly took 394 instructions, of which 218 are arithmetic, and 156 of them on the multiply pipe instead
 // of 111 (GB300, ncu); here it takes about 300, 120 on that pipe.  With the table layout and the swizzle above, BLS12-381
-// 2^20 went from 184 to 163 us and MNT4-753 2^18 / 2^20 from 302 / 1167 (inverse) to 294 / 1110.  Barriers are not what
-// is left (the stages without them: 283 / 1119 us for MNT4, 162 for BLS), nor is memory (every table and source read
-// from L1: 4% less).  At 2^18 a pass is 1024 tiles on 152 SMs; an SM's seventh tile runs alone, one warp per
+// 2^20 went from 184 to 163 us and MNT4-753 2^18 / 2^20 from 302 / 1167 (inverse) to 294 / 1110 (chained launches, the
+// low limb by shifts and the unreduced sums below have since made that 159 and 283 / 1090).  Barriers were not what
+// was left of the 294 / 1110 and 163 (without them in the stages: 283 / 1119 and 162), nor was memory (every table and
+// source read from L1: 4% less).  At 2^18 a pass is 1024 tiles on 152 SMs; an SM's seventh tile runs alone, one warp per
 // scheduler, and one warp of carry chains reaches 66% of the pipe where two reach 96%.
 //
 // Values stay in [0, 2p) between the phases and the passes (a product's last subtraction is left out) until the last
@@ -393,9 +394,10 @@ __device__ __forceinline__ void field_tile(const PassArgs& A, unsigned array, ui
   __syncthreads();
 }
 
-// Register cap of the per-pass kernel (255: no cap).  24 limbs: 128, 4 CTAs of 128 threads per SM; GB300, MNT4 2^18 /
-// 2^20 in us: 294 / 1104 at 128, 298 / 1141 at 144, 297 / 1137 at 168 (3 CTAs).  8 limbs: 64, 8 CTAs; without the cap
-// an earlier form of the tile took 84 registers and BLS 2^20 197 us (190.5 at 80, 186.4 at 72, 184.3 at 64).  One limb:
+// Register cap of the per-pass kernel.  24 limbs: 128, 4 CTAs of 128 threads per SM; GB300, MNT4 2^18 / 2^20 in us:
+// 294 / 1104 at 128, 298 / 1141 at 144, 297 / 1137 at 168 (3 CTAs); a later form's 2^20 1113 at 128, 1114 at 120, 1128
+// at 112.  8 limbs: 64, 8 CTAs: BLS 2^20 158.6 us, 157.3 at 56, 160.8 at 72, 163.9 at 80 and 96; the tile's first form
+// 197 without a cap (84 registers), 184.3 at 64.  One limb:
 // 64, so that blocks of 1024 threads launch.
 template <class P>
 constexpr int pass_max_regs() {
@@ -622,9 +624,10 @@ __device__ __forceinline__ void job_pass_args(PassArgs& A, const BatchJob& J, in
   A.tiles = (uint64_t)1 << (J.log_n - A.log_r - A.log_j);
 }
 
-// Register cap of the persistent kernel, so that it keeps about the per-pass
-// kernel's occupancy: 4 CTAs of 128 threads per SM for the 753-bit field
-// (the per-pass kernel uses 112), 32 warps per SM below.
+// Register cap of the persistent kernel: the per-pass kernel's, so the same
+// occupancy, 4 CTAs of 128 threads per SM for the 753-bit field and 32 warps
+// below.  256 BLS12-381 jobs of 2^10..2^16 take 495 us at 64, 512 at 56, 494
+// at 72.
 template <class P>
 constexpr int batch_max_regs() {
   return P::N >= 16 ? 128 : 64;

@@ -360,7 +360,7 @@ uint64_t gsn_kernel_launch_count(void);
 /* ---- measurement --------------------------------------------------------- */
 /* Integer-pipe roofline denominator (no reference counterpart): throughput of
  * the PTX carry-chain multiply-adds (mad.lo.cc / madc.hi.cc) the big-field
- * Montgomery products use, on every SM at full occupancy.  Returns PTX
+ * products use, on every SM at full occupancy.  Returns PTX
  * multiply-adds per second, per SM per clock, and the SM clock seen. */
 int gsn_microbench_imad(int iters, double* mads_per_s, double* mads_per_clk_sm, double* sm_mhz);
 /* The multiply-add forms without the carry flag, on every SM at full
@@ -373,7 +373,8 @@ int gsn_microbench_imad(int iters, double* mads_per_s, double* mads_per_clk_sm, 
 int gsn_microbench_imad_form(int form, int iters, double* ops_per_s);
 /* Throughput (products per second, all SMs) of the multi-limb Montgomery
  * product with schedule 0 (row chains) or 1 (even/odd accumulators, the
- * kernels' default); first checks 256 products of
+ * default of the pointwise kernels; a transform multiplies by table
+ * constants instead, with fewer word products); first checks 256 products of
  * that schedule against the host arithmetic (GSN_ERR_STATE on a mismatch). */
 int gsn_microbench_mont(int field, int schedule, int iters, double* muls_per_s);
 /* Same for the cooperative MNT4-753 product split over `lanes` (2 or 4)
