@@ -163,7 +163,9 @@ __global__ void __launch_bounds__(lanes::kMaxBlock) ntt_lanes_kernel(const __gri
         if (b0 + (threadIdx.x & ~31u) / kLanes >= count) break;  // the whole warp is past the end
         const bool valid = mine < count;
         const uint32_t b = valid ? mine : count - 1u;
-        const uint32_t jj = b & (J - 1u), t = b >> lj;
+        // A pass in the middle works in place, and with radix 2 no stage has brought its tile into shared memory: the two
+        // outputs of a column then go to neighbouring groups, so that one warp has read both rows before it stores either.
+        const uint32_t jj = lr == 1 ? b >> 1 : b & (J - 1u), t = lr == 1 ? b & 1u : b >> lj;
         Fe<P> x, y;
         Factor<P> f;
         bool mul_here = true;
