@@ -749,8 +749,11 @@ static int resolve_call(const FieldOps& F, uint32_t log_n, const uint32_t* omega
     out->plan = make_plan(F, (int)log_n, L.max_r, L.target_j, L.max_block);
   }
   if (out->plan.kernel == kKernelLanes && qap && log_n > kLanesMaxLogQap) {
-    const int radix[2] = {(int)log_n / 2, (int)log_n - (int)log_n / 2};
-    out->plan = make_split_plan(F, (int)log_n, radix, 2, /*target_j=*/0, 128);
+    // two near-equal passes, or more where a radix would pass the field's usual limit (2^12 does not fit shared memory)
+    const int npass = std::max(2, ((int)log_n + limits_of(F).max_r - 1) / limits_of(F).max_r);
+    int radix[kMaxPasses] = {0, 0, 0, 0};
+    for (int i = 0; i < npass; ++i) radix[i] = (int)log_n * (i + 1) / npass - (int)log_n * i / npass;
+    out->plan = make_split_plan(F, (int)log_n, radix, npass, /*target_j=*/0, 128);
   }
   rc = resolve_plan_tables(F, out->plan, &out->tables, s);
   if (rc) return rc;
