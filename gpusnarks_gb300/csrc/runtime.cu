@@ -40,6 +40,7 @@ int set_error(int code, const char* fmt, ...) {
 }
 
 int cuda_fail(cudaError_t e, const char* what) {
+  cudaGetLastError();  // a failed call leaves its error there, and the next launch would report it as its own
   return set_error(GSN_ERR_CUDA, "%s failed: %s (%d)", what, cudaGetErrorString(e), (int)e);
 }
 
