@@ -1102,8 +1102,8 @@ static void multiexp_fix(const FieldOps& F, int mode, uint32_t* fix) {
 static int multiexp_scratch(const FieldOps& F, cudaStream_t s, int* grid, uint32_t** out) {
   const size_t need = F.multiexp_bytes(*grid), block = F.multiexp_bytes(1), held = scratch_held(s, 0);
   if (scratch_held(s, kScratchSums) >= need) return scratch_for(s, need, out, kScratchSums);
-  if (held >= need || held < block) return scratch_for(s, need, out);
-  if (!capturing(s)) return scratch_for(s, need, out, kScratchSums);
+  if (held >= need || held == 0) return scratch_for(s, need, out);
+  if (held < block || !capturing(s)) return scratch_for(s, need, out, kScratchSums);
   *grid = (int)(held / block);
   return scratch_for(s, held, out);
 }
