@@ -24,6 +24,7 @@ struct gsn_batch {
   std::vector<gsn_batch_job> user;
   std::vector<gsn::Plan> plans;
   std::vector<gsn::BatchJob> jobs;
+  std::vector<std::shared_ptr<const void>> held;  // the jobs' tables
   gsn::BatchJob* jobs_dev = nullptr;
   uint64_t* work_dev = nullptr;
   uint64_t nwork = 0;
@@ -64,6 +65,7 @@ int plan_batch(const FieldOps& F, const gsn_batch_job* jobs, size_t njobs, Batch
   out->plans.resize(njobs);
   out->jobs.resize(njobs);
   out->work.clear();
+  out->held.clear();
   out->block = 0;
   out->smem = 0;
   out->elements = 0;
@@ -83,6 +85,7 @@ int plan_batch(const FieldOps& F, const gsn_batch_job* jobs, size_t njobs, Batch
       if (force && own.second.log_n != (int)u.log_n) return set_error(GSN_ERR_ARG, "forced plan size mismatch");
       rc = resolve_pass_tables(F, own.second, &own.first, nullptr);
       if (rc) return rc;
+      out->held.insert(out->held.end(), own.first.held.begin(), own.first.held.end());
       if (plain) it = seen.emplace(std::make_pair(u.log_n, u.dir), own).first;
     }
     const Tables& T = plain ? it->second.first : own.first;
@@ -163,6 +166,7 @@ int gsn_batch_create(int field, const gsn_batch_job* jobs, size_t njobs, int fla
   }
   b->plans = bp.plans;
   b->jobs = bp.jobs;
+  b->held = bp.held;
   b->elements = bp.elements;
   b->block = bp.block;
   b->smem = bp.smem;

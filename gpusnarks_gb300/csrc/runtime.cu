@@ -14,7 +14,9 @@
 #include <cstdio>
 #include <cstring>
 #include <map>
+#include <memory>
 #include <mutex>
+#include <set>
 #include <string>
 #include <tuple>
 #include <vector>
@@ -85,7 +87,7 @@ const FieldOps* field_ops(int field) {
 // ---------------------------------------------------------------------------
 // device allocations
 // ---------------------------------------------------------------------------
-int dev_alloc(void** p, size_t bytes) {
+static int dev_alloc_plain(void** p, size_t bytes) {
   cudaError_t e = cudaMalloc(p, bytes ? bytes : 16);
   if (e != cudaSuccess) {
     cudaGetLastError();
@@ -268,21 +270,37 @@ struct DevBuf {
   size_t bytes = 0;
 };
 
-struct PassTables {
-  const uint32_t* stage[kMaxPasses];
-  const uint32_t* step[kMaxPasses];
+// A table in device memory, freed with its last holder.
+struct Table {
+  void* p = nullptr;
+  size_t bytes = 0;
+  ~Table() { dev_free(p); }
 };
+using TableRef = std::shared_ptr<const Table>;
+
+struct PassTables {
+  const uint32_t* stage[kMaxPasses] = {nullptr, nullptr, nullptr, nullptr};
+  const uint32_t* step[kMaxPasses] = {nullptr, nullptr, nullptr, nullptr};
+  bool none = false;  // there was no memory for them: the full table is read until tables are given back
+  std::vector<std::shared_ptr<const void>> held;
+};
+struct Call;
 
 // Every entry belongs to the device that was current when it was built: tables and scratch are keyed by
 // device as well, so a process that drives several GPUs never hands one GPU another's memory.
 struct TableCache {
   std::mutex mu;
   // (device, field, tw_log, root limbs) -> powers of the root
-  std::map<std::tuple<int, int, int, std::string>, DevBuf> powers;
+  struct Powers {
+    TableRef table;
+    bool pinned;  // default roots, and what gsn_prepare or a server's warm-up asked for
+  };
+  std::map<std::tuple<int, int, int, std::string>, Powers> powers;
   // (device, field, log2 of the order, r, root limbs) -> four-step factors of a pass of radix 2^r
-  std::map<std::tuple<int, int, int, int, std::string>, DevBuf> steps;
+  std::map<std::tuple<int, int, int, int, std::string>, TableRef> steps;
   // (device, field, log_n, split, root limbs) -> the pass tables above, one lookup per call
-  std::map<std::tuple<int, int, int, std::string>, PassTables> passes;
+  std::map<std::tuple<int, int, int, std::string>, std::shared_ptr<const PassTables>> passes;
+  std::set<std::shared_ptr<const Call>> captured;  // what captured graphs run, kept until the caches are released
   std::map<std::tuple<int, cudaStream_t, int>, DevBuf> scratch;
   std::map<int, cudaStream_t> gen_stream;  // per device
 };
@@ -290,6 +308,61 @@ struct TableCache {
 static TableCache& cache() {
   static TableCache* c = new TableCache();  // never destroyed: outlives static teardown order
   return *c;
+}
+
+static bool capturing(cudaStream_t s) {
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (s && cudaStreamIsCapturing(s, &cap) != cudaSuccess) cudaGetLastError();
+  return cap != cudaStreamCaptureStatusNone;
+}
+
+// Frees the current device's tables that nobody holds, except pinned ones: the tables of roots and shifts that no call,
+// batch or captured graph is using, and all pass tables out of use.  They are rebuilt when they are next needed.  Caller
+// holds C.mu, so nobody takes a reference meanwhile; work already enqueued on them is waited for.  False: nothing freed.
+static bool give_back_tables(TableCache& C) {
+  const int dev = current_device();
+  forget_calls();  // the look-up's own references
+  std::atomic_thread_fence(std::memory_order_acquire);
+  if (cudaDeviceSynchronize() != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  size_t freed = 0;
+  for (auto it = C.passes.begin(); it != C.passes.end();)
+    it = std::get<0>(it->first) == dev && (it->second->none || it->second.use_count() == 1) ? C.passes.erase(it)
+                                                                                            : std::next(it);
+  for (auto it = C.steps.begin(); it != C.steps.end();) {
+    if (std::get<0>(it->first) == dev && it->second.use_count() == 1) {
+      freed += it->second->bytes;
+      it = C.steps.erase(it);
+    } else {
+      ++it;
+    }
+  }
+  for (auto it = C.powers.begin(); it != C.powers.end();) {
+    if (std::get<0>(it->first) == dev && !it->second.pinned && it->second.table.use_count() == 1) {
+      freed += it->second.table->bytes;
+      it = C.powers.erase(it);
+    } else {
+      ++it;
+    }
+  }
+  return freed > 0;
+}
+
+// dev_alloc with C.mu held, for a call on stream `s` (nothing is given back under capture).
+static int dev_alloc_locked(TableCache& C, void** p, size_t bytes, cudaStream_t s) {
+  int rc = dev_alloc_plain(p, bytes);
+  if (rc == GSN_ERR_NOMEM && !capturing(s) && give_back_tables(C)) rc = dev_alloc_plain(p, bytes);
+  return rc;
+}
+
+int dev_alloc(void** p, size_t bytes) {
+  int rc = dev_alloc_plain(p, bytes);
+  if (rc != GSN_ERR_NOMEM) return rc;
+  TableCache& C = cache();
+  std::lock_guard<std::mutex> g(C.mu);
+  return give_back_tables(C) ? dev_alloc_plain(p, bytes) : rc;
 }
 
 static std::string limbs_key(const uint32_t* x, int n) {
@@ -329,50 +402,51 @@ static void inv_memo(const FieldOps& F, const uint32_t* x, uint32_t* out) {
 }
 
 // Returns a cached table of base^e for e in [0, 2^log_count), entries as
-// fe_mul_tw takes them; builds it on first use.  Caller holds no lock.
-static int powers_table(const FieldOps& F, const uint32_t* base, int log_count, const uint32_t** out) {
+// fe_mul_tw takes them, held by T (Tables or PassTables); builds it on first use.  Caller holds no lock.
+// optional: the caller does without it when there is no memory, so nothing is given back for it.
+template <class Holder>
+static int powers_table(const FieldOps& F, const uint32_t* base, int log_count, const uint32_t** out, Holder* T,
+                        cudaStream_t s, bool pin, bool optional = false) {
   TableCache& C = cache();
   const int dev = current_device();
   std::lock_guard<std::mutex> g(C.mu);
   auto key = std::make_tuple(dev, F.id, log_count, limbs_key(base, F.limbs));
   auto it = C.powers.find(key);
-  if (it != C.powers.end()) {
-    *out = static_cast<const uint32_t*>(it->second.p);
-    return GSN_OK;
+  if (it == C.powers.end()) {
+    cudaStream_t& gen = C.gen_stream[dev];
+    if (!gen) GSN_CUDA(cudaStreamCreateWithFlags(&gen, cudaStreamNonBlocking));
+    const uint64_t count = (uint64_t)1 << log_count;
+    auto b = std::make_shared<Table>();
+    b->bytes = table_words(F, count) * sizeof(uint32_t);
+    int rc = optional ? dev_alloc_plain(&b->p, b->bytes) : dev_alloc_locked(C, &b->p, b->bytes, s);
+    if (rc) return rc;
+    cudaError_t e = F.powers(static_cast<uint32_t*>(b->p), count, base, gen);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(gen);
+    if (e != cudaSuccess) return cuda_fail(e, "twiddle generation");
+    count_launches(1);
+    it = C.powers.emplace(key, TableCache::Powers{b, false}).first;
   }
-  cudaStream_t& gen = C.gen_stream[dev];
-  if (!gen) GSN_CUDA(cudaStreamCreateWithFlags(&gen, cudaStreamNonBlocking));
-  const uint64_t count = (uint64_t)1 << log_count;
-  DevBuf b;
-  b.bytes = table_words(F, count) * sizeof(uint32_t);
-  int rc = dev_alloc(&b.p, b.bytes);
-  if (rc) return rc;
-  cudaError_t e = F.powers(static_cast<uint32_t*>(b.p), count, base, gen);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(gen);
-  if (e != cudaSuccess) {
-    dev_free(b.p);
-    return cuda_fail(e, "twiddle generation");
-  }
-  count_launches(1);
-  C.powers[key] = b;
-  *out = static_cast<const uint32_t*>(b.p);
+  it->second.pinned = it->second.pinned || pin;
+  T->held.push_back(it->second.table);
+  *out = static_cast<const uint32_t*>(it->second.table->p);
   return GSN_OK;
 }
 
 // The default root table covering log_n: reuse any cached default table of
 // order >= 2^log_n (its powers include every smaller root's), else build one
 // of order 2^max(log_n, default_tw_log).
-static int default_twiddles(const FieldOps& F, int log_n, const uint32_t** tw, int* tw_log) {
+static int default_twiddles(const FieldOps& F, int log_n, const uint32_t** tw, int* tw_log, Tables* T, cudaStream_t s) {
   if (find_default_twiddles(F, log_n, tw, tw_log)) return GSN_OK;
   const int k = std::min(F.max_log_n, std::max(log_n, F.default_tw_log));
   uint32_t r[kMaxLimbs];
   default_root(F, k, r);
   *tw_log = k;
-  return powers_table(F, r, k, tw);
+  return powers_table(F, r, k, tw, T, s, /*pin=*/true);
 }
 
 int resolve_tables(const FieldOps& F, uint32_t log_n, const uint32_t* omega, int dir, const uint32_t* shift,
-                   Tables* T, cudaStream_t) {
+                   Tables* T, cudaStream_t stream) {
+  T->held.clear();
   if ((int)log_n > F.max_log_n || (int)log_n > F.two_adicity)
     return set_error(GSN_ERR_SIZE, "log_n=%u exceeds the limit %d for field %d", log_n,
                      std::min(F.max_log_n, F.two_adicity), F.id);
@@ -382,13 +456,13 @@ int resolve_tables(const FieldOps& F, uint32_t log_n, const uint32_t* omega, int
   default_root(F, (int)log_n, def);
   int rc;
   if (!omega || std::memcmp(omega, def, sizeof(uint32_t) * N) == 0) {
-    rc = default_twiddles(F, (int)log_n, &T->tw, &T->tw_log);
+    rc = default_twiddles(F, (int)log_n, &T->tw, &T->tw_log, T, stream);
   } else {
     if (!F.is_canonical(omega)) return set_error(GSN_ERR_OMEGA, "omega is not reduced below the modulus");
     if (!F.is_primitive(omega, (int)log_n))
       return set_error(GSN_ERR_OMEGA, "omega is not a primitive 2^%u-th root of unity", log_n);
     T->tw_log = (int)log_n;
-    rc = powers_table(F, omega, (int)log_n, &T->tw);
+    rc = powers_table(F, omega, (int)log_n, &T->tw, T, stream, T->pin);
   }
   if (rc) return rc;
   std::memcpy(T->root, omega ? omega : def, sizeof(uint32_t) * N);
@@ -408,11 +482,11 @@ int resolve_tables(const FieldOps& F, uint32_t log_n, const uint32_t* omega, int
     for (int i = 0; i < N; ++i) zero = zero && s[i] == 0;
     if (zero) return set_error(GSN_ERR_ARG, "coset shift must be non-zero");
     if (dir == GSN_COSET_FORWARD) {
-      rc = powers_table(F, s, (int)log_n, &T->pre_table);
+      rc = powers_table(F, s, (int)log_n, &T->pre_table, T, stream, T->pin);
     } else {
       uint32_t si[kMaxLimbs];
       inv_memo(F, s, si);
-      rc = powers_table(F, si, (int)log_n, &T->post_table);
+      rc = powers_table(F, si, (int)log_n, &T->post_table, T, stream, T->pin);
     }
     if (rc) return rc;
   }
@@ -428,7 +502,8 @@ bool find_default_twiddles(const FieldOps& F, int log_n, const uint32_t** tw, in
     default_root(F, k, r);
     auto it = C.powers.find(std::make_tuple(dev, F.id, k, limbs_key(r, F.limbs)));
     if (it != C.powers.end()) {
-      *tw = static_cast<const uint32_t*>(it->second.p);
+      it->second.pinned = true;  // the caller takes no reference
+      *tw = static_cast<const uint32_t*>(it->second.table->p);
       *tw_log = k;
       return true;
     }
@@ -436,7 +511,7 @@ bool find_default_twiddles(const FieldOps& F, int log_n, const uint32_t** tw, in
   return false;
 }
 
-int resolve_p32_tables(const FieldOps& F, const Plan& plan, Tables* T) {
+int resolve_p32_tables(const FieldOps& F, const Plan& plan, Tables* T, cudaStream_t s) {
   uint32_t root[kMaxLimbs];
   std::memcpy(root, T->root, sizeof(uint32_t) * F.limbs);
   const int L = plan.log_n;
@@ -452,15 +527,15 @@ int resolve_p32_tables(const FieldOps& F, const Plan& plan, Tables* T) {
     const int r = plan.radix_log[p];
     uint32_t wr[kMaxLimbs];
     F.pow(root, (uint64_t)1 << (L - r), wr);  // a primitive 2^r-th root
-    int rc = powers_table(F, wr, r - 1, &T->p32_tile[p]);
+    int rc = powers_table(F, wr, r - 1, &T->p32_tile[p], T, s, T->pin);
     if (rc) return rc;
   }
   T->p32_lo_bits = (L + 1) / 2;
-  int rc = powers_table(F, root, T->p32_lo_bits, &T->p32_lo);
+  int rc = powers_table(F, root, T->p32_lo_bits, &T->p32_lo, T, s, T->pin);
   if (rc) return rc;
   uint32_t hb[kMaxLimbs];
   F.pow(root, (uint64_t)1 << T->p32_lo_bits, hb);
-  return powers_table(F, hb, L - T->p32_lo_bits, &T->p32_hi);
+  return powers_table(F, hb, L - T->p32_lo_bits, &T->p32_hi, T, s, T->pin);
 }
 
 void full_table_passes(const Plan& plan, Tables* T) {
@@ -473,7 +548,7 @@ void full_table_passes(const Plan& plan, Tables* T) {
 
 // Entry k 2^inner + j = w^(j k), w = (root of `tw`)^(2^shift) of order 2^(r + inner); key_root names w.
 static int step_table(const FieldOps& F, const uint32_t* tw, int shift, int r, int inner, const uint32_t* key_root,
-                      const uint32_t** out) {
+                      const uint32_t** out, PassTables* T) {
   TableCache& C = cache();
   const int dev = current_device();
   std::lock_guard<std::mutex> g(C.mu);
@@ -482,27 +557,19 @@ static int step_table(const FieldOps& F, const uint32_t* tw, int shift, int r, i
   if (it == C.steps.end()) {
     cudaStream_t& gen = C.gen_stream[dev];
     if (!gen) GSN_CUDA(cudaStreamCreateWithFlags(&gen, cudaStreamNonBlocking));
-    DevBuf b;
-    b.bytes = table_words(F, (uint64_t)1 << (r + inner)) * sizeof(uint32_t);
-    int rc = dev_alloc(&b.p, b.bytes);
+    auto b = std::make_shared<Table>();
+    b->bytes = table_words(F, (uint64_t)1 << (r + inner)) * sizeof(uint32_t);
+    int rc = dev_alloc_plain(&b->p, b->bytes);
     if (rc) return rc;
-    cudaError_t e = F.step_table(static_cast<uint32_t*>(b.p), tw, r, inner, shift, gen);
+    cudaError_t e = F.step_table(static_cast<uint32_t*>(b->p), tw, r, inner, shift, gen);
     if (e == cudaSuccess) e = cudaStreamSynchronize(gen);
-    if (e != cudaSuccess) {
-      dev_free(b.p);
-      return cuda_fail(e, "four-step table");
-    }
+    if (e != cudaSuccess) return cuda_fail(e, "four-step table");
     count_launches(1);
     it = C.steps.emplace(key, b).first;
   }
-  *out = static_cast<const uint32_t*>(it->second.p);
+  T->held.push_back(it->second);
+  *out = static_cast<const uint32_t*>(it->second->p);
   return GSN_OK;
-}
-
-static bool capturing(cudaStream_t s) {
-  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-  if (s && cudaStreamIsCapturing(s, &cap) != cudaSuccess) cudaGetLastError();
-  return cap != cudaStreamCaptureStatusNone;
 }
 
 int resolve_pass_tables(const FieldOps& F, const Plan& plan, Tables* T, cudaStream_t s) {
@@ -515,18 +582,15 @@ int resolve_pass_tables(const FieldOps& F, const Plan& plan, Tables* T, cudaStre
   std::string tail = limbs_key(T->root, F.limbs);
   for (int p = 0; p < plan.npass; ++p) tail.push_back((char)plan.radix_log[p]);
   const auto key = std::make_tuple(dev, F.id, L, tail);
-  PassTables t;
-  bool found = false;
+  std::shared_ptr<const PassTables> found;
   {
     std::lock_guard<std::mutex> g(C.mu);
     auto it = C.passes.find(key);
-    if (it != C.passes.end()) {
-      t = it->second;
-      found = true;
-    }
+    if (it != C.passes.end() && !(it->second->none && T->pin)) found = it->second;
   }
   if (!found) {
     if (capturing(s)) return GSN_OK;
+    auto t = std::make_shared<PassTables>();
     uint32_t def[kMaxLimbs];
     default_root(F, L, def);
     const bool is_def = std::memcmp(T->root, def, sizeof(uint32_t) * F.limbs) == 0;
@@ -537,40 +601,44 @@ int resolve_pass_tables(const FieldOps& F, const Plan& plan, Tables* T, cudaStre
         F.pow(T->root, (uint64_t)1 << (L - order_log), out);
       }
     };
-    int outer = 0;
-    for (int p = 0; p < plan.npass; ++p) {
+    int outer = 0, rc = GSN_OK;
+    for (int p = 0; p < plan.npass && !rc; ++p) {
       const int r = plan.radix_log[p], left = L - outer;
       uint32_t w[kMaxLimbs];
-      t.stage[p] = t.step[p] = nullptr;
-      int rc = GSN_OK;
       if (r >= 1) {
         power(r, w);
-        rc = powers_table(F, w, r - 1, &t.stage[p]);
+        rc = powers_table(F, w, r - 1, &t->stage[p], t.get(), s, T->pin, /*optional=*/true);
       }
       if (!rc && p < plan.npass - 1) {
         power(left, w);
-        rc = step_table(F, T->tw, T->tw_log - left, r, left - r, w, &t.step[p]);
+        rc = step_table(F, T->tw, T->tw_log - left, r, left - r, w, &t->step[p], t.get());
       }
-      if (rc == GSN_ERR_NOMEM) return GSN_OK;
-      if (rc) return rc;
       outer += r;
+    }
+    if (rc == GSN_ERR_NOMEM) {
+      t = std::make_shared<PassTables>();
+      t->none = true;
+    } else if (rc) {
+      return rc;
     }
     std::lock_guard<std::mutex> g(C.mu);
     C.passes[key] = t;
+    found = t;
   }
+  T->held.push_back(found);
   for (int p = 0; p < plan.npass; ++p) {
-    if (t.stage[p]) {
-      T->stage[p] = t.stage[p];
+    if (found->stage[p]) {
+      T->stage[p] = found->stage[p];
       T->stage_shift[p] = 0;
     }
-    T->step[p] = t.step[p];
+    T->step[p] = found->step[p];
   }
   T->own_passes = true;
   return GSN_OK;
 }
 
 int resolve_plan_tables(const FieldOps& F, const Plan& plan, Tables* T, cudaStream_t s) {
-  return plan.kernel == kKernelP32 ? resolve_p32_tables(F, plan, T) : resolve_pass_tables(F, plan, T, s);
+  return plan.kernel == kKernelP32 ? resolve_p32_tables(F, plan, T, s) : resolve_pass_tables(F, plan, T, s);
 }
 
 int scratch_for(cudaStream_t s, size_t bytes, uint32_t** out, int slot) {
@@ -585,7 +653,7 @@ int scratch_for(cudaStream_t s, size_t bytes, uint32_t** out, int slot) {
       b.p = nullptr;
       b.bytes = 0;
     }
-    int rc = dev_alloc(&b.p, bytes);
+    int rc = dev_alloc_locked(C, &b.p, bytes, s);
     if (rc) return rc;
     b.bytes = bytes;
   }
@@ -703,9 +771,9 @@ struct Calls {
   uint64_t generation = 0;
   // (device, field, log_n, direction, 16-byte aligned, within a QAP computation, omega limbs, shift limbs; empty
   // strings for the defaults)
-  std::map<std::tuple<int, int, uint32_t, int, bool, bool, std::string, std::string>, Call> known;
+  std::map<std::tuple<int, int, uint32_t, int, bool, bool, std::string, std::string>, std::shared_ptr<const Call>> known;
 };
-constexpr size_t kMaxCalls = 4096;  // about 1 KB each
+constexpr size_t kMaxCalls = 4096;  // about 1 KB each; the tables they hold are given back when memory runs out
 static Calls& calls() {
   static Calls* c = new Calls();
   return *c;
@@ -724,7 +792,8 @@ constexpr uint32_t kLanesMaxLogQap = 12;
 
 // ptrs: the arrays, and the caller's scratch, whose alignment counts; qap: a step of a QAP computation.
 static int resolve_call(const FieldOps& F, uint32_t log_n, const uint32_t* omega, int dir, const uint32_t* shift,
-                        const void* const* ptrs, int count, bool qap, cudaStream_t s, Call* out) {
+                        const void* const* ptrs, int count, bool qap, cudaStream_t s,
+                        std::shared_ptr<const Call>* out) {
   bool aligned = true;  // the multi-limb fields' arrays always are
   for (int i = 0; i < count; ++i) aligned = aligned && reinterpret_cast<uintptr_t>(ptrs[i]) % 16 == 0;
   const auto key = std::make_tuple(current_device(), F.id, log_n, dir, aligned, qap,
@@ -741,29 +810,39 @@ static int resolve_call(const FieldOps& F, uint32_t log_n, const uint32_t* omega
     }
     generation = K.generation;
   }
-  int rc = resolve_tables(F, log_n, omega, dir, shift, &out->tables, s);
+  auto call = std::make_shared<Call>();
+  int rc = resolve_tables(F, log_n, omega, dir, shift, &call->tables, s);
   if (rc) return rc;
-  out->plan = plan_for(F, (int)log_n);
-  if (out->plan.kernel == kKernelP32 && !aligned) {
+  call->plan = plan_for(F, (int)log_n);
+  if (call->plan.kernel == kKernelP32 && !aligned) {
     // the register-blocked 32-bit pass moves 16-byte vectors; 4-byte-aligned arrays take the generic pass
     const FieldLimits L = limits_of(F);
-    out->plan = make_plan(F, (int)log_n, L.max_r, L.target_j, L.max_block);
+    call->plan = make_plan(F, (int)log_n, L.max_r, L.target_j, L.max_block);
   }
-  if (out->plan.kernel == kKernelLanes && qap && log_n > kLanesMaxLogQap) {
+  if (call->plan.kernel == kKernelLanes && qap && log_n > kLanesMaxLogQap) {
     // two near-equal passes, or more where a radix would pass the field's usual limit (2^12 does not fit shared memory)
     const int npass = std::max(2, ((int)log_n + limits_of(F).max_r - 1) / limits_of(F).max_r);
     int radix[kMaxPasses] = {0, 0, 0, 0};
     for (int i = 0; i < npass; ++i) radix[i] = (int)log_n * (i + 1) / npass - (int)log_n * i / npass;
-    out->plan = make_split_plan(F, (int)log_n, radix, npass, /*target_j=*/0, 128);
+    call->plan = make_split_plan(F, (int)log_n, radix, npass, /*target_j=*/0, 128);
   }
-  rc = resolve_plan_tables(F, out->plan, &out->tables, s);
+  rc = resolve_plan_tables(F, call->plan, &call->tables, s);
   if (rc) return rc;
-  if (out->plan.kernel == kKernelP32 || out->tables.own_passes) {
+  *out = call;
+  if (call->plan.kernel == kKernelP32 || call->tables.own_passes) {
     std::lock_guard<std::mutex> g(K.mu);
     if (K.known.size() >= kMaxCalls) K.known.clear();  // a shift drawn anew for every call
-    if (K.generation == generation) K.known.emplace(key, *out);
+    if (K.generation == generation) K.known.emplace(key, call);
   }
   return GSN_OK;
+}
+
+// A captured call's tables stay as long as its graph may run.
+static void hold_captured(const std::shared_ptr<const Call>& call, cudaStream_t s) {
+  if (!capturing(s)) return;
+  TableCache& C = cache();
+  std::lock_guard<std::mutex> g(C.mu);
+  C.captured.insert(call);
 }
 
 static int ntt_impl(int field, uint32_t* data, uint32_t log_n, const uint32_t* omega, int dir,
@@ -776,16 +855,17 @@ static int ntt_impl(int field, uint32_t* data, uint32_t log_n, const uint32_t* o
     rc = check_data_ptr(*F, scratch);
     if (rc) return rc;
   }
-  Call call;
+  std::shared_ptr<const Call> call;
   const void* const ptrs[2] = {data, scratch};
   rc = resolve_call(*F, log_n, omega, dir, shift, ptrs, 2, qap, s, &call);
   if (rc) return rc;
-  const Plan& plan = call.plan;
+  const Plan& plan = call->plan;
+  hold_captured(call, s);
   if (plan.npass > 1 && !scratch) {
     rc = scratch_for(s, ((size_t)1 << log_n) * F->limbs * sizeof(uint32_t), &scratch);
     if (rc) return rc;
   }
-  return enqueue_ntt(*F, plan, call.tables, data, scratch, s);
+  return enqueue_ntt(*F, plan, call->tables, data, scratch, s);
 }
 
 // zr2 = z * R^2 with z = 1 / Z(shift * w^i) = 1 / (shift^n - 1), the inverse vanishing polynomial of the
@@ -847,7 +927,7 @@ static int qap_arrays(const FieldOps& F, uint32_t* const* polys, uint32_t log_n,
     if (rc) return rc;
   }
   const void* const ptrs[kMaxArrays] = {polys[0], polys[1], polys[2]};
-  Call inv, fwd;
+  std::shared_ptr<const Call> inv, fwd;
   int rc = resolve_call(F, log_n, nullptr, GSN_INVERSE, nullptr, ptrs, kMaxArrays, true, s, &inv);
   if (!rc) rc = resolve_call(F, log_n, nullptr, GSN_COSET_FORWARD, shift, ptrs, kMaxArrays, true, s, &fwd);
   if (rc) return rc;
@@ -856,7 +936,7 @@ static int qap_arrays(const FieldOps& F, uint32_t* const* polys, uint32_t log_n,
   const size_t one = ((size_t)F.limbs << log_n) * sizeof(uint32_t);
   const size_t step = (one + 15) & ~(size_t)15, others = (kMaxArrays - 1) * step;  // 16-byte aligned
   uint32_t* scratch[kMaxArrays] = {nullptr, nullptr, nullptr};
-  if (std::max(inv.plan.npass, fwd.plan.npass) > 1) {
+  if (std::max(inv->plan.npass, fwd->plan.npass) > 1) {
     // growing a buffer would end a capture
     if (capturing(s) && (scratch_held(s, 0) < one || scratch_held(s, kScratchArrays) < others)) return GSN_ERR_NOMEM;
     rc = scratch_for(s, one, &scratch[0]);
@@ -864,8 +944,10 @@ static int qap_arrays(const FieldOps& F, uint32_t* const* polys, uint32_t log_n,
     if (rc) return rc;
     for (int i = 2; i < kMaxArrays; ++i) scratch[i] = scratch[1] + (i - 1) * (step / sizeof(uint32_t));
   }
-  rc = enqueue_ntts(F, inv.plan, inv.tables, polys, scratch, kMaxArrays, s);
-  return rc ? rc : enqueue_ntts(F, fwd.plan, fwd.tables, polys, scratch, kMaxArrays, s);
+  hold_captured(inv, s);
+  hold_captured(fwd, s);
+  rc = enqueue_ntts(F, inv->plan, inv->tables, polys, scratch, kMaxArrays, s);
+  return rc ? rc : enqueue_ntts(F, fwd->plan, fwd->tables, polys, scratch, kMaxArrays, s);
 }
 
 // Device buffers, streams and events of the host-memory entry points (gsn_ntt_host, gsn_ntt_host_batch).  A
@@ -1190,6 +1272,7 @@ int gsn_prepare(int field, uint32_t log_n, const uint32_t* omega) {
   const FieldOps* F = field_ops(field);
   if (!F) return set_error(GSN_ERR_FIELD, "unknown field %d", field);
   Tables T;
+  T.pin = true;
   int rc = resolve_tables(*F, log_n, omega, GSN_FORWARD, nullptr, &T, nullptr);
   if (rc || F->limbs == 1) return rc;
   return resolve_pass_tables(*F, plan_for(*F, (int)log_n), &T, nullptr);
@@ -1279,11 +1362,10 @@ int gsn_release_caches(void) {
   }
   TableCache& C = cache();
   std::lock_guard<std::mutex> g(C.mu);
-  for (auto& kv : C.powers) dev_free(kv.second.p);
-  C.powers.clear();
-  for (auto& kv : C.steps) dev_free(kv.second.p);
-  C.steps.clear();
+  C.captured.clear();
   C.passes.clear();
+  C.steps.clear();
+  C.powers.clear();
   for (auto& kv : C.scratch) dev_free(kv.second.p);
   C.scratch.clear();
   return GSN_OK;

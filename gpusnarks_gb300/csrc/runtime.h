@@ -5,6 +5,7 @@
 #include <cstdarg>
 #include <cstdint>
 #include <map>
+#include <memory>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -60,8 +61,12 @@ void set_tuned_plan(int field, int log_n, const Plan& p, int mode = 0);
 void clear_tuned_plans();
 bool get_tuned_plan(int field, int log_n, Plan* out, int mode = 0);
 
-// Resolved twiddle / coset tables for one transform.
+// Resolved twiddle / coset tables for one transform.  The tables named here stay in place while `held` lives: whoever
+// enqueues work on them keeps it until that is done, and whoever keeps their addresses (a batch, a captured call) as long
+// as those.  Tables that nobody holds are given back when device memory runs out (runtime.cu, give_back_tables).
 struct Tables {
+  std::vector<std::shared_ptr<const void>> held;
+  bool pin = false;  // asked for ahead of use: the powers resolved for this stay until the caches are released
   const uint32_t* tw = nullptr;
   int tw_log = 0;
   const uint32_t* pre_table = nullptr;
@@ -87,7 +92,7 @@ struct Tables {
 bool find_default_twiddles(const FieldOps& F, int log_n, const uint32_t** tw, int* tw_log);
 
 // Compact per-radix and two-level four-step tables for a kKernelP32 plan.
-int resolve_p32_tables(const FieldOps& F, const Plan& plan, Tables* T);
+int resolve_p32_tables(const FieldOps& F, const Plan& plan, Tables* T, cudaStream_t s);
 
 // Pass tables read from the full twiddle table alone: no allocation, no launch.
 void full_table_passes(const Plan& plan, Tables* T);
@@ -121,6 +126,7 @@ struct BatchPlan {
   int block = 0;
   size_t smem = 0;
   uint64_t elements = 0;
+  std::vector<std::shared_ptr<const void>> held;  // the tables that `jobs` names
 };
 // force: when non-null, every job uses this plan (the autotuner times
 // candidate plans this way); otherwise plan_for(..., batched=true).
@@ -132,7 +138,7 @@ uint64_t job_scratch_bytes(const FieldOps& F, const Plan& p);
 constexpr int kScratchArrays = 1, kScratchSums = 2;
 int scratch_for(cudaStream_t s, size_t bytes, uint32_t** out, int slot = 0);
 
-// Device allocation bookkeeping (for tests / stats).
+// Device memory; where there is none left, tables that nobody holds are given back first.
 int dev_alloc(void** p, size_t bytes);
 void dev_free(void* p);
 

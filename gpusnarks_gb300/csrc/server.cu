@@ -540,6 +540,7 @@ int gsn_server_warmup(gsn_server* S, int field, uint32_t lo, uint32_t hi) {
   for (uint32_t k = lo; k <= hi; ++k) {
     for (int dir = GSN_FORWARD; dir <= GSN_COSET_INVERSE; ++dir) {
       Tables T;
+      T.pin = true;
       int rc = resolve_tables(*F, k, nullptr, dir, nullptr, &T, nullptr);
       // the pass tables of the plan that such a request will run
       const bool single = request_work(F, k) > launch_work_cap(S);

@@ -130,7 +130,13 @@ int gsn_ntt_host(int field, uint32_t* data, uint32_t log_n, const uint32_t* omeg
 int gsn_ntt_host_batch(int field, uint32_t* const* data, size_t count, uint32_t log_n, const uint32_t* omega,
                        int dir, const uint32_t* shift);
 
-/* Build and cache the twiddle table for (field, log_n, omega). */
+/* Build and cache the twiddle tables for (field, log_n, omega).  Every call
+ * builds what it misses; the tables of roots and shifts that no running call,
+ * batch or captured graph uses are freed when a later allocation of this
+ * library finds no memory, except the default roots' and those asked for
+ * here, which stay until gsn_release_caches.  The four-step tables of a
+ * plan's passes are optional: without memory for them a transform reads the
+ * full table. */
 int gsn_prepare(int field, uint32_t log_n, const uint32_t* omega);
 
 /* a[i] = a[i] * b[i] mod p on device memory (canonical values). */
