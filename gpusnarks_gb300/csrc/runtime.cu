@@ -303,6 +303,7 @@ struct TableCache {
   std::set<std::shared_ptr<const Call>> captured;  // what captured graphs run, kept until the caches are released
   std::map<std::tuple<int, cudaStream_t, int>, DevBuf> scratch;
   std::map<int, cudaStream_t> gen_stream;  // per device
+  std::map<int, size_t> memory;            // per device: its memory in bytes
 };
 
 static TableCache& cache() {
@@ -348,6 +349,34 @@ static bool give_back_tables(TableCache& C) {
     }
   }
   return freed > 0;
+}
+
+// Room for a table of `need` bytes within half of the device's memory, which bounds what is kept of roots and shifts that
+// may never come again (pinned tables do not count).  At the bound everything out of use goes at once: a drain per
+// thousand tables of 2^20 elements, where dropping the oldest would drain for each.
+static bool table_room(TableCache& C, size_t need, cudaStream_t s) {
+  const int dev = current_device();
+  size_t& total = C.memory[dev];
+  if (total == 0) {
+    size_t avail = 0;
+    if (cudaMemGetInfo(&avail, &total) != cudaSuccess) {
+      cudaGetLastError();
+      total = 0;
+      return true;
+    }
+  }
+  auto fits = [&] {
+    size_t kept = need;
+    for (const auto& kv : C.steps)
+      if (std::get<0>(kv.first) == dev) kept += kv.second->bytes;
+    for (const auto& kv : C.powers)
+      if (std::get<0>(kv.first) == dev && !kv.second.pinned) kept += kv.second.table->bytes;
+    return kept <= total / 2;
+  };
+  if (fits()) return true;
+  if (capturing(s)) return false;
+  give_back_tables(C);
+  return fits();
 }
 
 // dev_alloc with C.mu held, for a call on stream `s` (nothing is given back under capture).
@@ -418,6 +447,7 @@ static int powers_table(const FieldOps& F, const uint32_t* base, int log_count, 
     const uint64_t count = (uint64_t)1 << log_count;
     auto b = std::make_shared<Table>();
     b->bytes = table_words(F, count) * sizeof(uint32_t);
+    if (!pin) table_room(C, b->bytes, s);  // held tables may be more than the bound
     int rc = optional ? dev_alloc_plain(&b->p, b->bytes) : dev_alloc_locked(C, &b->p, b->bytes, s);
     if (rc) return rc;
     cudaError_t e = F.powers(static_cast<uint32_t*>(b->p), count, base, gen);
@@ -559,7 +589,8 @@ static int step_table(const FieldOps& F, const uint32_t* tw, int shift, int r, i
     if (!gen) GSN_CUDA(cudaStreamCreateWithFlags(&gen, cudaStreamNonBlocking));
     auto b = std::make_shared<Table>();
     b->bytes = table_words(F, (uint64_t)1 << (r + inner)) * sizeof(uint32_t);
-    int rc = dev_alloc_plain(&b->p, b->bytes);
+    int rc = table_room(C, b->bytes, nullptr) ? dev_alloc_plain(&b->p, b->bytes)
+                                              : set_error(GSN_ERR_NOMEM, "held tables take half of the device's memory");
     if (rc) return rc;
     cudaError_t e = F.step_table(static_cast<uint32_t*>(b->p), tw, r, inner, shift, gen);
     if (e == cudaSuccess) e = cudaStreamSynchronize(gen);

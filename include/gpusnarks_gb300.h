@@ -133,7 +133,7 @@ int gsn_ntt_host_batch(int field, uint32_t* const* data, size_t count, uint32_t 
 /* Build and cache the twiddle tables for (field, log_n, omega).  Every call
  * builds what it misses; the tables of roots and shifts that no running call,
  * batch or captured graph uses are freed when a later allocation of this
- * library finds no memory, except the default roots' and those asked for
+ * library finds no memory or they reach half of the device's, except the default roots' and those asked for
  * here, which stay until gsn_release_caches.  The four-step tables of a
  * plan's passes are optional: without memory for them a transform reads the
  * full table. */

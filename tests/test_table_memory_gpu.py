@@ -146,3 +146,29 @@ def test_threads_under_pressure(gsn, cuda_device):
             t.join(120)
         assert not any(t.is_alive() for t in threads)
     assert not errors, errors[0]
+
+
+def test_tables_are_bounded(gsn, cuda_device):
+    """A shift drawn anew for every call: what is kept of them stays within half of the device's memory."""
+    import torch
+    from gpusnarks_gb300.batch import fill_random
+    f, log_n = gsn.BLS12_381, 24  # 1 GiB per shift
+    x = torch.empty(f.limbs << log_n, dtype=torch.int32, device="cuda")
+    fill_random(f, x, 0x5EED1620)
+    want = x.clone()
+    gsn.ntt(f, x)
+    gsn.ntt(f, x, direction=gsn.INVERSE)
+    torch.cuda.synchronize()
+    free, total = torch.cuda.mem_get_info()
+    least = free
+    try:
+        for i in range((total >> 30) * 11 // 20):
+            gsn.ntt(f, x, direction=gsn.COSET_FORWARD, shift=3 + i)
+            least = min(least, torch.cuda.mem_get_info()[0])
+        assert free - least <= total // 2 + (4 << 30)
+        x.copy_(want)
+        gsn.ntt(f, x, direction=gsn.COSET_FORWARD, shift=3)
+        gsn.ntt(f, x, direction=gsn.COSET_INVERSE, shift=3)
+        assert torch.equal(x, want)
+    finally:
+        gsn.load().gsn_release_caches()
