@@ -256,8 +256,15 @@ static int autotune_impl(int field, uint32_t lo, uint32_t hi, int reps, int mode
     Plan best;
     float best_ms = 1e30f;
     int timed = 0, skipped = 0;
-    for (const Plan& p : candidates(*F, (int)k)) {
+    // A candidate's pass tables go when the next split comes: those of all splits together (9 of 4.3 GB for BLS12-381 at
+    // 2^26) would fill the bound on tables, and later candidates would be timed without theirs.
+    const uint64_t mark = pass_tables_mark();
+    const int* split = nullptr;
+    const std::vector<Plan> plans = candidates(*F, (int)k);
+    for (const Plan& p : plans) {
       if (mode == 1 && p.kernel != kKernelGeneric) continue;
+      if (split && !std::equal(split, split + kMaxPasses, p.radix_log)) drop_pass_tables_since(mark);
+      split = p.radix_log;
       float ms = 0;
       int r = mode == 1 ? time_batch_plan(*F, p, data, scratch, batch_elems, reps, &ms)
                         : time_plan(*F, p, data, scratch, reps, &ms);
@@ -276,7 +283,10 @@ static int autotune_impl(int field, uint32_t lo, uint32_t hi, int reps, int mode
     if (verbose)
       std::fprintf(stderr, "autotune field %d mode %d 2^%u: %d timed, %d skipped, best %.4f ms\n", field, mode, k,
                    timed, skipped, best_ms);
+    drop_pass_tables_since(mark);
     if (best_ms < 1e30f) {
+      Tables T;  // the winner's again, for the calls that follow
+      if (!resolve_tables(*F, k, nullptr, GSN_FORWARD, nullptr, &T, nullptr)) resolve_plan_tables(*F, best, &T, nullptr);
       set_tuned_plan(F->id, (int)k, best, mode);
       {
         std::lock_guard<std::mutex> g(g_tuned_ms_mu);

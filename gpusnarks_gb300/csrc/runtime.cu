@@ -274,6 +274,7 @@ struct DevBuf {
 struct Table {
   void* p = nullptr;
   size_t bytes = 0;
+  uint64_t born = 0;  // four-step factors: TableCache::births when they were built
   ~Table() { dev_free(p); }
 };
 using TableRef = std::shared_ptr<const Table>;
@@ -281,6 +282,7 @@ using TableRef = std::shared_ptr<const Table>;
 struct PassTables {
   const uint32_t* stage[kMaxPasses] = {nullptr, nullptr, nullptr, nullptr};
   const uint32_t* step[kMaxPasses] = {nullptr, nullptr, nullptr, nullptr};
+  uint64_t born = 0;
   bool none = false;  // there was no memory for them: the full table is read until tables are given back
   std::vector<std::shared_ptr<const void>> held;
 };
@@ -303,6 +305,7 @@ struct TableCache {
   std::set<std::shared_ptr<const Call>> captured;  // what captured graphs run, kept until the caches are released
   std::map<std::tuple<int, cudaStream_t, int>, DevBuf> scratch;
   std::map<int, cudaStream_t> gen_stream;  // per device
+  uint64_t births = 0;                     // pass tables and their factors built so far
   std::map<int, size_t> memory;            // per device: its memory in bytes
 };
 
@@ -596,6 +599,7 @@ static int step_table(const FieldOps& F, const uint32_t* tw, int shift, int r, i
     if (e == cudaSuccess) e = cudaStreamSynchronize(gen);
     if (e != cudaSuccess) return cuda_fail(e, "four-step table");
     count_launches(1);
+    b->born = C.births++;
     it = C.steps.emplace(key, b).first;
   }
   T->held.push_back(it->second);
@@ -653,6 +657,7 @@ int resolve_pass_tables(const FieldOps& F, const Plan& plan, Tables* T, cudaStre
       return rc;
     }
     std::lock_guard<std::mutex> g(C.mu);
+    t->born = C.births++;
     C.passes[key] = t;
     found = t;
   }
@@ -666,6 +671,28 @@ int resolve_pass_tables(const FieldOps& F, const Plan& plan, Tables* T, cudaStre
   }
   T->own_passes = true;
   return GSN_OK;
+}
+
+uint64_t pass_tables_mark() {
+  TableCache& C = cache();
+  std::lock_guard<std::mutex> g(C.mu);
+  return C.births;
+}
+
+void drop_pass_tables_since(uint64_t mark) {
+  TableCache& C = cache();
+  std::lock_guard<std::mutex> g(C.mu);
+  const int dev = current_device();
+  if (C.births == mark || cudaDeviceSynchronize() != cudaSuccess) {
+    cudaGetLastError();
+    return;
+  }
+  for (auto it = C.passes.begin(); it != C.passes.end();)
+    it = std::get<0>(it->first) == dev && it->second->born >= mark && it->second.use_count() == 1 ? C.passes.erase(it)
+                                                                                                   : std::next(it);
+  for (auto it = C.steps.begin(); it != C.steps.end();)
+    it = std::get<0>(it->first) == dev && it->second->born >= mark && it->second.use_count() == 1 ? C.steps.erase(it)
+                                                                                                   : std::next(it);
 }
 
 int resolve_plan_tables(const FieldOps& F, const Plan& plan, Tables* T, cudaStream_t s) {

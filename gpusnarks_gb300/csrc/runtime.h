@@ -102,6 +102,10 @@ void full_table_passes(const Plan& plan, Tables* T);
 // when there is no memory for them, a plan whose tables are not there yet reads the full table instead.
 int resolve_pass_tables(const FieldOps& F, const Plan& plan, Tables* T, cudaStream_t s);
 
+// Frees the pass tables built since `mark` that nobody holds (the tuner's candidates).
+uint64_t pass_tables_mark();
+void drop_pass_tables_since(uint64_t mark);
+
 // The tables a plan's kernel needs beyond resolve_tables.
 int resolve_plan_tables(const FieldOps& F, const Plan& plan, Tables* T, cudaStream_t s);
 
