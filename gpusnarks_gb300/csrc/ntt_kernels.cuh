@@ -158,6 +158,10 @@ struct TileGeom {
   }
 };
 
+// CHAIN: the block's last stores are those of this tile, so the next kernel on the stream may be set up before them.  A
+// pass's block has one tile up to 2^20 of them.  Blocks of the batched kernel take tiles until none are left and let the
+// next kernel start as they end.
+
 // One tile of one pass, one-limb field.  `sm` holds 2^(log_r + log_j) words.  Small transforms and batches of them come
 // here (ntt_p32.cuh has the large ones), so latency and instructions count: a load phase (times the powers of the shift on
 // the first pass of a coset transform), radix-4 sub-steps of 4 rows a thread (one radix-2 stage first for odd log_r), and
@@ -173,7 +177,7 @@ __device__ __forceinline__ uint32_t word_slot(uint32_t i) {
   return i ^ ((u ^ (u << 2) ^ (u << 3) ^ (u >> 5)) & 31u);
 }
 
-template <class P>
+template <class P, bool CHAIN>
 __device__ void word_tile(const PassArgs& A, unsigned array, uint32_t tile, uint32_t* sm) {
   static_assert(P::N == 1, "one limb");
   const int lr = A.log_r, lj = A.log_j;
@@ -232,7 +236,7 @@ __device__ void word_tile(const PassArgs& A, unsigned array, uint32_t tile, uint
     }
     __syncthreads();
   }
-  chain_next();
+  if constexpr (CHAIN) chain_next();
 #pragma unroll 4
   for (uint32_t e = threadIdx.x; e < R * J; e += nthr) {
     const uint32_t k = e >> lj, jj = e & (J - 1u), pos = G.dst<P>(A, k, jj);
@@ -291,7 +295,7 @@ __device__ __forceinline__ void tile_sub(Fe<P>& r, const Fe<P>& x, const Fe<P>& 
   }
 }
 
-template <class P, int LJ>
+template <class P, int LJ, bool CHAIN>
 __device__ __forceinline__ void field_tile(const PassArgs& A, unsigned array, uint32_t tile, uint32_t* sm) {
   constexpr int N = P::N;
   const int lr = A.log_r, lj = LJ >= 0 ? LJ : A.log_j;
@@ -369,7 +373,7 @@ __device__ __forceinline__ void field_tile(const PassArgs& A, unsigned array, ui
       fe_store<P>(out, x);
     }
   };
-  chain_next();
+  if constexpr (CHAIN) chain_next();
 #pragma unroll 1
   for (uint32_t b = threadIdx.x; b < (lr > 0 ? (R >> 1) << lj : J); b += nthr) {
     const uint32_t jj = b & (J - 1u), t = b >> lj, r = bitrev_bits(t, lr);
@@ -414,9 +418,9 @@ __global__ void __maxnreg__(pass_max_regs<P>()) ntt_pass_kernel(const __grid_con
   chain_wait();
   for (uint64_t t = blockIdx.x; t < A.tiles; t += gridDim.x) {  // tiles < 2^28
     if constexpr (P::N == 1) {
-      word_tile<P>(A, array, (uint32_t)t, sm);
+      word_tile<P, true>(A, array, (uint32_t)t, sm);
     } else {
-      field_tile<P, LJ>(A, array, (uint32_t)t, sm);
+      field_tile<P, LJ, true>(A, array, (uint32_t)t, sm);
     }
   }
 }
@@ -670,9 +674,9 @@ __global__ void __maxnreg__(batch_max_regs<P>())
     __syncthreads();
     // each ends with __syncthreads(); s_args is rewritten only after it
     if constexpr (P::N == 1) {
-      word_tile<P>(s_args, 0, tile, sm);
+      word_tile<P, false>(s_args, 0, tile, sm);
     } else {
-      field_tile<P, -1>(s_args, 0, tile, sm);
+      field_tile<P, -1, false>(s_args, 0, tile, sm);
     }
     if (threadIdx.x == 0) {
       __threadfence();
