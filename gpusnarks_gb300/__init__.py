@@ -119,9 +119,10 @@ def _stream_handle(stream):
     if stream is None:
         import torch
         raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)
-        if raw is not None and torch.cuda.is_initialized():
+        device = getattr(torch._C, "_cuda_getDevice", None)
+        if raw is not None and device is not None and torch.cuda.is_initialized():
             # what torch.cuda.current_stream().cuda_stream is, without the stream object (3 us of a 10 us call)
-            return raw(torch._C._cuda_getDevice())
+            return raw(device())
         return torch.cuda.current_stream().cuda_stream
     if isinstance(stream, int):
         return stream
