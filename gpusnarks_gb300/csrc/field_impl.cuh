@@ -57,6 +57,7 @@ constexpr FieldOps make_field_ops(int max_log_n, int default_tw_log) {
                   &Kernels<P>::batch,
                   &Kernels<P>::batch_occupancy,
                   &Kernels<P>::load,
+                  &LanesKernels<P>::load,
                   &MultiexpKernels<P>::grid,
                   &MultiexpKernels<P>::partial_bytes,
                   &MultiexpKernels<P>::run,

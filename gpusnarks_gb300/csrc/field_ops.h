@@ -34,7 +34,8 @@ struct FieldOps {
                        uint32_t* counters_dev, uint32_t* status_dev, int grid, int block, size_t smem,
                        cudaStream_t s, long long wait_cycles /* <= 0: default (~1 s) */);
   int (*batch_occupancy)(int block, size_t smem);
-  cudaError_t (*load)();
+  cudaError_t (*load)();  // the code of the batched kernel and of the passes that run one array
+  cudaError_t (*load_lanes)();
   // sum_i a[i] b[i]: per-block partials of the first launch (multiexp_grid(n) of them, multiexp_bytes
   // in `partial`), then one block sums them into `out`; fix = the representation constant (multiexp.cuh)
   int (*multiexp_grid)(uint64_t n);

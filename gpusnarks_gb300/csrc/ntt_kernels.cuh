@@ -747,7 +747,8 @@ struct Kernels {
                                 wait_cycles > 0 ? wait_cycles : kWaitBudgetCycles);
     return cudaGetLastError();
   }
-  // Loads the transform kernels' code, which CUDA otherwise does at each one's first launch.
+  // Loads code that CUDA otherwise loads at each kernel's first launch: the batched kernel's and that of the passes that
+  // transform one array.
   static cudaError_t load() {
     cudaFuncAttributes attr;
     cudaError_t e = cudaFuncGetAttributes(&attr, batch_kernel<P>);

@@ -230,6 +230,13 @@ __global__ void __launch_bounds__(lanes::kMaxBlock) ntt_lanes_kernel(const __gri
 
 template <class P>
 struct LanesKernels {
+  static cudaError_t load() {
+    if constexpr (P::N == 24) {
+      cudaFuncAttributes attr;
+      return cudaFuncGetAttributes(&attr, ntt_lanes_kernel<P>);
+    }
+    return cudaSuccess;
+  }
   // Built for the 24-limb field only.
   static cudaError_t pass(const PassArgs& A, int arrays, int block, cudaStream_t s) {
     if constexpr (P::N != 24) {

@@ -559,9 +559,14 @@ namespace p32 {
 // the CTA's next tile), keeping at least two CTAs' worth of shared memory per SM.
 constexpr size_t kPipeTileMax = 48 * 1024;
 
+// arrays = 0: loads the kernel's code and launches nothing (load_plan).
 // buffers: tile-sized shared-memory buffers the kernel uses (1 plain, 2 with the column prefetch)
 template <class K>
 cudaError_t launch_kernel(K k, const P32Args& A, int arrays, int block, int grid_cap, cudaStream_t s, int buffers = 1) {
+  if (arrays == 0) {
+    cudaFuncAttributes attr;
+    return cudaFuncGetAttributes(&attr, k);
+  }
   P32Args B = A;
   B.pipe = buffers > 1 ? 1 : 0;
   const size_t tile = ((size_t)1 << (A.log_r + A.log_j)) * sizeof(uint32_t);

@@ -768,6 +768,21 @@ static int enqueue_p32(const Plan& plan, const Tables& T, uint32_t* const* data,
   return GSN_OK;
 }
 
+int load_plan(const FieldOps& F, const Plan& plan) {
+  cudaError_t e = plan.kernel == kKernelLanes ? F.load_lanes() : F.load();
+  if (plan.kernel == kKernelP32) {
+    P32Args A;
+    std::memset(&A, 0, sizeof(A));
+    for (int p = 0; p < plan.npass && e == cudaSuccess; ++p) {
+      A.last = p == plan.npass - 1;
+      A.log_r = plan.radix_log[p];
+      A.log_j = plan.log_j[p];
+      e = launch_p32_pass(A, /*arrays=*/0, plan.e_log, plan.block[p], 1, nullptr);
+    }
+  }
+  return e == cudaSuccess ? GSN_OK : cuda_fail(e, "kernel load");
+}
+
 int enqueue_ntt(const FieldOps& F, const Plan& plan, const Tables& T, uint32_t* data, uint32_t* scratch,
                 cudaStream_t s) {
   return enqueue_ntts(F, plan, T, &data, &scratch, 1, s);

@@ -109,6 +109,9 @@ void drop_pass_tables_since(uint64_t mark);
 // The tables a plan's kernel needs beyond resolve_tables.
 int resolve_plan_tables(const FieldOps& F, const Plan& plan, Tables* T, cudaStream_t s);
 
+// Loads the code of the kernels that a plan's passes run (CUDA otherwise does at each one's first launch).
+int load_plan(const FieldOps& F, const Plan& plan);
+
 // Validates arguments and resolves (and caches) all tables for a transform.
 int resolve_tables(const FieldOps& F, uint32_t log_n, const uint32_t* omega, int dir, const uint32_t* shift,
                    Tables* out, cudaStream_t s);

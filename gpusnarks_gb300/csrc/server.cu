@@ -534,19 +534,22 @@ int gsn_server_warmup(gsn_server* S, int field, uint32_t lo, uint32_t hi) {
   if (!S) return set_error(GSN_ERR_ARG, "null server");
   const FieldOps* F = field_ops(field);
   if (!F) return set_error(GSN_ERR_FIELD, "unknown field %d", field);
-  // a load waits for what is running: the first MNT4-753 launch took the scheduler 77 to 148 ms under load
-  const cudaError_t e = F->load();
-  if (e != cudaSuccess) return cuda_fail(e, "kernel load");
   for (uint32_t k = lo; k <= hi; ++k) {
+    Plan plan;
     for (int dir = GSN_FORWARD; dir <= GSN_COSET_INVERSE; ++dir) {
       Tables T;
       T.pin = true;
       int rc = resolve_tables(*F, k, nullptr, dir, nullptr, &T, nullptr);
+      if (rc) return rc;
       // the pass tables of the plan that such a request will run
       const bool single = request_work(F, k) > launch_work_cap(S);
-      if (!rc) rc = resolve_plan_tables(*F, plan_for(*F, (int)k, /*batched=*/!single), &T, nullptr);
+      plan = plan_for(*F, (int)k, /*batched=*/!single);
+      rc = resolve_plan_tables(*F, plan, &T, nullptr);
       if (rc) return rc;
     }
+    // a load waits for what is running: the first MNT4-753 launch took the scheduler 77 to 148 ms under load
+    int rc = load_plan(*F, plan);
+    if (rc) return rc;
   }
   return GSN_OK;
 }
