@@ -10,7 +10,8 @@
 // hard-codes 0xFFFFFFFF, device_field_operators.h:47).
 //
 // Element layout is the reference's: uint32_t limbs, little-endian
-// (cuda/device_field.h:75).  All functions keep values canonical, in [0, p).
+// (cuda/device_field.h:75).  Values are canonical, in [0, p), where a function's
+// comment gives no wider range (K = 2: below 2p; the unreduced sums: below 2^k p).
 // Montgomery products compute a*b*R^-1 mod p with R = 2^(32*N); they serve
 // products of two data elements.  The transform's products are by table
 // constants: fe_mul_tw computes x*w whatever representation x is held in

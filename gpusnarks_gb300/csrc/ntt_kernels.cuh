@@ -692,6 +692,7 @@ constexpr uint64_t kGridPerSm = 64;
 template <class P>
 struct Kernels {
   using PassKernel = void (*)(PassArgs);
+  static constexpr bool kManyOnly = P::N >= 16;  // one array goes by the many-array form too
   template <bool MANY>
   static PassKernel kernel_for(int log_j) {
     if constexpr (P::N > 1) {
@@ -705,7 +706,7 @@ struct Kernels {
   }
   static cudaError_t pass(const PassArgs& A, int arrays, int block, cudaStream_t s) {
     const size_t smem = tile_words(P::N, (uint64_t)1 << (A.log_r + A.log_j)) * sizeof(uint32_t);
-    auto k = arrays == 1 && P::N < 16 ? kernel_for<P::N >= 16>(A.log_j) : kernel_for<true>(A.log_j);
+    auto k = arrays == 1 ? kernel_for<kManyOnly>(A.log_j) : kernel_for<true>(A.log_j);
     if (smem > kDefaultSmemOptIn) {
       cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
       if (e != cudaSuccess) return e;
@@ -753,7 +754,7 @@ struct Kernels {
     cudaFuncAttributes attr;
     cudaError_t e = cudaFuncGetAttributes(&attr, batch_kernel<P>);
     for (int lj = 0; lj <= 3 && e == cudaSuccess; ++lj)
-      e = cudaFuncGetAttributes(&attr, kernel_for<P::N >= 16>(lj));
+      e = cudaFuncGetAttributes(&attr, kernel_for<kManyOnly>(lj));
     return e;
   }
   static int batch_occupancy(int block, size_t smem) {

@@ -1,16 +1,17 @@
 // Pass kernel of small 24-limb transforms: four lanes per product.
 //
 // A small transform leaves most SMs with one warp per scheduler or none, and its time is the chain of dependent products
-// (log2 n + passes). One warp takes 5,500 cycles for a 24-limb product: 923 multiply-adds on carry chains of 6.6 cycles a
-// step (GB300). Here four neighbouring lanes share a product: lane g takes rows i = g mod 4 of its three limb products,
-// a quarter of the chain. Rows of one warp instruction have to start at one word, so each lane holds the operand shifted
+// (log2 n + passes). One warp alone takes 5,410 cycles for a 24-limb product, 899 multiply-adds on carry chains at 6.0
+// cycles a step (GB300); the product below takes it 1,920. Four neighbouring lanes share a product: lane g takes rows
+// i = g mod 4 of its three limb products, a quarter of the chain. Rows of one warp instruction have to start at one word, so each lane holds the operand shifted
 // up by g words (27 words) and multiplies row 4c of that by limb 4c + g of the constant. The partial sums are added
 // across the lanes by shuffles, which leaves the quotient and the product in all four. Additions, subtractions and the
 // tile's addressing are done by all four alike. Total work grows by half, so this is for sizes that do not fill the
 // chip; the plan says which kernel a size takes.
 //
-// The arithmetic is fe_mul_tw's, word product by word product (the quotient leaves out the same ones), so the bounds
-// and the results are the same: values in [0, 2p) until the last pass's store. Tables, tiles and phases are field_tile's.
+// The quotient leaves out the same word products as fe_mul_tw's, so it is the same number and so are the bounds and the
+// results, values in [0, 2p) until the last pass's store. The modulus's low limb is multiplied like the others here (by
+// limbs of R - p), where fe_mul_tw shifts and subtracts: modulo R that is the same. Tables, tiles and phases are field_tile's.
 #pragma once
 #include <cuda_runtime.h>
 

@@ -163,8 +163,10 @@ namespace {
 
 uint64_t elem_bytes(const FieldOps* F, uint32_t log_n) { return ((uint64_t)1 << log_n) * F->limbs * sizeof(uint32_t); }
 
-// Integer multiply-adds of one transform: (n/2) log2 n products of
-// 2 (2 s^2 + s) word multiply-adds each (s limbs).
+// Size of one transform as max_launch_work counts it: (n/2) log2 n products of
+// 2 (2 s^2 + s) word multiply-adds each (s limbs), a Montgomery product's.  The
+// products by table constants take fewer; the unit stays, so that a caller's cap
+// packs what it did.
 double request_work(const FieldOps* F, uint32_t log_n) {
   const double s = F->limbs;
   return std::ldexp(1.0, (int)log_n - 1) * std::max(1u, log_n) * 2.0 * (2.0 * s * s + s);

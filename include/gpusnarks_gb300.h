@@ -18,7 +18,8 @@
  * Element layout (all fields): an element is LIMBS little-endian uint32
  * words, exactly the reference's `uint32_t im_rep[SIZE]`
  * (cuda/device_field.h:75); an array of n elements is n*LIMBS words,
- * element-major.  Transforms are representation-agnostic (linear): the output
+ * element-major.  Input elements are reduced, below p (nothing checks it).
+ * Transforms are representation-agnostic (linear): the output
  * is in whatever representation the input was stored in (canonical or
  * Montgomery), reduced to [0, p).  `omega` and `shift` arguments are
  * canonical integers.
@@ -276,10 +277,11 @@ typedef struct gsn_server_config {
   uint64_t hbm_budget_bytes; /* device bytes for polynomials + scratch            */
   int32_t max_inflight;      /* persistent launches in flight at once (>= 1)      */
   int32_t max_batch_jobs;    /* cap on requests per launch (0 = 4096)             */
-  uint64_t max_launch_work;  /* cap on the integer multiply-adds packed into one
-                                launch, (n/2) log2 n x 2(2s^2+s) per request;
+  uint64_t max_launch_work;  /* cap on the work packed into one launch, in units
+                                of a Montgomery product's multiply-adds:
+                                (n/2) log2 n x 2(2s^2+s) per request;
                                 the leading ready request always goes
-                                (0 = 4e10, a few milliseconds of GPU time)       */
+                                (0 = 4e10, about 2 ms of GPU time)               */
   int32_t policy;            /* order in which ready requests are launched:
                                 GSN_SERVE_OLDEST_FIRST (0, default) or
                                 GSN_SERVE_LEAST_WORK_FIRST                       */
