@@ -87,8 +87,13 @@ const FieldOps* field_ops(int field) {
 // ---------------------------------------------------------------------------
 // device allocations
 // ---------------------------------------------------------------------------
+// The thread's last failed allocation found no memory: cudaMalloc also fails while another thread captures, and freeing
+// or remembering anything for that would be wrong.
+static thread_local bool t_no_memory = false;
+
 static int dev_alloc_plain(void** p, size_t bytes) {
   cudaError_t e = cudaMalloc(p, bytes ? bytes : 16);
+  t_no_memory = e == cudaErrorMemoryAllocation;
   if (e != cudaSuccess) {
     cudaGetLastError();
     *p = nullptr;
@@ -385,13 +390,13 @@ static bool table_room(TableCache& C, size_t need, cudaStream_t s) {
 // dev_alloc with C.mu held, for a call on stream `s` (nothing is given back under capture).
 static int dev_alloc_locked(TableCache& C, void** p, size_t bytes, cudaStream_t s) {
   int rc = dev_alloc_plain(p, bytes);
-  if (rc == GSN_ERR_NOMEM && !capturing(s) && give_back_tables(C)) rc = dev_alloc_plain(p, bytes);
+  if (rc == GSN_ERR_NOMEM && t_no_memory && !capturing(s) && give_back_tables(C)) rc = dev_alloc_plain(p, bytes);
   return rc;
 }
 
 int dev_alloc(void** p, size_t bytes) {
   int rc = dev_alloc_plain(p, bytes);
-  if (rc != GSN_ERR_NOMEM) return rc;
+  if (rc != GSN_ERR_NOMEM || !t_no_memory) return rc;
   TableCache& C = cache();
   std::lock_guard<std::mutex> g(C.mu);
   return give_back_tables(C) ? dev_alloc_plain(p, bytes) : rc;
@@ -592,8 +597,10 @@ static int step_table(const FieldOps& F, const uint32_t* tw, int shift, int r, i
     if (!gen) GSN_CUDA(cudaStreamCreateWithFlags(&gen, cudaStreamNonBlocking));
     auto b = std::make_shared<Table>();
     b->bytes = table_words(F, (uint64_t)1 << (r + inner)) * sizeof(uint32_t);
-    int rc = table_room(C, b->bytes, nullptr) ? dev_alloc_plain(&b->p, b->bytes)
-                                              : set_error(GSN_ERR_NOMEM, "held tables take half of the device's memory");
+    const bool room = table_room(C, b->bytes, nullptr);
+    t_no_memory = !room;
+    int rc = room ? dev_alloc_plain(&b->p, b->bytes)
+                  : set_error(GSN_ERR_NOMEM, "held tables take half of the device's memory");
     if (rc) return rc;
     cudaError_t e = F.step_table(static_cast<uint32_t*>(b->p), tw, r, inner, shift, gen);
     if (e == cudaSuccess) e = cudaStreamSynchronize(gen);
@@ -651,6 +658,7 @@ int resolve_pass_tables(const FieldOps& F, const Plan& plan, Tables* T, cudaStre
       outer += r;
     }
     if (rc == GSN_ERR_NOMEM) {
+      if (!t_no_memory) return GSN_OK;
       t = std::make_shared<PassTables>();
       t->none = true;
     } else if (rc) {
