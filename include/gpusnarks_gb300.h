@@ -359,8 +359,8 @@ int gsn_synchronize(void* stream);
 int gsn_host_alloc(void** ptr, size_t bytes);  /* pinned host memory */
 int gsn_host_free(void* ptr);
 /* Free twiddle tables, scratch and the host-path buffers (they are rebuilt on
- * next use).  Synchronises the device first.  gsn_batch objects and servers
- * hold table pointers: destroy them before calling this. */
+ * next use).  Synchronises the device first.  gsn_batch objects, servers and
+ * captured graphs hold table pointers: destroy them before calling this. */
 int gsn_release_caches(void);
 /* number of NTT-path kernel launches issued by this library so far */
 uint64_t gsn_kernel_launch_count(void);
