@@ -50,6 +50,7 @@ constexpr FieldOps make_field_ops(int max_log_n, int default_tw_log) {
                   &LanesKernels<P>::pass,
                   &Kernels<P>::powers,
                   &Kernels<P>::step_table,
+                  &Kernels<P>::stage_table,
                   &Kernels<P>::pointwise,
                   &Kernels<P>::quotient,
                   &Kernels<P>::fill,

@@ -24,6 +24,8 @@ struct FieldOps {
   // step table of a pass of radix 2^r (ntt_common.h) from the twiddle table: out entry k 2^inner + j is
   // tw entry (j k) << shift, k < 2^r, j < 2^inner (multi-limb fields)
   cudaError_t (*step_table)(uint32_t* out, const uint32_t* tw, int r, int inner, int shift, cudaStream_t s);
+  // stage table: out entry j is tw entry j << shift, j < 2^log_count (multi-limb fields)
+  cudaError_t (*stage_table)(uint32_t* out, const uint32_t* tw, int log_count, int shift, cudaStream_t s);
   cudaError_t (*pointwise)(uint32_t* a, const uint32_t* b, uint64_t n, cudaStream_t s);
   // a[i] = (a[i] b[i] - c[i]) z, zr2 = z R^2 (limbs)
   cudaError_t (*quotient)(uint32_t* a, const uint32_t* b, const uint32_t* c, uint64_t n, const uint32_t* zr2,

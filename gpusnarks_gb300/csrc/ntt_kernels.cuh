@@ -452,8 +452,10 @@ __global__ void gen_powers_kernel(uint32_t* out, uint64_t count, Fe<P> base) {
   }
 }
 
-// Entry k 2^inner + j of `out`: entry (j k) << shift of `tw`.  One thread per 16-byte chunk, 8 threads a line.
-template <class P>
+// Entry k 2^inner + j of `out`: entry (j k) << shift of `tw`, or j << shift where STAGE (r = 0).  One thread per 16-byte
+// chunk, 8 threads a line.  Stage twiddles are copied too: computed as powers, and with the host exponentiations that named
+// them, they took 510 us of a first call on a root of MNT4-753 2^18 (1515 us in all).
+template <class P, bool STAGE>
 __global__ void step_table_kernel(uint32_t* out, const uint32_t* tw, int r, int inner, int shift) {
   constexpr int CH = P::N / 2;  // chunks per entry
   const uint64_t count = (uint64_t)1 << (r + inner);
@@ -463,7 +465,7 @@ __global__ void step_table_kernel(uint32_t* out, const uint32_t* tw, int r, int 
     const uint32_t c = (uint32_t)((t >> 3) % CH);
     const uint32_t e = (uint32_t)((t >> 3) / CH * 8 + (t & 7));
     if (e >= count) continue;
-    const uint32_t from = ((e & ((1u << inner) - 1u)) * (e >> inner)) << shift;
+    const uint32_t from = (STAGE ? e : (e & ((1u << inner) - 1u)) * (e >> inner)) << shift;
     *reinterpret_cast<uint4*>(out + tw_offset<P>(e) + c * kTwChunk) =
         *reinterpret_cast<const uint4*>(tw + tw_offset<P>(from) + c * kTwChunk);
   }
@@ -725,6 +727,13 @@ struct Kernels {
     return cudaGetLastError();
   }
   static cudaError_t step_table(uint32_t* out, const uint32_t* tw, int r, int inner, int shift, cudaStream_t s) {
+    return copy_table<false>(out, tw, r, inner, shift, s);
+  }
+  static cudaError_t stage_table(uint32_t* out, const uint32_t* tw, int log_count, int shift, cudaStream_t s) {
+    return copy_table<true>(out, tw, 0, log_count, shift, s);
+  }
+  template <bool STAGE>
+  static cudaError_t copy_table(uint32_t* out, const uint32_t* tw, int r, int inner, int shift, cudaStream_t s) {
     if constexpr (P::N == 1) {
       return cudaErrorInvalidValue;  // its passes read `tw` itself
     } else {
@@ -732,7 +741,7 @@ struct Kernels {
       const uint64_t threads = ((uint64_t)1 << (r + inner)) * (P::N / 2);
       const uint64_t grid =
           std::min<uint64_t>(threads / block + 1, kGridPerSm * (uint64_t)current_device_sms());
-      step_table_kernel<P><<<(unsigned)grid, block, 0, s>>>(out, tw, r, inner, shift);
+      step_table_kernel<P, STAGE><<<(unsigned)grid, block, 0, s>>>(out, tw, r, inner, shift);
       return cudaGetLastError();
     }
   }

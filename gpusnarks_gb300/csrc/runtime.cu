@@ -288,6 +288,7 @@ struct PassTables {
   const uint32_t* stage[kMaxPasses] = {nullptr, nullptr, nullptr, nullptr};
   const uint32_t* step[kMaxPasses] = {nullptr, nullptr, nullptr, nullptr};
   uint64_t born = 0;
+  bool stages_only = false;  // a caller's root, seen once: without its four-step factors
   bool none = false;  // there was no memory for them: the full table is read until tables are given back
   std::vector<std::shared_ptr<const void>> held;
 };
@@ -303,7 +304,8 @@ struct TableCache {
     bool pinned;  // default roots, and what gsn_prepare or a server's warm-up asked for
   };
   std::map<std::tuple<int, int, int, std::string>, Powers> powers;
-  // (device, field, log2 of the order, r, root limbs) -> four-step factors of a pass of radix 2^r
+  // (device, field, log2 of the order, r, name of the root) -> four-step factors of a pass of radix 2^r; r = kStage: the
+  // stage twiddles of that order.  The name is empty for the default roots, else the caller's root and its order.
   std::map<std::tuple<int, int, int, int, std::string>, TableRef> steps;
   // (device, field, log_n, split, root limbs) -> the pass tables above, one lookup per call
   std::map<std::tuple<int, int, int, std::string>, std::shared_ptr<const PassTables>> passes;
@@ -439,11 +441,9 @@ static void inv_memo(const FieldOps& F, const uint32_t* x, uint32_t* out) {
 }
 
 // Returns a cached table of base^e for e in [0, 2^log_count), entries as
-// fe_mul_tw takes them, held by T (Tables or PassTables); builds it on first use.  Caller holds no lock.
-// optional: the caller does without it when there is no memory, so nothing is given back for it.
-template <class Holder>
-static int powers_table(const FieldOps& F, const uint32_t* base, int log_count, const uint32_t** out, Holder* T,
-                        cudaStream_t s, bool pin, bool optional = false) {
+// fe_mul_tw takes them, held by T; builds it on first use.  Caller holds no lock.
+static int powers_table(const FieldOps& F, const uint32_t* base, int log_count, const uint32_t** out, Tables* T,
+                        cudaStream_t s, bool pin) {
   TableCache& C = cache();
   const int dev = current_device();
   std::lock_guard<std::mutex> g(C.mu);
@@ -456,7 +456,7 @@ static int powers_table(const FieldOps& F, const uint32_t* base, int log_count, 
     auto b = std::make_shared<Table>();
     b->bytes = table_words(F, count) * sizeof(uint32_t);
     if (!pin) table_room(C, b->bytes, s);  // held tables may be more than the bound
-    int rc = optional ? dev_alloc_plain(&b->p, b->bytes) : dev_alloc_locked(C, &b->p, b->bytes, s);
+    int rc = dev_alloc_locked(C, &b->p, b->bytes, s);
     if (rc) return rc;
     cudaError_t e = F.powers(static_cast<uint32_t*>(b->p), count, base, gen);
     if (e == cudaSuccess) e = cudaStreamSynchronize(gen);
@@ -584,27 +584,30 @@ void full_table_passes(const Plan& plan, Tables* T) {
   }
 }
 
-// Entry k 2^inner + j = w^(j k), w = (root of `tw`)^(2^shift) of order 2^(r + inner); key_root names w.
-static int step_table(const FieldOps& F, const uint32_t* tw, int shift, int r, int inner, const uint32_t* key_root,
+// Entry k 2^inner + j = w^(j k), w = (root of `tw`)^(2^shift) of order 2^(r + inner), k < 2^r.  r = kStage: entry j = w^j,
+// w of order 2^(inner + 1).
+constexpr int kStage = -1;
+static int pass_table(const FieldOps& F, const uint32_t* tw, int shift, int r, int inner, const std::string& name,
                       const uint32_t** out, PassTables* T) {
   TableCache& C = cache();
   const int dev = current_device();
   std::lock_guard<std::mutex> g(C.mu);
-  auto key = std::make_tuple(dev, F.id, r + inner, r, limbs_key(key_root, F.limbs));
+  auto key = std::make_tuple(dev, F.id, r == kStage ? inner + 1 : r + inner, r, name);
   auto it = C.steps.find(key);
   if (it == C.steps.end()) {
     cudaStream_t& gen = C.gen_stream[dev];
     if (!gen) GSN_CUDA(cudaStreamCreateWithFlags(&gen, cudaStreamNonBlocking));
     auto b = std::make_shared<Table>();
-    b->bytes = table_words(F, (uint64_t)1 << (r + inner)) * sizeof(uint32_t);
+    b->bytes = table_words(F, (uint64_t)1 << (r == kStage ? inner : r + inner)) * sizeof(uint32_t);
     const bool room = table_room(C, b->bytes, nullptr);
     t_no_memory = !room;
     int rc = room ? dev_alloc_plain(&b->p, b->bytes)
                   : set_error(GSN_ERR_NOMEM, "held tables take half of the device's memory");
     if (rc) return rc;
-    cudaError_t e = F.step_table(static_cast<uint32_t*>(b->p), tw, r, inner, shift, gen);
+    uint32_t* const p = static_cast<uint32_t*>(b->p);
+    cudaError_t e = r == kStage ? F.stage_table(p, tw, inner, shift, gen) : F.step_table(p, tw, r, inner, shift, gen);
     if (e == cudaSuccess) e = cudaStreamSynchronize(gen);
-    if (e != cudaSuccess) return cuda_fail(e, "four-step table");
+    if (e != cudaSuccess) return cuda_fail(e, "pass table");
     count_launches(1);
     b->born = C.births++;
     it = C.steps.emplace(key, b).first;
@@ -628,33 +631,28 @@ int resolve_pass_tables(const FieldOps& F, const Plan& plan, Tables* T, cudaStre
   {
     std::lock_guard<std::mutex> g(C.mu);
     auto it = C.passes.find(key);
-    if (it != C.passes.end() && !(it->second->none && T->pin)) found = it->second;
+    if (it != C.passes.end()) found = it->second;
   }
-  if (!found) {
+  if (!found || found->stages_only || (found->none && T->pin)) {
     if (capturing(s)) return GSN_OK;
+    const bool seen = found != nullptr;
     auto t = std::make_shared<PassTables>();
     uint32_t def[kMaxLimbs];
     default_root(F, L, def);
-    const bool is_def = std::memcmp(T->root, def, sizeof(uint32_t) * F.limbs) == 0;
-    auto power = [&](int order_log, uint32_t* out) {  // root^(2^(L - order_log))
-      if (is_def) {
-        default_root(F, order_log, out);
-      } else {
-        F.pow(T->root, (uint64_t)1 << (L - order_log), out);
-      }
-    };
+    std::string name;
+    if (std::memcmp(T->root, def, sizeof(uint32_t) * F.limbs) != 0) {
+      name = limbs_key(T->root, F.limbs);
+      name.push_back((char)L);
+    }
+    // The factors cost a first call more than they save it, an array's worth of memory to map and to write (BLS12-381 2^20:
+    // 577 us in all with them, 411 before there were any), and a program may draw a root for every call.
+    t->stages_only = T->single && !seen && !name.empty() && plan.npass > 1;
     int outer = 0, rc = GSN_OK;
     for (int p = 0; p < plan.npass && !rc; ++p) {
       const int r = plan.radix_log[p], left = L - outer;
-      uint32_t w[kMaxLimbs];
-      if (r >= 1) {
-        power(r, w);
-        rc = powers_table(F, w, r - 1, &t->stage[p], t.get(), s, T->pin, /*optional=*/true);
-      }
-      if (!rc && p < plan.npass - 1) {
-        power(left, w);
-        rc = step_table(F, T->tw, T->tw_log - left, r, left - r, w, &t->step[p], t.get());
-      }
+      if (r >= 1) rc = pass_table(F, T->tw, T->tw_log - r, kStage, r - 1, name, &t->stage[p], t.get());
+      if (!rc && p < plan.npass - 1 && !t->stages_only)
+        rc = pass_table(F, T->tw, T->tw_log - left, r, left - r, name, &t->step[p], t.get());
       outer += r;
     }
     if (rc == GSN_ERR_NOMEM) {
@@ -677,7 +675,7 @@ int resolve_pass_tables(const FieldOps& F, const Plan& plan, Tables* T, cudaStre
     }
     T->step[p] = found->step[p];
   }
-  T->own_passes = true;
+  T->own_passes = !found->stages_only;
   return GSN_OK;
 }
 
@@ -892,6 +890,7 @@ static int resolve_call(const FieldOps& F, uint32_t log_n, const uint32_t* omega
     generation = K.generation;
   }
   auto call = std::make_shared<Call>();
+  call->tables.single = true;
   int rc = resolve_tables(F, log_n, omega, dir, shift, &call->tables, s);
   if (rc) return rc;
   call->plan = plan_for(F, (int)log_n);

@@ -66,6 +66,7 @@ bool get_tuned_plan(int field, int log_n, Plan* out, int mode = 0);
 // as those.  Tables that nobody holds are given back when device memory runs out (runtime.cu, give_back_tables).
 struct Tables {
   std::vector<std::shared_ptr<const void>> held;
+  bool single = false;  // one call, of a root that may never come again: its four-step factors wait for the second
   bool pin = false;  // asked for ahead of use: the powers resolved for this stay until the caches are released
   const uint32_t* tw = nullptr;
   int tw_log = 0;
@@ -98,8 +99,9 @@ int resolve_p32_tables(const FieldOps& F, const Plan& plan, Tables* T, cudaStrea
 void full_table_passes(const Plan& plan, Tables* T);
 
 // Pass tables of a multi-limb plan: the stage twiddles of each radix and the four-step
-// factors in the order the tiles take them, built once per (root, split) and cached.  While `s` is capturing, or
-// when there is no memory for them, a plan whose tables are not there yet reads the full table instead.
+// factors in the order the tiles take them, built once per (root, split) and cached.  While `s` is capturing, when
+// there is no memory for them, and the factors in the first call on a root of the caller's (Tables::single), a plan whose
+// tables are not there yet reads the full table instead.
 int resolve_pass_tables(const FieldOps& F, const Plan& plan, Tables* T, cudaStream_t s);
 
 // Frees the pass tables built since `mark` that nobody holds (the tuner's candidates).
