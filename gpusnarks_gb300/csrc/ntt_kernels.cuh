@@ -426,14 +426,13 @@ __global__ void __maxnreg__(pass_max_regs<P>()) ntt_pass_kernel(const __grid_con
 }
 
 // Entry e of `out`: base^e, for e in [0, count), in the form fe_mul_tw takes.
-// `base` is canonical.  Each thread produces kPowChunk consecutive powers: one
-// square-and-multiply for the first, then one product per entry.
-constexpr int kPowChunk = 32;
-
+// `base` is canonical.  Each thread produces `chunk` consecutive powers: one
+// square-and-multiply for the first, then one product (and for the multi-limb
+// fields one reduction, the quotient) per entry.
 template <class P>
-__global__ void gen_powers_kernel(uint32_t* out, uint64_t count, Fe<P> base) {
+__global__ void gen_powers_kernel(uint32_t* out, uint64_t count, Fe<P> base, int chunk) {
   const uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const uint64_t e0 = t * kPowChunk;
+  const uint64_t e0 = t * chunk;
   if (e0 >= count) return;
   Fe<P> bm, acc;
   fe_to_mont<P>(bm, base);
@@ -445,7 +444,7 @@ __global__ void gen_powers_kernel(uint32_t* out, uint64_t count, Fe<P> base) {
       if ((e0 >> bit) & 1) fe_mul<P>(acc, acc, bm);
     }
   }
-  const uint64_t end = (e0 + kPowChunk < count) ? e0 + kPowChunk : count;
+  const uint64_t end = (e0 + chunk < count) ? e0 + chunk : count;
   for (uint64_t e = e0; e < end; ++e) {
     fe_store_tw<P>(out + tw_offset<P>((uint32_t)e), acc);
     fe_mul<P>(acc, acc, bm);
@@ -691,6 +690,11 @@ __global__ void __maxnreg__(batch_max_regs<P>())
 // Elementwise grid-stride kernels launch at most this many CTAs per SM.
 constexpr uint64_t kGridPerSm = 64;
 
+// Multi-limb tables of powers up to this size have 8 entries a thread and one warp a block: they do not fill the chip, and a
+// thread's chain of entries is their time. First call on a shift, GB300, us, 32 entries and 8: MNT4-753 2^10 355 and 185,
+// 2^14 495 and 322, 2^18 785 and 760, 2^20 1950 and 2550; BLS12-381 2^16 178 and 157, 2^20 366 and 389.
+constexpr uint64_t kPowSmall = (uint64_t)1 << 18;
+
 template <class P>
 struct Kernels {
   using PassKernel = void (*)(PassArgs);
@@ -721,9 +725,10 @@ struct Kernels {
   static cudaError_t powers(uint32_t* out, uint64_t count, const uint32_t* base_canon, cudaStream_t s) {
     Fe<P> b;
     for (int i = 0; i < P::N; ++i) b.l[i] = base_canon[i];
-    const uint64_t threads = (count + kPowChunk - 1) / kPowChunk;
-    const int block = 128;
-    gen_powers_kernel<P><<<(unsigned)((threads + block - 1) / block), block, 0, s>>>(out, count, b);
+    const bool small = P::N > 1 && count <= kPowSmall;
+    const int chunk = small ? 8 : 32, block = small ? 32 : 128;
+    const uint64_t threads = (count + chunk - 1) / chunk;
+    gen_powers_kernel<P><<<(unsigned)((threads + block - 1) / block), block, 0, s>>>(out, count, b, chunk);
     return cudaGetLastError();
   }
   static cudaError_t step_table(uint32_t* out, const uint32_t* tw, int r, int inner, int shift, cudaStream_t s) {
